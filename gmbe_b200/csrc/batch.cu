@@ -43,7 +43,7 @@ struct mbe_batch {
   cudaGraphExec_t exec = nullptr;
   uint64_t exec_gen = 0;
   mbe_params exec_prm;
-  int exec_warps = 0;
+  LaunchPlan plan;  // of the captured launch
 };
 
 namespace {
@@ -112,8 +112,14 @@ bool same_global(const mbe_params& a, const mbe_params& c) {
 // Captures (or re-captures) the launch when the workspace or the global
 // parameters changed since the last capture.  Caller holds the workspace lock.
 int ensure_captured(mbe_batch* b, Workspace& ws, const mbe_params& prm) {
-  if (b->exec && b->exec_gen == ws.gen && same_global(prm, b->exec_prm)) return MBE_OK;
-  LaunchPlan plan;
+  if (b->exec && b->exec_gen == ws.gen && same_global(prm, b->exec_prm)) {
+    // The captured launch starts from all-zero count maps.  Another launch on
+    // this device may have had its scratch laid out differently since, or
+    // have ended early: clear them as a fresh launch would.
+    b->plan.clear_maps = !engine_maps_clean(ws, b->plan);
+    return engine_clear_maps(ws, &b->plan, b->stream);
+  }
+  LaunchPlan& plan = b->plan;
   int rc = engine_prepare(ws, b->spec, prm, &plan);
   if (rc) return rc;
   if ((rc = engine_clear_maps(ws, &plan, b->stream))) return rc;
@@ -147,7 +153,6 @@ int ensure_captured(mbe_batch* b, Workspace& ws, const mbe_params& prm) {
   }
   b->exec_gen = ws.gen;
   b->exec_prm = prm;
-  b->exec_warps = plan.warps;
   return MBE_OK;
 }
 

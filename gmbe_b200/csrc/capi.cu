@@ -335,9 +335,9 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
   }
   // Every task leaves its warp's dense count map all-zero.  A different
   // layout puts the maps elsewhere: they are cleared (strided, maps only).
-  plan->clear_maps = ws.map_pitch_words != plan->sl.words_per_warp ||
-                     ws.map_words != spec.map_words || ws.map_warps < plan->warps ||
-                     ws.map_big != n_big || ws.map_big_pitch != big_sl.words_per_warp;
+  plan->ep.n_big_warps = n_big;
+  plan->ep.big_sl = big_sl;
+  plan->clear_maps = !engine_maps_clean(ws, *plan);
   int32_t qcap = prm.queue_capacity > 0
                      ? prm.queue_capacity
                      : (int32_t)std::min<int64_t>(1 << 22,
@@ -428,6 +428,12 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
   plan->pool.import_s = plan->sl.capS;
   plan->pool.pad = 0;
   return MBE_OK;
+}
+
+bool engine_maps_clean(const Workspace& ws, const LaunchPlan& plan) {
+  return ws.map_pitch_words == plan.sl.words_per_warp && ws.map_words == plan.map_words &&
+         ws.map_warps >= plan.warps && ws.map_big == plan.ep.n_big_warps &&
+         ws.map_big_pitch == plan.ep.big_sl.words_per_warp;
 }
 
 int engine_clear_maps(Workspace& ws, LaunchPlan* plan, cudaStream_t st) {

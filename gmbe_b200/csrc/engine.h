@@ -129,6 +129,9 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
 // the kernel's dynamic shared memory limit to `smem` where it is lower.
 int enum_blocks_per_sm(bool tiers, size_t smem, int* occ);
 
+// Whether every warp's count map is all-zero where the plan's layout has it.
+bool engine_maps_clean(const Workspace& ws, const LaunchPlan& plan);
+
 // Queues the strided clear of every warp's count map if the layout changed
 // since the maps were last cleared (capturable; a no-op otherwise).
 int engine_clear_maps(Workspace& ws, LaunchPlan* plan, cudaStream_t st);
