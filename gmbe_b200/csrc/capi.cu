@@ -149,41 +149,35 @@ ScratchLayout make_layout(int32_t nV, int32_t capC, int32_t capL, int32_t capS) 
   s.touched = take(C);
   s.cv = take(C);
   s.ncnt = take(C);
+  s.lv = take(Lc);
+  s.aoff = take(Lc + 1);
+  s.lkey = take(2 * T2);
+  s.lid = take(T2);
+  s.aadj = take(S);
+  s.ent = take(S);
+  // From here on a root's or a slot's bitmap sub-problem has everything to
+  // itself; the counts tier's own arrays end at ar_sub.
+  s.ar_root = off;
   s.bound = take(C);
   s.coff = take(C + 1);
   s.fill = take(C);
   s.sidx = take(C);
-  s.lv = take(Lc);
   s.llevel = take(Lc);
   s.lp = take(Lc);
-  s.aoff = take(Lc + 1);
   s.stack = take(Lc + 2);
   s.lent = take(Lc + 2);
   s.lbits = take((int64_t)kLevelBits * ((C + 31) / 32));
-  s.aadj = take(S);
   s.cadj = take(S);
-  s.masks = take((int64_t)(kKMax + 1) * C);  // bitmap-tier records (K+1 words each)
-  s.sub_v = take(2 * C);
   s.tcls = take(C);
   s.ckey = take(2 * C);
-  s.ent = take(S);
-  s.lkey = take(2 * T2);
-  s.lid = take(T2);
-  s.lmask = take((T2 + 3) * kKMax);
-  s.t2_rec = take(2 * (T2 + 3));
-  s.t2_n = take(T2 + 3);
-  s.t2_cur = take(T2 + 3);
-  s.t2_top = take(T2 + 3);
-  s.r_sum = take(2 * (T2 + 3));
-  s.r_cnt = take(T2 + 3);
   s.tlist = take(C);
-  // Arena of the bitmap tier's per-level record lists (a level that does not
-  // fit shares its parent's list).
-  s.act_cap = (int32_t)std::min<int64_t>(INT32_MAX / 2, 6 * C + 8192);
-  s.act = take(s.act_cap);
+  s.ar_sub = off;
+  take(13 * C + 9696);
+  s.ar_end = off;
   s.words_per_warp = off;
   const int64_t seen = ((int64_t)nV + 31) / 32;
-  s.seen_words = seen <= kSeenMaxWords ? (int32_t)seen : 0;
+  s.seen_words = seen <= kSeenMaxWords ? (int32_t)((seen + 3) & ~int64_t(3)) : 0;
+  s.smem_words = std::max(s.seen_words, kSmemWords);
   return s;
 }
 
@@ -427,6 +421,7 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
   plan->pool.import_l = plan->sl.capL;
   plan->pool.import_s = plan->sl.capS;
   plan->pool.pad = 0;
+  plan->pool.import_words = plan->sl.ar_end - plan->sl.ar_root;
   return MBE_OK;
 }
 

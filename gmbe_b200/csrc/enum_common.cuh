@@ -87,16 +87,20 @@ struct ScratchLayout {
   int64_t lv, llevel, lp, aoff, stack, lent;  // lent: entries of each level's L rows
   int64_t lbits;        // counts-tier level bitmaps (kLevelBits x ceil(capC / 32) words)
   int64_t aadj, cadj;
-  int64_t masks, sub_v, tcls;  // tcls: class of each touched candidate of a sparse push
-  int64_t ckey, ent;           // ckey: hash key per candidate (uint64); ent: packed entries
-  int64_t lkey, lmask;  // lkey is uint64 (8-byte aligned offset)
-  int64_t lid;          // internal U id of each bitmap-tier L bit (for emission)
-  int64_t t2_rec, t2_n, t2_cur, t2_top, r_sum, r_cnt;  // bitmap-tier stack; t2_rec, r_sum uint64
-  int64_t act, tlist;
-  int32_t act_cap;
+  int64_t tcls;                // class of each touched candidate of a sparse push
+  int64_t ckey, ent, tlist;    // ckey: hash key per candidate (uint64); ent: packed entries
+  int64_t lkey;                // uint64 key of each bitmap-tier L bit (8-byte aligned offset)
+  int64_t lid;                 // its internal U id (for emission)
+  // The bitmap tier's arena.  A sub-problem that starts at a root or a slot
+  // has [ar_root, ar_end), which takes in every counts-tier array; one below a
+  // counts-tier push has [ar_sub, ar_end).
+  int64_t ar_root, ar_sub, ar_end;
   // Words per warp of the first-touch bitmap in shared memory (one bit per
   // V vertex / candidate position); 0 = first touches found by global atomics.
   int32_t seen_words;
+  // Shared memory words per warp: the larger of that bitmap and what the
+  // bitmap tier uses (kSmemWords; fewer: it runs without, and merges nothing).
+  int32_t smem_words;
   // A first-touch bitmap in global memory (one bit per V vertex / candidate
   // position, gseen_words words), right after the count map: large counting
   // passes without the shared one mark touches with fire-and-forget atomics
@@ -121,6 +125,7 @@ struct SlotPool {
   int32_t import_l;   // most L vertices any warp can take in
   int32_t import_s;   // largest two-hop multiset any warp can take in
   int32_t pad;
+  long long import_words;  // bitmap-tier arena words any warp has for a slot's sub-problem
 };
 constexpr int kBigSlotWords = 1 << 20;  // 4 MiB
 
@@ -213,13 +218,18 @@ __device__ __forceinline__ uint64_t fmix64(uint64_t k) {
   return k;
 }
 
-__device__ __forceinline__ uint64_t biclique_hash(const DevGraph& g, uint64_t sU, uint64_t nU,
-                                                  uint64_t sV, uint64_t nV) {
+__device__ __forceinline__ uint64_t biclique_hash_s(int swapped, uint64_t sU, uint64_t nU,
+                                                    uint64_t sV, uint64_t nV) {
   // Internal U is the L side; the canonical hash takes the original-U side first.
-  uint64_t sL = g.swapped ? sV : sU, nL = g.swapped ? nV : nU;
-  uint64_t sR = g.swapped ? sU : sV, nR = g.swapped ? nU : nV;
+  uint64_t sL = swapped ? sV : sU, nL = swapped ? nV : nU;
+  uint64_t sR = swapped ? sU : sV, nR = swapped ? nU : nV;
   uint64_t rot = (sR << 29) | (sR >> 35);
   return fmix64(sL ^ rot ^ ((nL << 32) | nR));
+}
+
+__device__ __forceinline__ uint64_t biclique_hash(const DevGraph& g, uint64_t sU, uint64_t nU,
+                                                  uint64_t sV, uint64_t nV) {
+  return biclique_hash_s(g.swapped, sU, nU, sV, nV);
 }
 
 __device__ __forceinline__ unsigned lane_id() {

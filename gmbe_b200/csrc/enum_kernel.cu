@@ -16,15 +16,27 @@
 //     searching global rows on every push and pop.
 //   * Tier 2 (|L| <= 32*K) re-expresses the same DFS over K-word bitmaps of
 //     the current L: a push is an AND, the maximality test a compare, the
-//     pro-active pruning test an AND with the removed vertices.
+//     pro-active pruning test an AND with the removed vertices.  Candidates
+//     of one neighbourhood are one class, and a sub-problem of at most 32
+//     classes over 32 L vertices is walked in registers, a class per lane.
 //   * Split tasks go to a bounded MPMC ring; every device wait is bounded and
 //     reports a status instead of hanging.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdio>
 
 #include "enum_common.cuh"
 #include "enum_launch.h"
+
+// Loops are kept rolled unless they say otherwise, and what several places call
+// stays out of line.  The kernel is bound by instruction fetch: its warps are
+// each in another part of the code, a third of their fetches missed, and most
+// of their stalls were for want of an instruction.  Unrolled and inlined by the
+// compiler's own choice the code was 864 KB, rolled it is 303 KB; the bitmap
+// tier's time on a 300,000-edge graph, summed over the warps, went from 50 to
+// 20 s by that alone.
+#define ROLLED _Pragma("unroll 1")
 
 namespace gmbe {
 
@@ -40,22 +52,154 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return r;
 }
 
-__device__ void set_status(EnumCtl* ctl, int32_t code, unsigned long long info) {
+__device__ __noinline__ void set_status(EnumCtl* ctl, int32_t code, unsigned long long info) {
   if (atomicCAS(&ctl->status, 0, code) == 0) ctl->err_info = info;
   atomicExch(&ctl->abort, 1);
 }
 
+// Sums over the warp, out of line: a score of call sites would each hold the
+// reduction.
+__device__ __noinline__ unsigned long long warp_sum64(unsigned long long v) { return warp_sum(v); }
+// Exclusive prefix sum within the warp, and above it (32 bits up) the total.
+__device__ __noinline__ unsigned long long scan32(int v) {
+  int tot;
+  const int ex = warp_excl_scan(v, &tot);
+  return ((unsigned long long)(unsigned)tot << 32) | (unsigned)ex;
+}
+__device__ __forceinline__ int excl_scan(int v, int* tot) {
+  const unsigned long long r = scan32(v);
+  *tot = (int)(r >> 32);
+  return (int)r;
+}
+
+// Visits every entry of a list of rows with all 32 lanes busy, in order.
+// row_of(r, beg, len) describes row r; load(valid, pos) reads what the visit
+// needs, pos indexing the global entry array, and visit(valid, r, k, v) gets it,
+// k counting the entries; both are called by every lane (uniform control flow).
+// Two loads per lane are issued before the first visit: a walk is bound by
+// their latency (and, unrolled further, by its own code).
+template <typename RowOf, typename Load, typename Visit>
+__device__ __forceinline__ void flat_rows(int nr, RowOf row_of, Load load, Visit visit) {
+  const int lane = (int)lane_id();
+  int done = 0;
+  ROLLED for (int r0 = 0; r0 < nr; r0 += 32) {
+    int beg = 0, len = 0;
+    if (r0 + lane < nr) row_of(r0 + lane, beg, len);
+    int tot;
+    const int ex = excl_scan(len, &tot);
+    beg -= ex;
+    ROLLED for (int e0 = 0; e0 < tot; e0 += 64) {
+      int r[2];
+      decltype(load(true, 0)) v[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        r[u] = 0;
+        if (e0 + 32 * u < tot) {
+          const int e = e0 + 32 * u + lane;
+          int lo = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            const int cand = lo + step;
+            if (__shfl_sync(kFull, ex, cand) <= e) lo = cand;
+          }
+          r[u] = r0 + lo;
+          v[u] = load(e < tot, __shfl_sync(kFull, beg, lo) + e);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (e0 + 32 * u < tot)
+          visit(e0 + 32 * u + lane < tot, r[u], done + e0 + 32 * u + lane, v[u]);
+    }
+    done += tot;
+  }
+}
+
+// What every warp of a block shares, and each warp's own state.  Both live in
+// shared memory: functions that are not inlined reach them at a fixed address,
+// and nothing of them takes up registers or local memory (whose traffic would
+// evict the warps' working sets from L1).
+struct Block {
+  const EnumParams* p;   // the rest of the launch's parameters
+  EnumCtl* ctl;
+  Task* q_tasks;
+  unsigned long long* q_seq;
+  const DevGraph* graphs;  // every graph of the launch
+  int32_t* slots;        // exported bitmap sub-problems (nslot x kSlotWords)
+  uint32_t* slot_bits;   // slot occupancy
+  int32_t* bigslots;     // large slots (nbig x kBigSlotWords)
+  uint32_t* big_bits;
+  int32_t* emit;
+  uint64_t deadline;      // %globaltimer after which the launch gives up (0: never)
+  long long import_words; // arena words every warp of the launch has
+  int nslot, nbig;
+  int import_cap;        // most candidates any warp of the launch can take in
+  int import_l, import_s; // most L vertices / two-hop entries any warp can take in
+  // Copies of parameters read often.
+  int32_t prune, server, share_min_work, slot_records, eager_share, share_counts, touch_scan;
+  int32_t smem_words;
+  int32_t lookout;  // 1 while an idle warp of the block watches the queue
+};
+
+struct Warp {
+  int32_t* base;           // this warp's scratch
+  const DevGraph* gp;      // graph of the task being run
+  int32_t gid;
+  int32_t tier;            // index of the warp's layout in s_sl
+  // Accumulators, kept by lane 0 (acc).
+  unsigned long long cnt, hash, nonmax, splits;
+  unsigned long long ns_t2, n_t2;  // time inside the bitmap tier, sub-problems run
+  unsigned long long pushes;       // pushes so far: counts tier | bitmap tier << 32
+  unsigned long long shape;        // last task set up: |C| | (part << 32) | (parts << 48)
+  unsigned long long ns_t1;        // time inside the counts tier (bitmap tier excluded)
+  uint32_t* seen;                  // this warp's first-touch bitmap in shared memory, or null
+  long long dem_t;                 // clock64 of the last export-demand reading (lane 0)
+  int dem;                         // that reading
+
+  __device__ __forceinline__ const ScratchLayout& sl() const;
+  __device__ __forceinline__ int32_t* A(int64_t off) const { return base + off; }
+  __device__ __forceinline__ uint64_t* A64(int64_t off) const {
+    return reinterpret_cast<uint64_t*>(base + off);
+  }
+  // This warp's first-touch bitmap in global memory.
+  __device__ __forceinline__ uint32_t* gseen() const;
+  // Arena words of a sub-problem that starts at a root or a slot, or below a
+  // counts-tier push.
+  __device__ __forceinline__ long long root_words() const;
+  __device__ __forceinline__ long long sub_words() const;
+};
+
+__shared__ Block s_blk;
+__shared__ ScratchLayout s_sl[2];
+__shared__ Warp s_warp[kEnumWarps];
+extern __shared__ uint4 enum_smem4[];
+
+__device__ __forceinline__ Warp& this_warp() { return s_warp[threadIdx.x >> 5]; }
+// This warp's part of the dynamic shared memory.
+__device__ __forceinline__ uint32_t* this_smem() {
+  return reinterpret_cast<uint32_t*>(enum_smem4) + (size_t)(threadIdx.x >> 5) * s_blk.smem_words;
+}
+__device__ __forceinline__ const ScratchLayout& Warp::sl() const { return s_sl[tier]; }
+__device__ __forceinline__ uint32_t* Warp::gseen() const {
+  return reinterpret_cast<uint32_t*>(base + sl().gseen);
+}
+__device__ __forceinline__ long long Warp::root_words() const { return sl().ar_end - sl().ar_root; }
+__device__ __forceinline__ long long Warp::sub_words() const { return sl().ar_end - sl().ar_sub; }
+// Adds to one of the warp's accumulators (v: the same in every lane).
+__device__ __forceinline__ void acc(unsigned long long& a, unsigned long long v) {
+  if (lane_id() == 0) a += v;
+}
+
 // Whether this warp should leave its task (lane-uniform): the launch is
 // aborting, or its time limit has passed (which starts the abort).
-template <typename WarpT>
-__device__ __forceinline__ bool must_stop(const WarpT& W) {
+__device__ __noinline__ bool must_stop() {
   int s = 0;
   if (lane_id() == 0) {
-    s = *(volatile int32_t*)&W.ctl->abort;
-    if (!s && W.deadline != 0) {
+    s = *(volatile int32_t*)&s_blk.ctl->abort;
+    if (!s && s_blk.deadline != 0) {
       const uint64_t now = globaltimer_ns();
-      if (now > W.deadline) {
-        set_status(W.ctl, kStDeadline, now - W.deadline);
+      if (now > s_blk.deadline) {
+        set_status(s_blk.ctl, kStDeadline, now - s_blk.deadline);
         s = 1;
       }
     }
@@ -63,68 +207,13 @@ __device__ __forceinline__ bool must_stop(const WarpT& W) {
   return __shfl_sync(0xffffffffu, s, 0) != 0;
 }
 
-// Visits every entry of a list of rows with all 32 lanes busy.  row_of(r, beg,
-// len) describes row r; visit(valid, r, pos) is called by every lane (uniform
-// control flow), pos indexing the global entry array.
-template <typename RowOf, typename Visit>
-__device__ __forceinline__ void flat_rows(int nr, RowOf row_of, Visit visit) {
-  const int lane = (int)lane_id();
-  for (int r0 = 0; r0 < nr; r0 += 32) {
-    int r = r0 + lane, beg = 0, len = 0;
-    if (r < nr) row_of(r, beg, len);
-    int tot;
-    int ex = warp_excl_scan(len, &tot);
-    for (int e0 = 0; e0 < tot; e0 += 32) {
-      int e = e0 + lane;
-      int lo = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        int cand = lo + step;
-        int exc = __shfl_sync(kFull, ex, cand & 31);
-        if (cand < 32 && exc <= e) lo = cand;
-      }
-      int b = __shfl_sync(kFull, beg, lo);
-      int exl = __shfl_sync(kFull, ex, lo);
-      bool valid = e < tot;
-      visit(valid, r0 + lo, b + (e - exl));
-    }
-  }
+// Before a counting pass over `words` bitmap words: the bitmap tier, which uses
+// the same shared memory, may have left anything there.
+__device__ __forceinline__ void clear_seen(const Warp& W, int words) {
+  if (!W.seen) return;
+  ROLLED for (int i = (int)lane_id(); i < words; i += 32) W.seen[i] = 0u;
+  __syncwarp();
 }
-
-struct Warp {
-  // Launch constants, read in place from the kernel's parameter space.
-  const EnumParams& p;
-  const ScratchLayout& sl;
-  EnumCtl* ctl;
-  Task* q_tasks;
-  unsigned long long* q_seq;
-  int32_t* slots;        // exported bitmap sub-problems (nslot x slot_words)
-  uint32_t* slot_bits;   // slot occupancy
-  int nslot;
-  int32_t* bigslots;     // large slots (nbig x kBigSlotWords)
-  uint32_t* big_bits;
-  int nbig;
-  int import_cap;        // most candidates any warp of the launch can take in
-  int import_l, import_s; // most L vertices / two-hop entries any warp can take in
-  int32_t* base;
-  const DevGraph* graphs;  // every graph of the launch
-  const DevGraph* gp;      // graph of the task being run
-  int32_t gid;
-  // accumulators (uniform over lanes)
-  unsigned long long cnt, hash, nonmax, splits;
-  unsigned long long ns_t2, n_t2;  // time inside the bitmap tier, sub-problems run
-  unsigned long long pushes;       // pushes so far: counts tier | bitmap tier << 32
-  unsigned long long shape;        // last task set up: |C| | (part << 32) | (parts << 48)
-  unsigned long long ns_t1;        // time inside the counts tier (bitmap tier excluded)
-  uint32_t* seen;                  // this warp's first-touch bitmap in shared memory, or null
-  uint64_t deadline;               // %globaltimer after which the launch gives up (0: never)
-  uint32_t* gseen;                 // this warp's first-touch bitmap in global memory
-  long long dem_t;                 // clock64 of the last export-demand reading (lane 0)
-  int dem;                         // that reading
-
-  __device__ int32_t* A(int64_t off) const { return base + off; }
-  __device__ uint64_t* A64(int64_t off) const { return reinterpret_cast<uint64_t*>(base + off); }
-};
 
 // Adds 1 to counts[i] and tells whether this was i's first touch since the
 // counts were last cleared.  With a shared-memory bitmap the first touch is a
@@ -146,7 +235,7 @@ __device__ __forceinline__ void counts_done(const Warp& W, const int32_t* idx, i
   __threadfence_block();
   __syncwarp();
   if (W.seen) {
-    for (int i = (int)lane_id(); i < n; i += 32) W.seen[idx[i] >> 5] = 0u;
+    ROLLED for (int i = (int)lane_id(); i < n; i += 32) W.seen[idx[i] >> 5] = 0u;
     __syncwarp();
   }
 }
@@ -157,7 +246,7 @@ __device__ __forceinline__ void counts_done(const Warp& W, const int32_t* idx, i
 // that a scan of the words costs less than an atomic round trip per 32
 // entries.
 __device__ __forceinline__ bool use_gseen(const Warp& W, long long entries, int words) {
-  if (W.p.touch_scan != 0) return W.p.touch_scan > 0;
+  if (s_blk.touch_scan != 0) return s_blk.touch_scan > 0;
   return W.seen == nullptr && entries >= (long long)words;
 }
 
@@ -166,15 +255,15 @@ __device__ __forceinline__ bool use_gseen(const Warp& W, long long entries, int 
 // returns the number of set bits.  Every lane takes one word per round, so
 // the loads are independent and coalesced.  The bits were set by this warp's
 // atomics: the fence before the call makes them visible here.
-__device__ int collect_bits(uint32_t* bits, int words, int32_t* out, int cap) {
+__device__ __noinline__ int collect_bits(uint32_t* bits, int words, int32_t* out, int cap) {
   const int lane = (int)lane_id();
   int n = 0;
-  for (int w0 = 0; w0 < words; w0 += 32) {
+  ROLLED for (int w0 = 0; w0 < words; w0 += 32) {
     const int w = w0 + lane;
     uint32_t m = w < words ? __ldcg(bits + w) : 0u;
     if (m) bits[w] = 0u;
     int tot;
-    int o = n + warp_excl_scan(__popc(m), &tot);
+    int o = n + excl_scan(__popc(m), &tot);
     while (m) {
       if (o < cap) out[o] = (w << 5) + __ffs(m) - 1;
       ++o;
@@ -214,7 +303,7 @@ __device__ __forceinline__ EmitDst emit_dst(const EnumParams& p) {
 }
 
 // Reserves a record of `count` ids (lane-uniform); -1 if it is dropped.
-__device__ long long emit_reserve(EnumCtl* ctl, const EmitDst& d, int count) {
+__device__ __noinline__ long long emit_reserve(EnumCtl* ctl, const EmitDst& d, int count) {
   const unsigned long long need = (unsigned long long)count + 2;
   long long pos = 0;
   if (lane_id() == 0) {
@@ -260,7 +349,7 @@ __device__ __noinline__ void emit_list(EnumCtl* ctl, EmitDst d, int gid, int n,
                                        const int32_t* ids, const int32_t* idx) {
   const long long pos = emit_reserve(ctl, d, n);
   if (pos < 0) return;
-  for (int i = (int)lane_id(); i < n; i += 32) emit_at(d, pos + 2 + i) = idx ? ids[idx[i]] : ids[i];
+  ROLLED for (int i = (int)lane_id(); i < n; i += 32) emit_at(d, pos + 2 + i) = idx ? ids[idx[i]] : ids[i];
   emit_header(d, pos, n, gid);
 }
 
@@ -270,7 +359,7 @@ __device__ __noinline__ void emit_level(EnumCtl* ctl, EmitDst d, int gid, int co
   const long long pos = emit_reserve(ctl, d, count);
   if (pos < 0) return;
   int out = 0;
-  for (int b0 = 0; b0 < nscan; b0 += 32) {
+  ROLLED for (int b0 = 0; b0 < nscan; b0 += 32) {
     const int l = b0 + (int)lane_id();
     const bool s = l < nscan && llevel[l] == level;
     const unsigned bal = __ballot_sync(kFull, s);
@@ -280,16 +369,15 @@ __device__ __noinline__ void emit_level(EnumCtl* ctl, EmitDst d, int gid, int co
   emit_header(d, pos, count, gid);
 }
 
-// L = lid[b] for the set bits b of the K-word mask (m0..m3), count of them.
-__device__ __noinline__ void emit_mask(EnumCtl* ctl, EmitDst d, int gid, int count, int K,
-                                       uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3,
-                                       const int32_t* lid) {
+// L = lid[b] for the set bits b of a K-word mask (lane w: word w), count of them.
+__device__ __noinline__ void emit_words(EnumCtl* ctl, EmitDst d, int gid, int count, int K,
+                                        uint32_t mw, const int32_t* lid) {
   const long long pos = emit_reserve(ctl, d, count);
   if (pos < 0) return;
   const int lane = (int)lane_id();
   int out = 0;
-  for (int w = 0; w < K; ++w) {
-    const uint32_t m = w == 0 ? m0 : (w == 1 ? m1 : (w == 2 ? m2 : m3));
+  ROLLED for (int w = 0; w < K; ++w) {
+    const uint32_t m = __shfl_sync(kFull, mw, w);
     const bool s = (m >> lane) & 1u;
     if (s) emit_at(d, pos + 2 + out + __popc(m & lanemask_lt())) = lid[w * 32 + lane];
     out += __popc(m);
@@ -300,13 +388,13 @@ __device__ __noinline__ void emit_mask(EnumCtl* ctl, EmitDst d, int gid, int cou
 // Serving block of graph `gid` (a block index into the arena, which the
 // launch receives in place of the descriptor array).
 __device__ __forceinline__ ServeGraph* serve_graph(const Warp& W, int32_t gid) {
-  char* arena = const_cast<char*>(reinterpret_cast<const char*>(W.graphs));
+  char* arena = const_cast<char*>(reinterpret_cast<const char*>(s_blk.graphs));
   return reinterpret_cast<ServeGraph*>(arena + ((size_t)(uint32_t)gid << kServeBlockShift));
 }
 
 // Descriptor of graph `gid` of this launch.
 __device__ __forceinline__ const DevGraph* graph_at(const Warp& W, int32_t gid) {
-  return W.p.server ? &serve_graph(W, gid)->g : W.graphs + gid;
+  return s_blk.server ? &serve_graph(W, gid)->g : s_blk.graphs + gid;
 }
 
 // Most parts a root is split into.
@@ -321,65 +409,130 @@ __device__ __forceinline__ int part_of(int w, int parts) {
 // Children of the current graph about to be queued (serving: a graph
 // completes when its roots and every queued child have finished).
 __device__ __forceinline__ void graph_spawned(const Warp& W, unsigned long long n) {
-  if (W.p.server) atomicAdd(&serve_graph(W, W.gid)->pending, n);
+  if (s_blk.server) atomicAdd(&serve_graph(W, W.gid)->pending, n);
 }
 
 // ---------------------------------------------------------------------------
 // Bitmap sub-problems.
 //
-// A sub-problem is an L of at most 128 vertices (K = 1, 2 or 4 words) and a
-// list of candidate records of rec_stride(K) words: word 0 = (index << 8) | bound,
-// words 1..K = the candidate's neighbourhood inside L.  index is the
-// candidate's position in the sub-problem, whose order is [Q | P]; bound is
-// GMBE's level bound in 8 bits (kB8Free = live at every level; levels stay
-// at or below 129).  subkey[index] is the candidate's hash key, lkey[b] that
-// of L bit b.
-constexpr uint32_t kB8Free = 255;
-// Words per record: K + 1, except that K = 2 records are padded to 4 words so
-// that one 16-byte access reads or writes a record (one-word records are one
-// 8-byte access).  Lists start at 32-byte aligned scratch slices or slots and
-// follow one another in whole records, so K = 1 and K = 2 lists stay 8- and
-// 16-byte aligned.
-__host__ __device__ constexpr int rec_stride(int K) { return K == 2 ? 4 : K + 1; }
+// A sub-problem is an L of kn vertices (K words of bits) and a list of
+// candidate classes.  A class is one or more candidates with the same
+// neighbourhood inside L: its K mask words, the sum of its P candidates' hash
+// keys, and an info word with their number and two flags, kInfoQ (some
+// candidate of it is in Q) and kInfoP (some candidate of it is in P, i.e. is
+// still to be pushed).  Classes are in push order: those with a P candidate
+// stand at the position of their first one.
+//
+// Merging candidates into classes leaves GMBE's search tree as it is.  When a
+// candidate x is popped, finder_pop retires every candidate whose
+// neighbourhood lies inside x's, so of several candidates with one
+// neighbourhood only the first P candidate is ever pushed at that level; that
+// push is non-maximal exactly if one of them is in Q (or another Q candidate
+// covers it).  A biclique that is counted is covered by no Q candidate, and a
+// retired candidate always has a popped one (in Q from then on) above it, so
+// R consists of P candidates that are still live: summing a class's P keys
+// gives the same R.  Without pruning the rule does not hold, and nothing is
+// merged.
+//
+// What a push costs is the list it goes through.  On a 300,000-edge graph the
+// average push met 848 candidates and meets 88 classes (319 and 62, 190 and 34
+// on graphs of 20,000 to 40,000 edges), and 73 % of the pushes have at most 32,
+// one per lane.  Together with the rolled code: 28 x 40 vertices at
+// density 0.8 10.1 -> 2.2 ms, 160 graphs through a server 447 -> 336 ms, the 300,000-edge
+// graph 61 -> 52 ms (where one root's counts tier, on one warp, is most of it).
+//
+// Lists live in memory as planes (word w of class i at m[w * stride + i]), so
+// a warp's sweep over 32 classes reads one line per mask word.
+constexpr uint32_t kInfoQ = 1u << 31;
+constexpr uint32_t kInfoP = 1u << 30;
+constexpr uint32_t kInfoCnt = kInfoP - 1u;
 
-struct T2Src {
-  uint32_t* rec;           // nsub records, writable (their bounds change)
-  const uint64_t* subkey;
-  const uint64_t* lkey;
-  const int32_t* lid;      // internal U id of each L bit (emission only)
-  uint32_t L0[4];          // the sub-problem's L
-  int nsub, nq;            // records [0, nq) are Q, [nq, nsub) P
-  int nend;                // the first level pushes records [nq, nend) only
-  uint64_t sR0;            // R of the sub-problem's root biclique
-  uint32_t nR0;
+struct ClsList {
+  uint32_t* m;     // K planes of `stride` words
+  uint64_t* key;   // [stride] sum of the P candidates' hash keys
+  uint32_t* info;  // [stride] number of P candidates | flags
+  int n, stride, K;
 };
 
-// Slot layout (int32 words): header, lkey (128 x uint64), records, subkey.
-constexpr int kSlotWords = 32768;
-constexpr int kSlotHdr = 16;
-constexpr int kSlotLkey = kSlotHdr;
-constexpr int kSlotLid = kSlotLkey + 2 * 32 * 4;  // 128 int32: the L bits' vertex ids
-constexpr int kSlotRec = kSlotLid + 32 * 4;
-__host__ __device__ constexpr int slot_cap(int K) {
-  return ((kSlotWords - kSlotRec - 2) / (rec_stride(K) + 2)) & ~31;
-}
-__host__ __device__ constexpr int big_slot_cap(int K) {
-  return ((kBigSlotWords - kSlotRec - 2) / (rec_stride(K) + 2)) & ~31;
-}
-static_assert(slot_cap(1) == kSlotMaxRecords && slot_cap(1) >= slot_cap(2) &&
-                  slot_cap(2) >= slot_cap(4) && kSlotWords == kSlotWordsHost,
-              "host view of the slot size");
-// header words: 0 K, 1 nsub, 2 nq, 3 graph, 4..7 L0, 8..9 sR0, 10 nR0
-__device__ __forceinline__ uint64_t* slot_subkey(int32_t* sp, int K, int nsub) {
-  return reinterpret_cast<uint64_t*>(sp + kSlotRec + ((nsub * rec_stride(K) + 1) & ~1));
+__host__ __device__ __forceinline__ long long cls_stride(long long n) { return (n + 31) & ~31LL; }
+// Words of a list of n classes with K-word masks (a multiple of 32).
+__host__ __device__ __forceinline__ long long cls_list_words(long long n, int K) {
+  return cls_stride(n) * (K + 3);
 }
 
+__device__ __forceinline__ ClsList cls_list_at(uint32_t* base, int n, int K) {
+  ClsList l;
+  l.n = n;
+  l.K = K;
+  l.stride = (n + 31) & ~31;
+  l.m = base;
+  l.key = reinterpret_cast<uint64_t*>(base + (size_t)l.stride * K);
+  l.info = base + (size_t)l.stride * (K + 2);
+  return l;
+}
+
+// One level of the walk while a deeper one runs, in the warp's arena: the
+// list it works on and where its live, Q and P bits (a bit per class) are; its
+// L words follow.
+struct ClsFrame {
+  ClsList l;
+  const uint64_t* lk;  // hash key of each L bit
+  const int32_t* lid;  // internal U id of each L bit (emission only)
+  uint64_t sR;         // R of the push that opened the level
+  ClsFrame* prev;
+  uint32_t* A;         // live, Q and P bits
+  uint32_t *top, *stop;  // first free word above the level: arena, shared memory
+  uint32_t nR;
+  int nend;            // classes [0, nend) may be pushed here
+  int curw;            // word the scan for the next candidate stands at
+};
+constexpr int kFrameWords = (int)((sizeof(ClsFrame) / 4 + 3) & ~3u);
+__host__ __device__ __forceinline__ long long cls_frame_words(long long n, int K) {
+  return kFrameWords + 3 * ((((n + 31) >> 5) + 1) & ~1LL) + ((K + 1) & ~1);
+}
+// Most levels of a sub-problem: a level's L and its classes to push are both
+// fewer than those of the level above.
+__host__ __device__ __forceinline__ int cls_levels(int kn, int np) {
+  return kn < np + 1 ? kn : np + 1;
+}
+// Words a sub-problem of n classes, K words and so many levels may need: its
+// list, two words of bits per 32 classes that a push makes, a frame per level
+// (a level that finds no room for a list of its own works on the one above it
+// with bits of its own), and room for the keys of a leaf's L bits.
+__host__ __device__ __forceinline__ long long cls_need(long long n, int K, int levels) {
+  return cls_list_words(n, K) + 4 * ((n + 63) >> 6) + (long long)levels * cls_frame_words(n, K) +
+         512;
+}
+
+__device__ __forceinline__ int words_k(int n) {
+  int w = (n + 31) >> 5;
+  return w <= 2 ? (w < 1 ? 1 : w) : (w <= 4 ? 4 : w);
+}
+
+// Slot layout (int32 words): header, L words, L keys, L ids, then the list.
+constexpr int kSlotWords = 32768;
+constexpr int kSlotHdr = 16;
+constexpr int kSlotL = kSlotHdr;
+constexpr int kSlotLk = kSlotL + kKMax;             // 32 kKMax uint64
+constexpr int kSlotLid = kSlotLk + 2 * 32 * kKMax;  // 32 kKMax int32
+constexpr int kSlotList = (kSlotLid + 32 * kKMax + 31) & ~31;
+__host__ __device__ constexpr int slot_cap(int K) {
+  return ((kSlotWords - kSlotList) / (K + 3)) & ~31;
+}
+__host__ __device__ constexpr int big_slot_cap(int K) {
+  return ((kBigSlotWords - kSlotList) / (K + 3)) & ~31;
+}
+static_assert(slot_cap(1) <= kSlotMaxRecords && slot_cap(1) >= slot_cap(2) &&
+                  slot_cap(2) >= slot_cap(4) && kSlotWords == kSlotWordsHost,
+              "host view of the slot size");
+// header words: 0 K, 1 n, 2 kn, 3 graph, 4..5 sR, 6 nR
+
 // Claims a free slot of an occupancy bitmap of n slots (lane 0); -1 if none.
-__device__ int bits_alloc(uint32_t* bits, int n) {
+__device__ __noinline__ int bits_alloc(uint32_t* bits, int n) {
   const int nw = n >> 5;
   if (nw == 0) return -1;
   int start = (int)(((blockIdx.x * 32u + (threadIdx.x >> 5)) * 2654435761u) % (unsigned)nw);
-  for (int t = 0; t < nw; ++t) {
+  ROLLED for (int t = 0; t < nw; ++t) {
     int wi = (start + t) % nw;
     unsigned cur = *(volatile unsigned*)&bits[wi];
     while (cur != 0xffffffffu) {
@@ -393,38 +546,38 @@ __device__ int bits_alloc(uint32_t* bits, int n) {
 }
 
 // A regular slot (lane 0); -1 if none.
-__device__ int slot_alloc(Warp& W) { return bits_alloc(W.slot_bits, W.nslot); }
+__device__ int slot_alloc(Warp& W) { return bits_alloc(s_blk.slot_bits, s_blk.nslot); }
 
-// A slot for a sub-problem of nsub candidates with K-word masks (lane 0): a
-// regular one when it fits, else a large one if some warp of every tier can
-// take it in; -1 if none.
-__device__ __forceinline__ bool regular_fits(const Warp& W, int nsub, int K) {
-  return nsub <= slot_cap(K) && (W.p.slot_records <= 0 || nsub <= W.p.slot_records);
+__device__ __forceinline__ bool regular_fits(const Warp& W, int n, int K) {
+  return n <= slot_cap(K) && (s_blk.slot_records <= 0 || n <= s_blk.slot_records);
 }
 
-__device__ int slot_alloc_for(Warp& W, int nsub, int K) {
-  if (regular_fits(W, nsub, K)) return slot_alloc(W);
-  if (nsub > big_slot_cap(K) || nsub > W.import_cap) return -1;
-  const int b = bits_alloc(W.big_bits, W.nbig);
-  return b < 0 ? -1 : W.nslot + b;
+// A slot for a sub-problem of n classes with K-word masks (lane 0): a regular
+// one when it fits, else a large one; -1 if none.
+__device__ int slot_alloc_for(Warp& W, int n, int K) {
+  if (regular_fits(W, n, K)) return slot_alloc(W);
+  if (n > big_slot_cap(K)) return -1;
+  const int b = bits_alloc(s_blk.big_bits, s_blk.nbig);
+  return b < 0 ? -1 : s_blk.nslot + b;
 }
 
-// Whether a child of nsub candidates can be exported at all.
-__device__ __forceinline__ bool slot_fits(const Warp& W, int nsub, int K) {
-  return regular_fits(W, nsub, K) ||
-         (W.nbig > 0 && nsub <= big_slot_cap(K) && nsub <= W.import_cap);
+// Whether a child of n classes and so many levels can be exported at all:
+// some kind of slot holds it, and every warp of the launch can run it.
+__device__ __forceinline__ bool slot_fits(const Warp& W, int n, int K, int levels) {
+  if (s_blk.nslot == 0 || cls_need(n, K, levels) + 96LL * K > s_blk.import_words) return false;
+  return regular_fits(W, n, K) || (s_blk.nbig > 0 && n <= big_slot_cap(K));
 }
 
 __device__ __forceinline__ int32_t* slot_ptr(const Warp& W, int s) {
-  return s < W.nslot ? W.slots + (size_t)s * kSlotWords
-                     : W.bigslots + (size_t)(s - W.nslot) * kBigSlotWords;
+  return s < s_blk.nslot ? s_blk.slots + (size_t)s * kSlotWords
+                     : s_blk.bigslots + (size_t)(s - s_blk.nslot) * kBigSlotWords;
 }
 
 __device__ void slot_free(Warp& W, int s) {
-  if (s < W.nslot) atomicAnd(&W.slot_bits[s >> 5], ~(1u << (s & 31)));
+  if (s < s_blk.nslot) atomicAnd(&s_blk.slot_bits[s >> 5], ~(1u << (s & 31)));
   else {
-    const int b = s - W.nslot;
-    atomicAnd(&W.big_bits[b >> 5], ~(1u << (b & 31)));
+    const int b = s - s_blk.nslot;
+    atomicAnd(&s_blk.big_bits[b >> 5], ~(1u << (b & 31)));
   }
 }
 
@@ -436,14 +589,15 @@ __device__ bool queue_push_one(Warp& W, const Task& t);
 // child, so a reading is reused for kDemandCycles SM clocks (about 2 us):
 // demand moves with warps going idle, far more slowly than children come.
 constexpr long long kDemandCycles = 4096;
-__device__ int export_demand(Warp& W) {
+__device__ __noinline__ int export_demand() {
+  Warp& W = this_warp();
   int want = 0;
   if (lane_id() == 0) {
     const long long now = clock64();
     if (now - W.dem_t < kDemandCycles) {
       want = W.dem;
     } else {
-      EnumCtl* c = W.ctl;
+      EnumCtl* c = s_blk.ctl;
       int idle = *(volatile int32_t*)&c->idle_warps;
       unsigned long long queued = *(volatile unsigned long long*)&c->q_tail -
                                   *(volatile unsigned long long*)&c->q_head;
@@ -464,7 +618,7 @@ __device__ __forceinline__ bool big_enough(const Warp& W, int nP, int nL) {
          (long long)nP * nL > (long long)W.gp->bound_size;
 }
 
-// Whether to hand a child (nP P-candidates, |L| = nL) to another warp.  A
+// Whether to hand a child (nP classes to push, |L| = nL) to another warp.  A
 // child that passes GMBE's split test goes whenever warps wait for work.
 // When many warps wait, smaller children go too: the size test misjudges
 // dense graphs, where a few dozen candidates can hold millions of
@@ -474,19 +628,20 @@ __device__ __forceinline__ bool big_enough(const Warp& W, int nP, int nL) {
 // (the counts tier's parents are the heaviest tasks of a launch and are
 // claimed first; their children, queued ahead of new roots, keep every warp
 // busy instead of lengthening the parent).
-__device__ bool should_export(Warp& W, int nP, int nL, bool eager = false) {
+__device__ __forceinline__ bool should_export(Warp& W, int nP, int nL, bool eager = false) {
   if (nP < 2 || nL < 2) return false;
+  const bool sizable = (long long)nP * nL >= s_blk.share_min_work;
   const bool big = big_enough(W, nP, nL);
-  const bool sizable = (long long)nP * nL >= W.p.share_min_work;
   if (!big && !sizable) return false;  // goes at no demand: skip reading it
   if (eager && big) return true;
-  const int d = export_demand(W);
+  const int d = export_demand();
   return (d == 2 && (big || sizable)) || (d == 1 && big);
 }
 
 // Enqueues a filled slot as a task; false if the ring is full.
 // kind 0: a bitmap sub-problem; kind 1: a counts-tier child (vertex lists).
-__device__ bool slot_publish(Warp& W, int slot, int kind = 0) {
+__device__ __noinline__ bool slot_publish(int slot, int kind) {
+  Warp& W = this_warp();
   __syncwarp();
   __threadfence();
   Task t;
@@ -497,374 +652,1117 @@ __device__ bool slot_publish(Warp& W, int slot, int kind = 0) {
   return queue_push_one(W, t);
 }
 
-__device__ void slot_header(int32_t* sp, int K, int nsub, int nq, const uint32_t* L0, uint64_t sR,
-                            uint64_t nR, int gid) {
+__device__ void slot_header(int32_t* sp, int K, int n, int kn, uint64_t sR, uint64_t nR, int gid) {
   sp[0] = K;
-  sp[1] = nsub;
-  sp[2] = nq;
+  sp[1] = n;
+  sp[2] = kn;
   sp[3] = gid;
-  for (int w = 0; w < 4; ++w) sp[4 + w] = w < K ? (int32_t)L0[w] : 0;
-  *reinterpret_cast<uint64_t*>(sp + 8) = sR;
-  sp[10] = (int32_t)nR;
+  *reinterpret_cast<uint64_t*>(sp + 4) = sR;
+  sp[6] = (int32_t)nR;
 }
 
-// Exports the child of a push of a bitmap sub-problem (its records
-// `child`, in order, the first nbefore of them Q) to an idle warp.
-template <int K>
-__device__ bool t2_try_export(Warp& W, const T2Src& src, const uint32_t* child, int nchild,
-                              int nbefore, const uint32_t* Ln, int kn, uint64_t sR, uint64_t nR) {
-  if (!slot_fits(W, nchild, K) || !should_export(W, nchild - nbefore, kn))
-    return false;
+// Bit i of word w set below i classes: the first n bits of a bit string.
+__device__ __forceinline__ uint32_t first_bits(int n, int w) {
+  const int b = n - 32 * w;
+  return b >= 32 ? 0xffffffffu : (b <= 0 ? 0u : (1u << b) - 1u);
+}
+
+// ---------------------------------------------------------------------------
+// Shared memory of a warp, in words: the merge table, the level being walked,
+// the indices of a child's classes, and an arena for the masks and the live, Q
+// and P bits of the levels being walked.  A warp waits about 30 cycles for
+// shared memory and ten times that for a line another lane's store has sent to
+// L2, and a push is a chain of such accesses.
+constexpr int kSlots = 256;  // entries of the merge table
+constexpr int kSmTab = 0;    // five arrays: mask, leader, key sum (low, high), info
+constexpr int kSmCur = kSmTab + 5 * kSlots;
+constexpr int kSmIdx = kSmCur + 40;
+constexpr int kSmArena = kSmIdx + kChildMax;
+static_assert(kSmArena < kSmemWords && kSmArena % 8 == 0, "shared memory layout");
+static_assert(kChildMax * 2 <= kSlots, "probing ends");
+
+struct MergeTab {  // all-zero between merges
+  uint32_t *mask, *lead, *lo, *hi, *info;
+};
+__device__ __forceinline__ MergeTab this_tab() {
+  uint32_t* t = this_smem() + kSmTab;
+  return MergeTab{t, t + kSlots, t + 2 * kSlots, t + 3 * kSlots, t + 4 * kSlots};
+}
+// Adds a class to the sums of its leader's entry.  Shared-memory atomics: a
+// popular mask (one vertex of L, say) takes in hundreds of candidates, and
+// that many global atomics on one address held up every warp's memory traffic
+// (432,000 cycles for a merge).
+__device__ __forceinline__ void merge_add(const MergeTab& t, uint32_t h, uint64_t key,
+                                          uint32_t info) {
+  if (info & kInfoP) {
+    const uint32_t lo = (uint32_t)key;
+    const uint32_t old = atomicAdd(&t.lo[h], lo);
+    atomicAdd(&t.hi[h], (uint32_t)(key >> 32) + (old + lo < lo ? 1u : 0u));
+    atomicAdd(&t.info[h], info & kInfoCnt);
+  }
+  atomicOr(&t.info[h], info & (kInfoQ | kInfoP));
+}
+
+__device__ __forceinline__ uint32_t hash_mix(uint32_t h) {
+  h *= 0x9e3779b1u;
+  h ^= h >> 15;
+  return h * 0x85ebca6bu;
+}
+
+// Merges the classes of a list that have one mask, in place and in order
+// (pruning on only); returns the new length, and in `nend` (a prefix length)
+// the number of kept classes among the first nend.  The table holds, per hash
+// of a mask, the class that stands first among those with a P candidate (or,
+// without any, first of all); every other class of the slot with the leader's
+// mask joins it, and one with another mask stays as it is (the merge may miss
+// some: duplicates are retired later, as single candidates would be).  A list
+// longer than the table holds is merged in parts, by hash.  The planes move to
+// the new, smaller stride.  S: one word per 32 classes of scratch.
+__device__ __noinline__ int cls_merge(uint32_t* m, uint64_t* key, uint32_t* info, int n, int K,
+                                      int* stride_io, uint32_t* S, int* nend_io) {
   const int lane = (int)lane_id();
-  int slot = lane == 0 ? slot_alloc_for(W, nchild, K) : 0;
-  slot = __shfl_sync(0xffffffffu, slot, 0);
-  if (slot < 0) return false;
-  constexpr int RS = rec_stride(K);
-  int32_t* sp = slot_ptr(W, slot);
-  uint32_t* rec = reinterpret_cast<uint32_t*>(sp + kSlotRec);
-  uint64_t* key = slot_subkey(sp, K, nchild);
-  uint64_t* lk = reinterpret_cast<uint64_t*>(sp + kSlotLkey);
-  for (int q = lane; q < nchild; q += 32) {
-    const uint32_t* c = child + (size_t)q * RS;
-    rec[(size_t)q * RS] = ((uint32_t)q << 8) | kB8Free;
+  const MergeTab t = this_tab();
+  const size_t st = (size_t)*stride_io;
+  constexpr int U = 2;
+  // The hashes of U chunks of classes, their loads in flight together.
+  const auto hashes = [&](int b, uint32_t* h) {
 #pragma unroll
-    for (int w = 0; w < K; ++w) rec[(size_t)q * RS + 1 + w] = c[1 + w];
-    key[q] = src.subkey[c[0] >> 8];
+    for (int u = 0; u < U; ++u) h[u] = 0x51ed270bu;
+    ROLLED for (int w = 0; w < K; ++w) {
+      uint32_t x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b + 32 * u + lane;
+        x[u] = i < n ? m[w * st + i] : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) h[u] = (h[u] ^ x[u]) * 0x9e3779b1u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) h[u] = hash_mix(h[u]);
+  };
+  const uint32_t parts = n <= 1024 ? 1u : (n <= 2048 ? 2u : (n <= 4096 ? 4u : (n <= 8192 ? 8u : 16u)));
+  ROLLED for (int w = lane; w < ((n + 31) >> 5); w += 32) S[w] = first_bits(n, w);
+  ROLLED for (uint32_t part = 0; part < parts; ++part) {
+    ROLLED for (int b = 0; b < n; b += 32 * U) {
+      uint32_t h[U], v[U];
+      hashes(b, h);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b + 32 * u + lane;
+        v[u] = 0u;
+        if (i < n) {
+          v[u] = ((info[i] & kInfoP) ? 0x7fffffffu : 0x3fffffffu) - (uint32_t)i;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v[u] && (h[u] & (parts - 1u)) == part) atomicMax(&t.lead[h[u] >> 24], v[u]);
+    }
+    __syncwarp();
+    ROLLED for (int b = 0; b < n; b += 32 * U) {
+      int j[U];
+      uint32_t h[U];
+      hashes(b, h);
+      bool gone[U], any = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b + 32 * u + lane;
+        j[u] = i;
+        if (i < n && (h[u] & (parts - 1u)) == part) {
+          const uint32_t v = t.lead[h[u] >> 24];
+          j[u] = (int)(v > 0x3fffffffu ? 0x7fffffffu - v : 0x3fffffffu - v);
+        }
+        gone[u] = j[u] != i;
+        any |= gone[u];
+      }
+      if (!__any_sync(kFull, any)) continue;
+      ROLLED for (int w = 0; w < K; ++w) {
+        uint32_t x[U], y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          x[u] = gone[u] ? m[w * st + b + 32 * u + lane] : 0u;
+          y[u] = gone[u] ? m[w * st + j[u]] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) gone[u] &= x[u] == y[u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b + 32 * u + lane;
+        if (gone[u]) {
+          const uint32_t f = info[i];
+          merge_add(t, h[u] >> 24, (f & kInfoP) ? key[i] : 0ULL, f);
+        }
+        const unsigned bal = __ballot_sync(kFull, gone[u]);
+        if (lane == 0 && bal) S[(b >> 5) + u] &= ~bal;
+      }
+    }
+    __syncwarp();
+    // the leaders' sums; the table back to zero
+    ROLLED for (int h = lane; h < kSlots; h += 32) {
+      const uint32_t v = t.lead[h];
+      if (v) {
+        const uint32_t f = t.info[h];
+        if (f) {
+          const int j = (int)(v > 0x3fffffffu ? 0x7fffffffu - v : 0x3fffffffu - v);
+          key[j] += (uint64_t)t.lo[h] | ((uint64_t)t.hi[h] << 32);
+          info[j] = (info[j] + (f & kInfoCnt)) | (f & (kInfoQ | kInfoP));
+          t.lo[h] = t.hi[h] = t.info[h] = 0u;
+        }
+        t.lead[h] = 0u;
+      }
+    }
+    __syncwarp();
   }
-  for (int b = lane; b < 32 * K; b += 32) lk[b] = src.lkey[b];
-  if (W.p.emit) {  // L ids are needed for emission only
-    int32_t* li = sp + kSlotLid;
-    for (int b = lane; b < 32 * K; b += 32) li[b] = src.lid[b];
+  const int nend = *nend_io;
+  int kept = 0, kend = 0;
+  ROLLED for (int w = lane; w < ((n + 31) >> 5); w += 32) {
+    const uint32_t k = S[w];
+    kept += __popc(k);
+    kend += __popc(k & first_bits(nend, w));
   }
-  if (lane == 0) slot_header(sp, K, nchild, nbefore, Ln, sR, nR, W.gid);
-  if (slot_publish(W, slot)) return true;
+  kept = (int)__reduce_add_sync(kFull, (unsigned)kept);
+  *nend_io = (int)__reduce_add_sync(kFull, (unsigned)kend);
+  if (kept == n) return n;
+  const size_t ns = (size_t)((kept + 31) & ~31);
+  // Every class moves down, plane after plane: what is written lies below
+  // everything still to be read.
+  ROLLED for (int w = 0; w < K; ++w) {
+    int o = 0;
+    ROLLED for (int b = 0; b < n; b += 32 * U) {
+      uint32_t x[U], bal[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b + 32 * u;
+        bal[u] = i < n ? S[i >> 5] : 0u;
+        x[u] = (bal[u] >> lane) & 1u ? m[w * st + i + lane] : 0u;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if ((bal[u] >> lane) & 1u) m[w * ns + o + __popc(bal[u] & lanemask_lt())] = x[u];
+        o += __popc(bal[u]);
+      }
+      __syncwarp();
+    }
+  }
+  int o = 0;
+  ROLLED for (int b = 0; b < n; b += 32 * U) {
+    uint64_t k[U];
+    uint32_t f[U], bal[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = b + 32 * u;
+      bal[u] = i < n ? S[i >> 5] : 0u;
+      const bool mine = (bal[u] >> lane) & 1u;
+      k[u] = mine ? key[i + lane] : 0ULL;
+      f[u] = mine ? info[i + lane] : 0u;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if ((bal[u] >> lane) & 1u) {
+        const int d = o + __popc(bal[u] & lanemask_lt());
+        key[d] = k[u];
+        info[d] = f[u];
+      }
+      o += __popc(bal[u]);
+    }
+    __syncwarp();
+  }
+  *stride_io = (int)ns;
+  return kept;
+}
+
+__device__ __noinline__ void emit_bits(int count, int K, uint32_t mw, const int32_t* lid) {
+  emit_words(s_blk.ctl, emit_dst(*s_blk.p), this_warp().gid, count, K, mw, lid);
+}
+
+// ---------------------------------------------------------------------------
+// Leaf sub-problems: at most 32 classes over at most 32 L vertices.  Lane i
+// holds class i's mask, key sum and count, lane b the key of L bit b, and a
+// level is four words (live, Q and P classes and L) that every lane knows;
+// lane d keeps level d's while a deeper one runs.  A push is then a handful of
+// ballots: the walk touches no memory at all.  Maximal bicliques are only
+// noted (their L), one per lane, and hashed 32 at a time, every lane its own.
+struct Leaf {
+  uint32_t m;  // this lane's class: mask
+  uint32_t cnt;
+  uint64_t key;
+  uint64_t lk;  // key of L bit `lane`
+  uint32_t A, Q, P, L;
+  uint32_t lim;  // classes the first level may push
+  uint32_t nR;   // R of the sub-problem's root biclique
+  uint64_t sR;
+};
+
+// Hashes the noted bicliques (one L per lane, `nb` of them): L's keys over its
+// bits, R as the classes of P0 covering it.
+__device__ __forceinline__ uint64_t leaf_flush(const Leaf& f, uint32_t P0, uint32_t L0,
+                                               uint32_t buf, int nb, int swapped) {
+  uint64_t sL = 0, sR = f.sR, nR = f.nR;
+  ROLLED for (uint32_t b = L0; b; b &= b - 1) {
+    const int i = __ffs(b) - 1;
+    const uint64_t k = __shfl_sync(kFull, f.lk, i);
+    if ((buf >> i) & 1u) sL += k;
+  }
+  ROLLED for (uint32_t b = P0; b; b &= b - 1) {
+    const int i = __ffs(b) - 1;
+    const uint32_t mi = __shfl_sync(kFull, f.m, i);
+    const uint64_t k = __shfl_sync(kFull, f.key, i);
+    const uint32_t c = __shfl_sync(kFull, f.cnt, i);
+    if ((mi & buf) == buf) {
+      sR += k;
+      nR += c;
+    }
+  }
+  return (int)lane_id() < nb ? biclique_hash_s(swapped, sL, (uint64_t)__popc(buf), sR, nR) : 0ULL;
+}
+
+// Hands the child (classes sel, of them p to push and q in Q, L = ln) of a
+// leaf sub-problem to an idle warp; all: every class of R of its push.
+__device__ __noinline__ bool leaf_export(uint32_t m, uint64_t key, uint32_t cnt,
+                                         uint64_t lk, const int32_t* lid, uint64_t sR, uint32_t nR,
+                                         uint32_t sel, uint32_t q, uint32_t p, uint32_t ln,
+                                         uint32_t all) {
+  Warp& W = this_warp();
+  const int lane = (int)lane_id();
+  const int n = __popc(sel), kn = __popc(ln);
+  if (!slot_fits(W, n, 1, cls_levels(kn, __popc(p))) || !should_export(W, __popc(p), kn))
+    return false;
+  int slot = lane == 0 ? slot_alloc_for(W, n, 1) : 0;
+  slot = __shfl_sync(kFull, slot, 0);
+  if (slot < 0) return false;
+  int32_t* sp = slot_ptr(W, slot);
+  const ClsList d = cls_list_at(reinterpret_cast<uint32_t*>(sp + kSlotList), n, 1);
+  if ((sel >> lane) & 1u) {
+    const int o = __popc(sel & lanemask_lt());
+    d.m[o] = m & ln;
+    d.key[o] = key;
+    d.info[o] = cnt | (((q >> lane) & 1u) ? kInfoQ : 0u) | (((p >> lane) & 1u) ? kInfoP : 0u);
+  }
+  reinterpret_cast<uint64_t*>(sp + kSlotLk)[lane] = lk;
+  if (s_blk.emit) sp[kSlotLid + lane] = lid[lane];
+  const bool r = (all >> lane) & 1u;
+  const uint64_t sR1 = warp_sum64(r ? key : 0ULL) + sR;
+  const uint32_t nR1 = __reduce_add_sync(kFull, r ? cnt : 0u) + nR;
+  if (lane == 0) {
+    sp[kSlotL] = (int32_t)ln;
+    slot_header(sp, 1, n, kn, sR1, nR1, W.gid);
+  }
+  if (slot_publish(slot, 0)) return true;
   if (lane == 0) slot_free(W, slot);
   __syncwarp();
   return false;
 }
 
-// ---------------------------------------------------------------------------
-// Tier 2: the DFS of IterProcess / finder_push / finder_pop on a bitmap
-// sub-problem.  Every level owns a contiguous record list: the candidates
-// that still meet the level's L and are neither absorbed nor retired
-// (MBEA's shrinking P and Q), copied with their masks so each pass is a
-// unit-stride sweep.  Level bounds live in the records: a deeper level only
-// changes its own copies, which is equivalent to GMBE's shared bound array
-// because a pop at a level re-derives every bound >= that level.  A child
-// list that does not fit the arena shares its parent's records (GMBE's
-// shared-array semantics for that pair of levels).  R of the push that
-// opened a level is carried on the stack: absorbed candidates leave the
-// lists but stay in every R below.
-//
-// finder_pop is not a pass of its own: a pop at a level is only remembered
-// (the candidate and the L vertices it leaves, `rem`), and its bound rule is
-// applied record by record by the next pass over the level, the scan for the
-// next candidate and that candidate's push, which write each header once.
-// A level that ends with a pop pending drops it: its records are discarded,
-// or (a list shared with the parent) every bound the pop would set is one
-// the parent's own pop re-derives.
-template <int K>
-__device__ void tier2_run(Warp& W, const T2Src& src) {
-  constexpr int RS = rec_stride(K);
-  const int lane = (int)lane_id();
-  const uint64_t* subkey = src.subkey;
-  const uint64_t* lkey = src.lkey;
-  uint32_t* arena = reinterpret_cast<uint32_t*>(W.A(W.sl.act));
-  const int actcap = W.sl.act_cap;
-  uint64_t* lrec = W.A64(W.sl.t2_rec);   // record list of each level
-  int32_t* ln = W.A(W.sl.t2_n);          // its length
-  int32_t* lcur = W.A(W.sl.t2_cur);      // scan position in it
-  int32_t* ltop = W.A(W.sl.t2_top);      // first free arena word above it
-  uint32_t* lmask = reinterpret_cast<uint32_t*>(W.A(W.sl.lmask));
-  uint64_t* rsum = W.A64(W.sl.r_sum);
-  uint32_t* rcnt = reinterpret_cast<uint32_t*>(W.A(W.sl.r_cnt));
-  const bool emitting = W.p.emit != nullptr;
-  const bool prune = W.p.prune != 0;
+// What a walk adds to its warp's totals, in registers.
+struct Tally {
+  unsigned long long hl;  // this lane's part of the hash sum
+  uint32_t cnt, nonmax;   // bicliques found, pushes rejected
+  uint32_t steps;
+  int swapped;
+  int share_floor;        // |P|*|L| from which a child may be shared out
+};
 
-  for (int q = lane; q < src.nsub; q += 32) {
-    uint32_t h = src.rec[(size_t)q * RS];
-    src.rec[(size_t)q * RS] = (h & ~0xffu) | kB8Free;
+// Walks a leaf sub-problem (lid: the internal U id of each L bit, for
+// emission); false if the launch is stopping.
+__device__ __forceinline__ bool leaf_run(Tally& y, const Leaf& f, const int32_t* const* lid) {
+  const int lane = (int)lane_id();
+  const bool prune = s_blk.prune != 0;
+  const uint32_t m = f.m, P0 = f.P;
+  uint32_t A = f.A, Q = f.Q, P = f.P, L = f.L, lim = f.lim;
+  uint32_t sA = 0, sQ = 0, sP = 0, sL = 0, buf = 0;
+  int depth = 0, nb = 0;
+  while (true) {
+    const uint32_t t = P & A & lim;
+    const bool stop = t == 0u && depth == 0;
+    if (nb == 32 || (stop && nb > 0)) {
+      y.hl += leaf_flush(f, P0, f.L, buf, nb, y.swapped);
+      nb = 0;
+    }
+    if (t == 0u) {
+      if (stop) return true;
+      --depth;
+      A = __shfl_sync(kFull, sA, depth);
+      Q = __shfl_sync(kFull, sQ, depth);
+      P = __shfl_sync(kFull, sP, depth);
+      L = __shfl_sync(kFull, sL, depth);
+      if (depth == 0) lim = f.lim;
+      continue;
+    }
+    if ((++y.steps & 4095u) == 0u && must_stop()) return false;
+    // ---- push (finder_push) of class c, and what its pop leaves ----
+    const int c = __ffs(t) - 1;
+    const uint32_t cb = t & (0u - t);
+    const uint32_t mc = __shfl_sync(kFull, m, c);
+    const uint32_t ln = L & mc;
+    const uint32_t x = m & ln;
+    const uint32_t all = __ballot_sync(kFull, x == ln);
+    const uint32_t meet = __ballot_sync(kFull, x != 0u);
+    const uint32_t out = __ballot_sync(kFull, (m & L & ~mc) != 0u);
+    const uint32_t cov = all & A;
+    const uint32_t sel = A & meet & ~cov;
+    const bool bad = (cov & Q) != 0u;
+    if (prune) A &= out | cb;  // retired: nothing outside the popped one's neighbourhood
+    P &= ~cb;
+    Q |= cb;
+    if (bad) {
+      ++y.nonmax;
+      continue;
+    }
+    ++y.cnt;
+    if (lane == nb) buf = ln;
+    ++nb;
+    if (s_blk.emit) emit_bits(__popc(ln), 1, ln, *lid);
+    const uint32_t p = sel & P;
+    const int kn = __popc(ln);
+    if (p != 0u && kn > 1) {
+      // (a class of an upper level's R covers ln too: all & P0 is all of R)
+      if (__popc(p) * kn >= y.share_floor &&
+          leaf_export(m, f.key, f.cnt, f.lk, *lid, f.sR, f.nR, sel, sel & Q, p, ln, all & P0))
+        continue;
+      if (lane == depth) {
+        sA = A;
+        sQ = Q;
+        sP = P;
+        sL = L;
+      }
+      ++depth;
+      A = sel;
+      Q &= sel;
+      P = p;
+      L = ln;
+      lim = kFull;
+    }
   }
-  if (lane == 0) {
-    lrec[0] = reinterpret_cast<uint64_t>(src.rec);
-    ln[0] = src.nsub;
-    lcur[0] = src.nq;
-    ltop[0] = 0;
-    rsum[0] = src.sR0;
-    rcnt[0] = src.nR0;
-  }
-  if (lane < K) {
-    uint32_t v = 0;
+}
+
+// ---------------------------------------------------------------------------
+// The walk over larger sub-problems: the DFS of IterProcess / finder_push /
+// finder_pop, a level at a time.  One sweep over a level's live classes does a
+// push and its pop together: which classes cover the new L (absorbed, or a Q
+// one that makes the push non-maximal), which go to the child, and which the
+// pop retires.  A child that comes down to 32 classes over 32 L vertices is a
+// leaf; a larger one gets a list of its own, its masks cut down to the L
+// vertices left and merged again, or, when the arena has no room for it, works
+// on its parent's list with live, Q and P bits of its own.
+struct ClsCur {             // the level being walked, in shared memory
+  ClsList l;
+  const uint64_t* lk;
+  const int32_t* lid;
+  uint32_t* A;              // live bits; Q and P bits follow, nwp words each
+  uint32_t *S, *C;          // bits of the child being made, and of the covering classes
+  ClsFrame* fr;
+  uint32_t *top, *stop;     // first free word of the arena, and of the shared one
+  const int32_t* leaf_lid;  // of the leaf being walked (emission)
+  uint64_t sR;
+  uint32_t nR;
+  int nw, nwp;              // words of A, Q, P
+  int nend;
+};
+static_assert(sizeof(ClsCur) <= 40 * 4, "shared memory layout");
+__device__ __forceinline__ ClsCur& this_cur() {
+  return *reinterpret_cast<ClsCur*>(this_smem() + kSmCur);
+}
+
+// Visits four words of classes at a time, those whose bit is set in `live`
+// (word sb + j for bit j): word(w, x) is called for each of the K mask words
+// with x[0..3], this lane's class of each of the four, then done(j) with the
+// four's numbers (fewer left: the last one again).  Four loads per lane are in
+// flight at once: little else hides a warp's latency.
+template <typename Word, typename Done>
+__device__ __forceinline__ void cls_words4(const uint32_t* m, int st, int K, int sb, unsigned live,
+                                           Word word, Done done) {
+  const int lane = (int)lane_id();
+  while (live) {
+    int j[4], i[4];
 #pragma unroll
-    for (int w = 0; w < K; ++w)
-      if (w == lane) v = src.L0[w];
-    lmask[lane] = v;
+    for (int u = 0; u < 4; ++u) {
+      j[u] = live ? __ffs(live) - 1 : j[u > 0 ? u - 1 : 0];
+      live &= live - 1;
+      i[u] = (sb + j[u]) * 32 + lane;
+    }
+    const uint32_t* p = m;
+    ROLLED for (int w = 0; w < K; ++w, p += st) {
+      uint32_t x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = p[i[u]];
+      word(w, x);
+    }
+    done(j);
+  }
+}
+
+struct SweepOut {
+  bool nm;            // a Q class covers the new L
+  int nsel, nselp;    // classes of the child, P classes among them
+};
+
+// One push's sweep over the level's live classes.  lnw and rmw (lane w: word
+// w) are the new L and the L vertices it leaves; cpos is the pushed class,
+// which stays live, and is in Q and no longer in P from here on.  Bits C: the
+// classes covering the new L; bits S: the child's.
+__device__ __forceinline__ SweepOut cls_sweep(const ClsCur& c, uint32_t lnw, uint32_t rmw,
+                                              int cpos) {
+  const int lane = (int)lane_id();
+  const int K = c.l.K, st = c.l.stride, nw = c.nw, nwp = c.nwp;
+  const uint32_t* m = c.l.m;
+  uint32_t* A = c.A;
+  const bool prune = s_blk.prune != 0;
+  uint32_t bad = 0u, nsel = 0u, nselp = 0u;
+  ROLLED for (int sb = 0; sb < nw; sb += 32) {
+    const int wl = sb + lane;
+    const bool in = wl < nw;
+    const uint32_t aw = in ? A[wl] : 0u;
+    uint32_t qw = in ? A[nwp + wl] : 0u;
+    uint32_t pw = in ? A[2 * nwp + wl] : 0u;
+    uint32_t sel = 0u, out = 0u, cv = 0u;
+    uint32_t miss[4] = {0u, 0u, 0u, 0u}, meet[4] = {0u, 0u, 0u, 0u}, leave[4] = {0u, 0u, 0u, 0u};
+    cls_words4(
+        m, st, K, sb, __ballot_sync(kFull, aw != 0u),
+        [&](int w, const uint32_t* x) {
+          const uint32_t ln = __shfl_sync(kFull, lnw, w), rm = __shfl_sync(kFull, rmw, w);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            miss[u] |= ln & ~x[u];
+            meet[u] |= ln & x[u];
+            leave[u] |= rm & x[u];
+          }
+        },
+        [&](const int* j) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t b0 = __ballot_sync(kFull, miss[u] == 0u);
+            const uint32_t b1 = __ballot_sync(kFull, meet[u] != 0u);
+            const uint32_t b2 = __ballot_sync(kFull, leave[u] != 0u);
+            miss[u] = meet[u] = leave[u] = 0u;
+            if (lane == j[u]) {
+              cv = b0;
+              sel = b1;
+              out = b2;
+            }
+          }
+        });
+    cv &= aw;
+    sel &= aw & ~cv;
+    bad |= cv & qw;
+    if (in) {
+      uint32_t an = prune ? aw & out : aw;
+      if (wl == (cpos >> 5)) {
+        const uint32_t bit = 1u << (cpos & 31);
+        an |= bit;
+        qw |= bit;
+        pw &= ~bit;
+        A[nwp + wl] = qw;
+        A[2 * nwp + wl] = pw;
+      }
+      if (prune) A[wl] = an;
+      c.S[wl] = sel;
+      c.C[wl] = cv;
+    }
+    nsel += __popc(sel);
+    nselp += __popc(sel & pw);
+  }
+  SweepOut o;
+  o.nm = __any_sync(kFull, bad != 0u);
+  o.nsel = (int)__reduce_add_sync(kFull, nsel);
+  o.nselp = (int)__reduce_add_sync(kFull, nselp);
+  return o;
+}
+
+// A mask's bits inside ln moved together: bit r of the result is the r-th set
+// bit of ln (lane w of lnw: word w, of base: the number of set bits below it).
+// Word 0 of the result; the others, up to four, in hi when asked for.
+template <bool kHi>
+__device__ __forceinline__ uint32_t cls_pack(const uint32_t* m, int stride, int K, uint32_t lnw,
+                                             uint32_t base, int i, bool valid, uint32_t* hi) {
+  uint32_t lo = 0u;
+  if (kHi) hi[0] = hi[1] = hi[2] = 0u;
+  ROLLED for (int w = 0; w < K; ++w) {
+    const uint32_t lw = __shfl_sync(kFull, lnw, w);
+    const uint32_t bw = __shfl_sync(kFull, base, w);
+    if (lw == 0u) continue;
+    uint32_t x = valid ? m[(size_t)w * stride + i] & lw : 0u;
+    ROLLED for (; x; x &= x - 1) {
+      const uint32_t r = bw + __popc(lw & ((x & (0u - x)) - 1u));
+      const uint32_t bit = 1u << (r & 31);
+      if (!kHi) {
+        lo |= bit;
+      } else {
+        const uint32_t ww = r >> 5;
+        lo |= ww == 0u ? bit : 0u;
+        hi[0] |= ww == 1u ? bit : 0u;
+        hi[1] |= ww == 2u ? bit : 0u;
+        hi[2] |= ww == 3u ? bit : 0u;
+      }
+    }
+  }
+  return lo;
+}
+
+// Keys (and ids) of the L bits kept in ln, moved together.
+__device__ __noinline__ void cls_pack_keys(const uint64_t* slk, const int32_t* slid, int K,
+                                           uint32_t lnw, uint32_t base, uint64_t* lk,
+                                           int32_t* lid) {
+  const int lane = (int)lane_id();
+  ROLLED for (int w = 0; w < K; ++w) {
+    const uint32_t lw = __shfl_sync(kFull, lnw, w);
+    const uint32_t bw = __shfl_sync(kFull, base, w);
+    if ((lw >> lane) & 1u) {
+      const uint32_t r = bw + __popc(lw & lanemask_lt());
+      lk[r] = slk[w * 32 + lane];
+      if (lid) lid[r] = slid[w * 32 + lane];
+    }
   }
   __syncwarp();
-  int level = 1;
-  unsigned steps = 0;
-  // The pending pop at `level`: its candidate (-1: none) and the L vertices
-  // of the level it does not meet.
-  int pcp = -1;
-  uint32_t prem[K];
-#pragma unroll
-  for (int w = 0; w < K; ++w) prem[w] = 0u;
-  // A record's bound after the pending pop (finder_pop: a bound >= level is
-  // re-derived, FREE if the record meets rem or is the popped one, else
-  // level - 1; without pruning always FREE).
-  auto popped = [&](int q, uint32_t b, const uint32_t* m) -> uint32_t {
-    if (pcp < 0 || (int)b < level) return b;
-    if (!prune || q == pcp) return kB8Free;
-    uint32_t any = 0;
-#pragma unroll
-    for (int w = 0; w < K; ++w) any |= m[w] & prem[w];
-    return any ? kB8Free : (uint32_t)(level - 1);
-  };
-  while (level != 0) {
-    if ((++steps & 4095u) == 0u && must_stop(W)) return;
-    uint32_t* R = reinterpret_cast<uint32_t*>(lrec[level - 1]);
-    const int n = ln[level - 1];
-    uint32_t Lm[K];
-#pragma unroll
-    for (int w = 0; w < K; ++w) Lm[w] = lmask[(level - 1) * K + w];
-    int cp = -1;
-    const int e = level == 1 ? src.nend : n;  // the first level may push a part only
-    for (int b0 = lcur[level - 1]; b0 < e; b0 += 32) {
-      int q = b0 + lane;
-      bool ok = false;
-      if (q < e) {
-        uint32_t h, m[K];
-        if constexpr (K == 1) {
-          // One 8-byte load per record (lists start 8-byte aligned, records
-          // are two words): half the load instructions and L1 wavefronts.
-          const uint2 hm = reinterpret_cast<const uint2*>(R)[q];
-          h = hm.x;
-          m[0] = hm.y;
-        } else if constexpr (K == 2) {
-          const uint4 hm = reinterpret_cast<const uint4*>(R)[q];  // padded to 4 words
-          h = hm.x;
-          m[0] = hm.y;
-          m[1] = hm.z;
-        } else {
-          const uint32_t* r = R + (size_t)q * RS;
-          h = r[0];
-#pragma unroll
-          for (int w = 0; w < K; ++w) m[w] = r[1 + w];
-        }
-        if ((int)popped(q, h & 0xffu, m) > level - 1) {
-          uint32_t any = 0;
-#pragma unroll
-          for (int w = 0; w < K; ++w) any |= m[w] & Lm[w];
-          ok = any != 0;
-        }
+}
+
+// Writes the child's classes (selection bits S) to list d: masks cut down to
+// ln, moved together to dK words when that is fewer (at most four then).
+__device__ __noinline__ void cls_copy_child(uint32_t lnw, uint32_t base, uint32_t* dbase, int dn,
+                                            int dK) {
+  const ClsCur& c = this_cur();
+  const int lane = (int)lane_id();
+  const ClsList d = cls_list_at(dbase, dn, dK);
+  const ClsList l = c.l;
+  const uint32_t *Q = c.A + c.nwp, *P = Q + c.nwp;
+  const bool pack = dK < l.K;
+  int o = 0;
+  ROLLED for (int b0 = 0; b0 < c.nw; b0 += 32) {
+    const uint32_t sl = b0 + lane < c.nw ? c.S[b0 + lane] : 0u;
+    ROLLED for (unsigned todo = __ballot_sync(kFull, sl != 0u); todo; todo &= todo - 1) {
+      const int j = __ffs(todo) - 1;
+      const uint32_t sw = __shfl_sync(kFull, sl, j);
+      const int b = b0 + j, i = b * 32 + lane;
+      const bool mine = (sw >> lane) & 1u;
+      const int t = o + __popc(sw & lanemask_lt());
+      if (mine) {
+        d.key[t] = l.key[i];
+        d.info[t] = (l.info[i] & kInfoCnt) | (((Q[b] >> lane) & 1u) ? kInfoQ : 0u) |
+                    (((P[b] >> lane) & 1u) ? kInfoP : 0u);
       }
-      unsigned bal = __ballot_sync(kFull, ok);
-      if (bal) {
-        cp = b0 + __ffs(bal) - 1;
-        break;
-      }
-    }
-    if (cp >= 0) {
-      // ---- push (finder_push) ----
-      W.pushes += 1ULL << 32;
-      uint32_t Ln[K];
-      int kn = 0;
+      if (pack) {
+        uint32_t hi[3];
+        const uint32_t lo = cls_pack<true>(l.m, l.stride, l.K, lnw, base, i, mine, hi);
+        if (mine) {
+          d.m[t] = lo;
 #pragma unroll
-      for (int w = 0; w < K; ++w) {
-        Ln[w] = Lm[w] & R[(size_t)cp * RS + 1 + w];
-        kn += __popc(Ln[w]);
-      }
-      const int ctop = ltop[level - 1];
-      const bool fits = ctop + n * RS <= actcap;
-      uint32_t* child = arena + ctop;
-      bool ism = true;
-      uint64_t sR = 0;
-      unsigned long long nR = 0;
-      int nchild = 0, nbefore = 0;
-      // The pass is bound by load latency: each lane loads U records before
-      // any of them is used, so U loads per lane are in flight at once.
-      constexpr int U = K <= 2 ? 4 : 2;
-      for (int b0 = 0; b0 < n; b0 += 32 * U) {
-        uint32_t hu[U], mu[U][K];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int q = b0 + u * 32 + lane;
-          hu[u] = 0u;
-#pragma unroll
-          for (int w = 0; w < K; ++w) mu[u][w] = 0u;
-          if (q < n) {
-            if constexpr (K == 1) {
-              const uint2 hm = reinterpret_cast<const uint2*>(R)[q];
-              hu[u] = hm.x;
-              mu[u][0] = hm.y;
-            } else if constexpr (K == 2) {
-              const uint4 hm = reinterpret_cast<const uint4*>(R)[q];
-              hu[u] = hm.x;
-              mu[u][0] = hm.y;
-              mu[u][1] = hm.z;
-            } else {
-              const uint32_t* r = R + (size_t)q * RS;
-              hu[u] = r[0];
-#pragma unroll
-              for (int w = 0; w < K; ++w) mu[u][w] = r[1 + w];
-            }
-          }
+          for (int w = 1; w < 4; ++w)
+            if (w < dK) d.m[(size_t)w * d.stride + t] = hi[w - 1];
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int q = b0 + u * 32 + lane;
-          const uint32_t h = hu[u];
-          bool keep = false;
-          if (q < n) {
-            bool cover = true, meet = false;
-#pragma unroll
-            for (int w = 0; w < K; ++w) {
-              uint32_t x = mu[u][w] & Ln[w];
-              cover &= x == Ln[w];
-              meet |= x != 0;
-            }
-            const uint32_t b0h = h & 0xffu;
-            const int b = (int)popped(q, b0h, mu[u]);
-            uint32_t nb = (uint32_t)b;
-            if (cover) {
-              sR += subkey[h >> 8];
-              ++nR;
-              if (q < cp && b >= level) ism = false;
-              else if (b > level) nb = (uint32_t)level;
-            } else {
-              keep = meet && b > level;
-            }
-            if (nb != b0h) R[(size_t)q * RS] = (h & ~0xffu) | nb;
-          }
-          unsigned bal = __ballot_sync(kFull, keep);
-          if (fits && keep) {
-            const int ci = nchild + __popc(bal & lanemask_lt());
-            if constexpr (K == 1) {
-              reinterpret_cast<uint2*>(child)[ci] = make_uint2((h & ~0xffu) | kB8Free, mu[u][0]);
-            } else if constexpr (K == 2) {
-              reinterpret_cast<uint4*>(child)[ci] =
-                  make_uint4((h & ~0xffu) | kB8Free, mu[u][0], mu[u][1], 0u);
-            } else {
-              uint32_t* c = child + (size_t)ci * RS;
-              c[0] = (h & ~0xffu) | kB8Free;
-#pragma unroll
-              for (int w = 0; w < K; ++w) c[1 + w] = mu[u][w];
-            }
-          }
-          nchild += __popc(bal);
-          nbefore += __popc(__ballot_sync(kFull, keep && q < cp));
-        }
-      }
-      pcp = -1;  // applied by this pass
-      ism = __all_sync(kFull, ism);
-      sR = warp_sum(sR) + rsum[level - 1];
-      nR = warp_sum(nR) + rcnt[level - 1];
-      if (ism) {
-        uint64_t sL = 0;
-#pragma unroll
-        for (int w = 0; w < K; ++w)
-          if ((Ln[w] >> lane) & 1u) sL += lkey[w * 32 + lane];
-        sL = warp_sum(sL);
-        W.cnt += 1;
-        W.hash += biclique_hash(*W.gp, sL, (uint64_t)kn, sR, nR);
-        if (emitting)
-          emit_mask(W.ctl, emit_dst(W.p), W.gid, kn, K, Ln[0], K > 1 ? Ln[1 % K] : 0u,
-                    K > 2 ? Ln[2 % K] : 0u, K > 3 ? Ln[3 % K] : 0u, src.lid);
       } else {
-        W.nonmax += 1;
+        ROLLED for (int w = 0; w < l.K; ++w) {
+          const uint32_t lw = __shfl_sync(kFull, lnw, w);
+          if (mine) d.m[(size_t)w * d.stride + t] = l.m[(size_t)w * l.stride + i] & lw;
+        }
       }
-      __syncwarp();
-      // A big enough child goes to an idle warp instead, at any depth, so a
-      // subtree that started inline can still be shared once warps run out of
-      // work (the state after the pop below does not depend on the child).
-      bool exported = false;
-      if (ism && kn > 1 && nchild > 0 && fits)
-        exported = t2_try_export<K>(W, src, child, nchild, nbefore, Ln, kn, sR, nR);
-      if (ism && kn > 1 && nchild > 0 && !exported) {
-        if (lane == 0) {
-          lcur[level - 1] = cp;
-          rsum[level] = sR;
-          rcnt[level] = (uint32_t)nR;
-          if (fits) {
-            lrec[level] = reinterpret_cast<uint64_t>(child);
-            ln[level] = nchild;
-            lcur[level] = nbefore;  // the child takes candidates after cp
-            ltop[level] = ctop + nchild * RS;
-          } else {
-            lrec[level] = lrec[level - 1];
-            ln[level] = n;
-            lcur[level] = cp + 1;
-            ltop[level] = ctop;
+      o += __popc(sw);
+    }
+  }
+  __syncwarp();
+}
+
+// Hands the child just selected to an idle warp.
+__device__ __noinline__ bool cls_export(uint32_t lnw, uint32_t base, int nsel, int nselp, int kn,
+                                        uint64_t sR, uint32_t nR) {
+  Warp& W = this_warp();
+  const ClsCur& c = this_cur();
+  const int lane = (int)lane_id();
+  const int kc = words_k(kn);
+  const int cK = c.l.K, K = kc <= kKMax && kc < cK ? kc : cK;
+  if (!slot_fits(W, nsel, K, cls_levels(kn, nselp)) || !should_export(W, nselp, kn)) return false;
+  int slot = lane == 0 ? slot_alloc_for(W, nsel, K) : 0;
+  slot = __shfl_sync(kFull, slot, 0);
+  if (slot < 0) return false;
+  int32_t* sp = slot_ptr(W, slot);
+  cls_copy_child(lnw, base, reinterpret_cast<uint32_t*>(sp + kSlotList), nsel, K);
+  uint64_t* lk = reinterpret_cast<uint64_t*>(sp + kSlotLk);
+  int32_t* lid = s_blk.emit ? sp + kSlotLid : nullptr;
+  if (K < cK) {
+    cls_pack_keys(c.lk, c.lid, cK, lnw, base, lk, lid);
+  } else {
+    ROLLED for (int b = lane; b < 32 * K; b += 32) {
+      lk[b] = c.lk[b];
+      if (lid) lid[b] = c.lid[b];
+    }
+  }
+  if (lane < K) sp[kSlotL + lane] = K < cK ? (int32_t)first_bits(kn, lane) : (int32_t)lnw;
+  if (lane == 0) slot_header(sp, K, nsel, kn, sR, nR, W.gid);
+  if (slot_publish(slot, 0)) return true;
+  if (lane == 0) slot_free(W, slot);
+  __syncwarp();
+  return false;
+}
+
+// The leaf of a list of at most 32 one-word classes.
+__device__ __forceinline__ void leaf_of_list(const ClsList& l, uint32_t L, int nend,
+                                             const uint64_t* lk, uint64_t sR, uint32_t nR,
+                                             Leaf& f) {
+  const int lane = (int)lane_id();
+  const bool in = lane < l.n;
+  const uint32_t info = in ? l.info[lane] : 0u;
+  f.m = in ? l.m[lane] : 0u;
+  f.key = in ? l.key[lane] : 0ULL;
+  f.cnt = info & kInfoCnt;
+  f.lk = (L >> lane) & 1u ? lk[lane] : 0ULL;
+  f.A = first_bits(l.n, 0);
+  f.Q = __ballot_sync(kFull, (info & kInfoQ) != 0u);
+  f.P = __ballot_sync(kFull, (info & kInfoP) != 0u);
+  f.L = L;
+  f.lim = first_bits(nend, 0);
+  f.sR = sR;
+  f.nR = nR;
+}
+
+// The indices of the selected classes, in order, into g.
+__device__ __forceinline__ void cls_indices(const uint32_t* S, int nw, uint32_t* g) {
+  int o = 0;
+  ROLLED for (int b0 = 0; b0 < nw; b0 += 32) {
+    const int w = b0 + (int)lane_id();
+    uint32_t s = w < nw ? S[w] : 0u;
+    int t;
+    int at = o + excl_scan(__popc(s), &t);
+    ROLLED for (; s; s &= s - 1) g[at++] = (uint32_t)(w * 32 + __ffs(s) - 1);
+    o += t;
+  }
+  __syncwarp();
+}
+
+// A child of 33 to kChildMax selected classes over at most 32 L vertices, its
+// classes merged on the way (pruning on): the table (one entry per mask, found
+// by probing) keeps each mask's leader and the sums, and the leaders, in order,
+// are the child's classes; their number is returned, they themselves go to lm
+// (masks), key and info.
+__device__ __noinline__ int cls_child(uint32_t lnw, uint32_t base, int nsel, uint32_t* lm,
+                                      uint64_t* key, uint32_t* info) {
+  const ClsCur& c = this_cur();
+  const int lane = (int)lane_id();
+  const MergeTab t = this_tab();
+  uint32_t* g = this_smem() + kSmIdx;
+  const bool merge = s_blk.prune != 0;
+  const ClsList l = c.l;
+  const uint32_t *Qw = c.A + c.nwp, *Pw = Qw + c.nwp;
+  cls_indices(c.S, c.nw, g);
+  const uint32_t ln0 = __shfl_sync(kFull, lnw, 0);
+  int n = 0;
+  // Without merging every class is its own leader: one pass.
+  ROLLED for (int pass = merge ? 0 : 1; pass < 2; ++pass) {
+    ROLLED for (int b = 0; b < nsel; b += 32) {
+      const int at = b + lane;
+      const bool in = at < nsel;
+      uint32_t x = 0u, f = 0u, h = 0u;
+      uint64_t k = 0ULL;
+      const int i = in ? (int)g[at] : 0;  // the class, or (second pass) its entry
+      if (pass == 0 || !merge) {
+        // (one-word masks keep their bits where they are)
+        x = l.K == 1 ? (in ? l.m[i] & ln0 : 0u)
+                     : cls_pack<false>(l.m, l.stride, l.K, lnw, base, i, in, nullptr);
+        if (in) {
+          f = (((Qw[i >> 5] >> (i & 31)) & 1u) << 31) | (((Pw[i >> 5] >> (i & 31)) & 1u) << 30);
+          if (f & kInfoP) {
+            f |= l.info[i] & kInfoCnt;
+            k = l.key[i];
           }
         }
-        if (lane < K) {
-          uint32_t v = 0;
-#pragma unroll
-          for (int w = 0; w < K; ++w)
-            if (w == lane) v = Ln[w];
-          lmask[level * K + lane] = v;
-        }
-        __syncwarp();
-        ++level;
-        continue;
       }
-      if (lane == 0) lcur[level - 1] = cp + 1;
-    } else {
-      --level;  // the ended level's pending pop (if any) is dropped
-      if (level == 0) break;
-      cp = lcur[level - 1];
-      __syncwarp();
-      if (lane == 0) lcur[level - 1] = cp + 1;
-    }
-    // ---- pop (finder_pop) of the candidate at position cp of `level`:
-    // remembered, applied by the next pass over the level ----
-    {
-      const uint32_t* R2 = reinterpret_cast<const uint32_t*>(lrec[level - 1]);
-      pcp = cp;
-#pragma unroll
-      for (int w = 0; w < K; ++w)
-        prem[w] = lmask[(level - 1) * K + w] & ~R2[(size_t)cp * RS + 1 + w];
+      if (pass == 0) {
+        if (x) {
+          h = hash_mix(x) >> 24;
+          while (true) {
+            const uint32_t old = atomicCAS(&t.mask[h], 0u, x);
+            if (old == 0u || old == x) break;
+            h = (h + 1) & (kSlots - 1);
+          }
+          // the earlier the larger, P classes first
+          const uint32_t rank = ((f & kInfoP) ? 0x8000u : 0x4000u) - (uint32_t)at;
+          atomicMax(&t.lead[h], rank);
+          merge_add(t, h, k, f);
+          g[at] = h;
+        }
+      } else {
+        bool is = x != 0u;
+        if (merge && in) {
+          h = (uint32_t)i;
+          const uint32_t v = t.lead[h];
+          is = (v > 0x4000u ? 0x8000u : 0x4000u) - v == (uint32_t)at;
+          if (is) {
+            x = t.mask[h];
+            f = t.info[h];
+            k = (uint64_t)t.lo[h] | ((uint64_t)t.hi[h] << 32);
+          }
+        }
+        const unsigned bal = __ballot_sync(kFull, is);
+        if (is) {
+          const int r = n + __popc(bal & lanemask_lt());
+          lm[r] = x;
+          key[r] = k;
+          info[r] = f;
+        }
+        n += __popc(bal);
+      }
     }
     __syncwarp();
   }
-}
-
-__device__ void tier2_dispatch(Warp& W, const T2Src& src, int words) {
-  uint64_t t0 = globaltimer_ns();
-  if (words <= 1) tier2_run<1>(W, src);
-  else if (words <= 2) tier2_run<2>(W, src);
-  else tier2_run<4>(W, src);
-  W.ns_t2 += globaltimer_ns() - t0;
-  W.n_t2 += 1;
-}
-
-__device__ __forceinline__ int words_k(int n) {
-  int w = (n + 31) >> 5;
-  return w <= 1 ? 1 : (w <= 2 ? 2 : 4);
-}
-
-__device__ __forceinline__ void full_mask(uint32_t* L0, int n) {
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    int bits = n - 32 * w;
-    L0[w] = bits >= 32 ? 0xffffffffu : (bits <= 0 ? 0u : ((1u << bits) - 1u));
+  if (merge) {
+    ROLLED for (int at = lane; at < nsel; at += 32) {
+      const uint32_t h = g[at];
+      t.mask[h] = t.lead[h] = t.lo[h] = t.hi[h] = t.info[h] = 0u;
+    }
   }
+  __syncwarp();
+  return n;
 }
 
-// Sub-problem built in the warp's own scratch over n L vertices (all bits).
-__device__ void tier2(Warp& W, int n, int nsub, int nq, int nend, uint64_t sR0, uint64_t nR0) {
-  T2Src src;
-  src.rec = reinterpret_cast<uint32_t*>(W.A(W.sl.masks));
-  src.subkey = W.A64(W.sl.sub_v);
-  src.lkey = W.A64(W.sl.lkey);
-  src.lid = W.A(W.sl.lid);
-  full_mask(src.L0, n);
-  src.nsub = nsub;
-  src.nq = nq;
-  src.nend = nend;
-  src.sR0 = sR0;
-  src.nR0 = (uint32_t)nR0;
-  tier2_dispatch(W, src, words_k(n));
+// A level of its own for a list (masks at l.m): live, Q and P bits and a frame.
+__device__ __noinline__ void cls_enter(ClsList l, uint32_t L, int nend, const uint64_t* lk,
+                                       const int32_t* lid, uint64_t sR, uint32_t nR,
+                                       uint32_t* top, uint32_t* stop, bool own_bits) {
+  ClsCur& c = this_cur();
+  const int lane = (int)lane_id();
+  const uint32_t* send = this_smem() + kSmemWords;
+  ClsFrame* fr = reinterpret_cast<ClsFrame*>(top);
+  const int nw = (l.n + 31) >> 5, nwp = (nw + 1) & ~1;
+  uint32_t* Lw = top + kFrameWords;
+  top = Lw + ((l.K + 1) & ~1);
+  uint32_t* A;
+  if (3 * nwp <= send - stop) {
+    A = stop;
+    stop += 3 * nwp;
+  } else {
+    A = top;
+    top += 3 * nwp;
+  }
+  uint32_t *Q = A + nwp, *P = Q + nwp;
+  if (own_bits) {  // a fresh list: everything is live, Q and P as the info words say
+    ROLLED for (int b = 0; b < nw; ++b) {
+      const int i = b * 32 + lane;
+      const uint32_t f = i < l.n ? l.info[i] : 0u;
+      const uint32_t q = __ballot_sync(kFull, (f & kInfoQ) != 0u);
+      const uint32_t p = __ballot_sync(kFull, (f & kInfoP) != 0u);
+      if (lane == 0) {
+        A[b] = first_bits(l.n, b);
+        Q[b] = q;
+        P[b] = p;
+      }
+    }
+    // The masks too, when there is room.
+    const int words = l.K * l.stride;
+    if (words <= send - stop && (l.m < this_smem() || l.m >= send)) {
+      ROLLED for (int i = lane; i < words; i += 32) stop[i] = l.m[i];
+      l.m = stop;
+      stop += words;
+    }
+  } else {  // the parent's list: the selected classes
+    const uint32_t *S = c.S, *Qp = c.A + c.nwp, *Pp = Qp + c.nwp;
+    ROLLED for (int b = lane; b < nw; b += 32) {
+      const uint32_t s = S[b];
+      A[b] = s;
+      Q[b] = Qp[b] & s;
+      P[b] = Pp[b] & s;
+    }
+  }
+  if (lane < l.K) Lw[lane] = L;
+  ClsFrame* prev = c.fr;
+  __syncwarp();
+  if (lane == 0) {
+    fr->l = l;
+    fr->lk = lk;
+    fr->lid = lid;
+    fr->sR = sR;
+    fr->prev = prev;
+    fr->A = A;
+    fr->top = top;
+    fr->stop = stop;
+    fr->nR = nR;
+    fr->nend = nend;
+    fr->curw = 0;
+    c.l = l;
+    c.lk = lk;
+    c.lid = lid;
+    c.A = A;
+    c.fr = fr;
+    c.top = top;
+    c.stop = stop;
+    c.nw = nw;
+    c.nwp = nwp;
+    c.sR = sR;
+    c.nR = nR;
+    c.nend = nend;
+  }
+  __syncwarp();
+}
+
+// Back to the level above (false: there is none); its L in L (lane w: word w),
+// and where its scan stood in curw.
+__device__ __forceinline__ bool cls_leave(ClsCur& c, uint32_t& L, int& curw) {
+  const int lane = (int)lane_id();
+  const ClsFrame* fr = c.fr->prev;
+  if (!fr) return false;
+  __syncwarp();
+  const int K = fr->l.K;
+  L = lane < K ? (reinterpret_cast<const uint32_t*>(fr) + kFrameWords)[lane] : 0u;
+  curw = fr->curw;
+  if (lane == 0) {
+    c.l = fr->l;
+    c.lk = fr->lk;
+    c.lid = fr->lid;
+    c.nw = (fr->l.n + 31) >> 5;
+    c.nwp = (c.nw + 1) & ~1;
+    c.A = fr->A;
+    c.fr = const_cast<ClsFrame*>(fr);
+    c.top = fr->top;
+    c.stop = fr->stop;
+    c.sR = fr->sR;
+    c.nR = fr->nR;
+    c.nend = fr->nend;
+  }
+  __syncwarp();
+  return true;
+}
+
+// Starts a sub-problem: merges its list, sets up the first level.  True if the
+// list came down to a leaf, left as l.
+__device__ __noinline__ bool cls_begin(ClsList* lp, uint32_t L, int* nend, const uint64_t* lk,
+                                       const int32_t* lid, uint64_t sR0, uint32_t nR0,
+                                       uint32_t* top) {
+  ClsCur& c = this_cur();
+  uint32_t* sm = this_smem();
+  ClsList l = *lp;
+  uint32_t* S = top;
+  uint32_t* C = top + 2 * ((l.n + 63) >> 6);
+  top += 4 * ((l.n + 63) >> 6);
+  if (s_blk.prune && l.n > 32) l.n = cls_merge(l.m, l.key, l.info, l.n, l.K, &l.stride, S, nend);
+  *lp = l;
+  if (l.n <= 32 && l.K == 1) return true;
+  // The two bit strings a push makes go to the shared arena.
+  uint32_t* stop = sm + kSmArena;
+  const int nwp = (((l.n + 31) >> 5) + 1) & ~1;
+  if (2 * nwp <= sm + kSmemWords - stop) {
+    S = stop;
+    C = stop + nwp;
+    stop += 2 * nwp;
+  }
+  __syncwarp();
+  if (lane_id() == 0) {
+    c.fr = nullptr;
+    c.S = S;
+    c.C = C;
+  }
+  __syncwarp();
+  cls_enter(l, L, *nend, lk, lid, sR0, nR0, top, stop, true);
+  return false;
+}
+
+// A maximal push's biclique: R (the covering classes, all of them live P ones)
+// into sR and nR, its hash returned.
+__device__ __forceinline__ uint64_t cls_biclique(const ClsCur& c, uint32_t lnw, int kn, int swapped,
+                                                 uint64_t& sR, uint32_t& nR) {
+  const int lane = (int)lane_id();
+  sR = 0;
+  nR = 0;
+  uint64_t sL = 0;
+  const uint32_t* C = c.C;
+  ROLLED for (int w = lane; w < c.nw; w += 32)
+    ROLLED for (uint32_t b = C[w]; b; b &= b - 1) {
+      const int i = w * 32 + __ffs(b) - 1;
+      sR += c.l.key[i];
+      nR += c.l.info[i] & kInfoCnt;
+    }
+  const uint64_t* lk = c.lk;
+  ROLLED for (int w = 0; w < c.l.K; ++w)
+    if ((__shfl_sync(kFull, lnw, w) >> lane) & 1u) sL += lk[w * 32 + lane];
+  sR = warp_sum64(sR) + c.sR;
+  nR = __reduce_add_sync(kFull, nR) + c.nR;
+  sL = warp_sum64(sL);
+  return biclique_hash_s(swapped, sL, (uint64_t)kn, sR, (uint64_t)nR);
+}
+
+// Runs a sub-problem: the list l (in the warp's scratch; its classes may be
+// merged), L words `L` (lane w: word w), the first level pushing classes
+// [0, nend) only.  [top, end) is the arena.
+__device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint64_t* lk,
+                                     const int32_t* lid, uint64_t sR0, uint64_t nR0, uint32_t* top,
+                                     uint32_t* end) {
+  const int lane = (int)lane_id();
+  const uint64_t t0 = globaltimer_ns();
+  ClsCur& c = this_cur();
+  Tally y;
+  y.hl = 0;
+  y.cnt = y.nonmax = y.steps = 0;
+  {
+    const DevGraph* g = this_warp().gp;
+    y.swapped = g->swapped;
+    y.share_floor =
+        s_blk.nslot == 0 ? INT_MAX : min(s_blk.share_min_work, max(g->bound_size, 0));
+  }
+  unsigned long long hash = 0;
+  Leaf f;
+  int curw = 0;
+  bool leaf = cls_begin(&l, L, &nend, lk, lid, sR0, (uint32_t)nR0, top);
+  const bool root_leaf = leaf;
+  if (leaf) {
+    leaf_of_list(l, __shfl_sync(kFull, L, 0), nend, lk, sR0, (uint32_t)nR0, f);
+    if (lane == 0) c.leaf_lid = lid;
+    __syncwarp();
+  }
+  while (true) {
+    if (leaf) {
+      leaf = false;
+      if (!leaf_run(y, f, &c.leaf_lid) || root_leaf) break;
+    }
+    // ---- the next class to push: the first live P one ----
+    int cpos = -1;
+    {
+      const uint32_t* A = c.A;
+      const int nw = c.nw, pofs = 2 * c.nwp;
+      const int e = c.nend;
+      ROLLED for (int b0 = curw; b0 < nw; b0 += 32) {
+        const int w = b0 + lane;
+        const uint32_t t = w < nw ? A[w] & A[pofs + w] & first_bits(e, w) : 0u;
+        const unsigned bal = __ballot_sync(kFull, t != 0u);
+        if (bal) {
+          const int j = __ffs(bal) - 1;
+          cpos = (b0 + j) * 32 + __ffs(__shfl_sync(kFull, t, j)) - 1;
+          break;
+        }
+      }
+    }
+    if (cpos < 0) {
+      if (!cls_leave(c, L, curw)) break;
+      continue;
+    }
+    if ((++y.steps & 1023u) == 0u && must_stop()) break;
+    curw = cpos >> 5;
+    const int K = c.l.K;
+    const uint32_t mc = lane < K ? c.l.m[(size_t)lane * c.l.stride + cpos] : 0u;
+    const uint32_t lnw = L & mc, rmw = L & ~mc;
+    const int kn = (int)__reduce_add_sync(kFull, (unsigned)__popc(lnw));
+    const SweepOut o = cls_sweep(c, lnw, rmw, cpos);
+    if (o.nm) {
+      ++y.nonmax;
+      continue;
+    }
+    ++y.cnt;
+    uint64_t sR;
+    uint32_t nR;
+    hash += cls_biclique(c, lnw, kn, y.swapped, sR, nR);
+    if (s_blk.emit) emit_bits(kn, K, lnw, c.lid);
+    const int nsel = o.nsel, nselp = o.nselp;
+    if (kn <= 1 || nselp == 0) continue;
+    // Bits of the new L below each word (lane w: word w).
+    uint32_t base = 0u;
+    if (K > 1) {
+      int tot;
+      base = (uint32_t)excl_scan(__popc(lnw), &tot);
+    }
+    // A big enough child goes to an idle warp instead, at any depth, so that a
+    // subtree that started here can still be shared once warps run out of work.
+    if (nselp * (long long)kn >= y.share_floor && cls_export(lnw, base, nsel, nselp, kn, sR, nR))
+      continue;
+    const int kc = words_k(kn);
+    const int dK = kc <= kKMax && kc < K ? kc : K;
+    const bool pack = dK < K;
+    const long long keys = pack ? 64LL * dK + (s_blk.emit ? 32LL * dK : 0) : 0;
+    const bool tiny = kn <= 32 && nsel <= 32;
+    uint32_t* at = c.top;
+    if (lane == 0) c.fr->curw = curw;
+    if (!tiny && cls_need(nsel, dK, cls_levels(kn, nselp)) + keys > end - at) {
+      // ---- no room: a level on the parent's list ----
+      cls_enter(c.l, lnw, c.l.n, c.lk, c.lid, sR, nR, at, c.stop, false);
+      L = lnw;
+      curw = 0;
+      continue;
+    }
+    const uint64_t* clk = c.lk;
+    const int32_t* clid = c.lid;
+    if (pack) {
+      uint64_t* nlk = reinterpret_cast<uint64_t*>(at);
+      int32_t* nlid = s_blk.emit ? reinterpret_cast<int32_t*>(at + 64 * dK) : nullptr;
+      cls_pack_keys(clk, clid, K, lnw, base, nlk, nlid);
+      clk = nlk;
+      clid = nlid;
+      at += keys;
+    }
+    const uint32_t nl = pack ? first_bits(kn, lane) : lnw;
+    if (tiny) {
+      // ---- straight into the lanes ----
+      uint32_t* g = this_smem() + kSmIdx;
+      cls_indices(c.S, c.nw, g);
+      const bool in = lane < nsel;
+      const int i = in ? (int)g[lane] : 0;
+      const uint32_t* Q = c.A + c.nwp;
+      f.A = first_bits(nsel, 0);
+      f.Q = __ballot_sync(kFull, in && ((Q[i >> 5] >> (i & 31)) & 1u));
+      f.P = __ballot_sync(kFull, in && ((Q[c.nwp + (i >> 5)] >> (i & 31)) & 1u));
+      const bool p = (f.P >> lane) & 1u;
+      f.key = p ? c.l.key[i] : 0ULL;
+      f.cnt = p ? c.l.info[i] & kInfoCnt : 0u;
+      if (K == 1) {
+        const uint32_t l0 = __shfl_sync(kFull, lnw, 0);
+        f.m = in ? c.l.m[i] & l0 : 0u;
+      } else {
+        f.m = cls_pack<false>(c.l.m, c.l.stride, K, lnw, base, i, in, nullptr);
+      }
+      leaf = true;
+    } else {
+      ClsList d = cls_list_at(at, nsel, dK);
+      uint32_t* stop = c.stop;
+      if (kn <= 32 && nsel <= kChildMax) {
+        uint32_t* lm = d.m;
+        if (d.stride <= this_smem() + kSmemWords - stop) lm = stop;
+        d.n = cls_child(lnw, base, nsel, lm, d.key, d.info);
+        d.stride = (d.n + 31) & ~31;
+        d.m = lm;
+        leaf = d.n <= 32;
+        if (leaf) leaf_of_list(d, 0u, d.n, clk, sR, nR, f);
+        else if (lm == stop) stop += d.stride;
+      } else {
+        cls_copy_child(lnw, base, d.m, nsel, dK);
+        int dend = nsel;
+        if (s_blk.prune && nsel > 32)
+          d.n = cls_merge(d.m, d.key, d.info, nsel, dK, &d.stride, c.S, &dend);
+        if (d.n <= 32 && dK == 1) {
+          leaf_of_list(d, __shfl_sync(kFull, nl, 0), d.n, clk, sR, nR, f);
+          leaf = true;
+        }
+      }
+      if (!leaf) {
+        cls_enter(d, nl, d.n, clk, clid, sR, nR, at + cls_list_words(nsel, dK), stop, true);
+        L = lane < dK ? nl : 0u;
+        curw = 0;
+      }
+    }
+    if (leaf) {
+      const uint32_t l0 = __shfl_sync(kFull, nl, 0);
+      f.L = l0;
+      f.lk = (l0 >> lane) & 1u ? clk[lane] : 0ULL;
+      f.lim = kFull;
+      f.sR = sR;
+      f.nR = nR;
+      __syncwarp();
+      if (lane == 0) c.leaf_lid = clid;
+      __syncwarp();
+    }
+  }
+  hash += warp_sum64(y.hl);
+  Warp& W = this_warp();
+  acc(W.hash, hash);
+  acc(W.cnt, y.cnt);
+  acc(W.nonmax, y.nonmax);
+  acc(W.pushes, (unsigned long long)(y.cnt + y.nonmax) << 32);
+  acc(W.ns_t2, globaltimer_ns() - t0);
+  acc(W.n_t2, 1);
+  __syncwarp();
+}
+
+// Sub-problem list in the warp's own scratch over n L vertices (all bits):
+// [top, ...) is what follows the list.
+__device__ __forceinline__ void tier2(Warp& W, const ClsList& l, int n, int nend, uint64_t sR0,
+                                      uint64_t nR0) {
+  cls_run(l, first_bits(n, (int)lane_id()), nend, W.A64(W.sl().lkey), W.A(W.sl().lid), sR0, nR0,
+          l.m + cls_list_words(l.n, l.K), reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)));
 }
 
 // Runs an exported sub-problem and releases its slot.  The slot was written
@@ -873,59 +1771,217 @@ __device__ void tier2(Warp& W, int n, int nsub, int nq, int nend, uint64_t sR0, 
 // volatile loads and the body is copied through L2 (ld.global.cg) into this
 // warp's own scratch, where the sub-problem then runs.  The slot is freed as
 // soon as it is copied; nothing here writes it, so no store can land on the
-// records of its next owner.
-__device__ void tier2_from_slot(Warp& W, int slot) {
+// classes of its next owner.
+__device__ __noinline__ void tier2_from_slot(int slot) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
   int32_t* sp = slot_ptr(W, slot);
   volatile const int32_t* vh = sp;
   const int K = vh[0];
-  const int nsub = vh[1];
-  const int nq = vh[2];
+  const int n = vh[1];
   const int32_t gid = vh[3];
-  T2Src src;
-  for (int w = 0; w < 4; ++w) src.L0[w] = (uint32_t)vh[4 + w];
-  src.sR0 = (uint64_t)(uint32_t)vh[8] | ((uint64_t)(uint32_t)vh[9] << 32);
-  src.nR0 = (uint32_t)vh[10];
-  const int RS = rec_stride(K);
-  uint32_t* rec = reinterpret_cast<uint32_t*>(W.A(W.sl.masks));
-  uint64_t* subkey = W.A64(W.sl.sub_v);
-  uint64_t* lkey = W.A64(W.sl.lkey);
-  const unsigned* srec = reinterpret_cast<const unsigned*>(sp + kSlotRec);
-  const unsigned long long* skey =
-      reinterpret_cast<const unsigned long long*>(slot_subkey(sp, K, nsub));
-  const unsigned long long* slk = reinterpret_cast<const unsigned long long*>(sp + kSlotLkey);
-  const int nw = nsub * RS;
-  for (int i = lane; i < nw; i += 32) rec[i] = __ldcg(srec + i);
-  for (int i = lane; i < nsub; i += 32) subkey[i] = __ldcg(skey + i);
-  int32_t* lid = W.A(W.sl.lid);
+  const uint64_t sR = (uint64_t)(uint32_t)vh[4] | ((uint64_t)(uint32_t)vh[5] << 32);
+  const uint64_t nR = (uint32_t)vh[6];
+  const uint32_t L = lane < K ? (uint32_t)vh[kSlotL + lane] : 0u;
+  uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_root));
+  uint64_t* lkey = reinterpret_cast<uint64_t*>(at);
+  int32_t* lid = reinterpret_cast<int32_t*>(at + 64 * K);
+  const ClsList l = cls_list_at(at + 96 * K, n, K);
+  const int nw = (int)cls_list_words(n, K);
+  const uint4* src = reinterpret_cast<const uint4*>(sp + kSlotList);
+#pragma unroll 4
+  for (int i = lane; i < nw / 4; i += 32) reinterpret_cast<uint4*>(l.m)[i] = __ldcg(src + i);
+  const unsigned long long* slk = reinterpret_cast<const unsigned long long*>(sp + kSlotLk);
+  ROLLED for (int i = lane; i < 32 * K; i += 32) lkey[i] = __ldcg(slk + i);
   const unsigned* sli = reinterpret_cast<const unsigned*>(sp + kSlotLid);
-  for (int i = lane; i < 32 * K; i += 32) lkey[i] = __ldcg(slk + i);
-  if (W.p.emit)
-    for (int i = lane; i < 32 * K; i += 32) lid[i] = (int32_t)__ldcg(sli + i);
+  if (s_blk.emit)
+    ROLLED for (int i = lane; i < 32 * K; i += 32) lid[i] = (int32_t)__ldcg(sli + i);
   __syncwarp();
   if (lane == 0) slot_free(W, slot);
   __syncwarp();
   W.gid = gid;
   W.gp = graph_at(W, gid);
-  src.rec = rec;
-  src.subkey = subkey;
-  src.lkey = lkey;
-  src.lid = lid;
-  src.nsub = nsub;
-  src.nq = nq;
-  src.nend = nsub;
-  tier2_dispatch(W, src, K);
+  __syncwarp();
+  cls_run(l, L, n, lkey, lid, sR, nR, l.m + nw, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)));
 }
 
-// Zeroes nsub records of K mask words, each with its index and a free bound.
-__device__ void init_records(uint32_t* rec, int K, int nsub) {
+// Words of scratch cls_build may use on top of cls_need for a list of `eff`
+// classes made of n candidates over nL vertices.
+__host__ __device__ __forceinline__ long long cls_build_words(long long n, long long eff, int K,
+                                                              int nL) {
+  return cls_stride(eff) * (K + 1) + 4 * ((n + 63) >> 5) + 4LL * nL + 64;
+}
+
+// The edges between a sub-problem's candidates and its vertices: edge e joins
+// candidate tab[ids[e]] - bias (below 0: none) and vertex rows[e]; without
+// rows, ids holds both, id << 7 | vertex.
+struct ClsEdges {
+  const int32_t *ids, *rows, *tab;
+  int n, bias;
+};
+
+// Builds the class list of n candidates, [Q | P], the first nq of them Q, over
+// nL vertices, at `at` ([at, end): at least cls_need + cls_build_words).
+// Candidate i has cnt[i] of the vertices and hash key keys[vidx[i]].  *nend:
+// candidates [0, nend) may be pushed at the first level; classes [0, nend) on
+// return.
+//
+// Most candidates of a root have one of its vertices only (on the 300,000-edge
+// serving graph a root has 1,565 candidates and 1,867 edges to them).  Those
+// need no record: the candidates of one vertex are one class from the start,
+// summed up per vertex as the edges are walked, and only the others get masks.
+__device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, int nq, int K, int nL,
+                                          int* nend, const int32_t* cnt, const uint64_t* keys,
+                                          const int32_t* vidx, ClsEdges ed) {
   const int lane = (int)lane_id();
-  const int RS = rec_stride(K);
-  for (int q = lane; q < nsub; q += 32) {
-    rec[(size_t)q * RS] = ((uint32_t)q << 8) | kB8Free;
-    for (int w = 0; w < K; ++w) rec[(size_t)q * RS + 1 + w] = 0u;
+  const bool merge = s_blk.prune != 0;
+  const int nw = (n + 31) >> 5;
+  // Bits and ranks of the candidates with masks (M) and of all classes (F).
+  uint32_t* sm = this_smem() + kSmArena;
+  uint32_t* send = this_smem() + kSmemWords;
+  uint32_t* MB;
+  if (4 * nw <= send - sm) {
+    MB = sm;
+    sm += 4 * nw;
+  } else {
+    end -= 4 * ((nw + 1) & ~1);
+    MB = end;
+  }
+  uint32_t *MP = MB + nw, *FB = MP + nw, *FP = FB + nw;
+  int nm = 0;
+#pragma unroll 2
+  for (int b = 0; b < nw; ++b) {
+    const int i = b * 32 + lane;
+    const unsigned bal = __ballot_sync(kFull, i < n && (!merge || cnt[i] >= 2));
+    if (lane == 0) {
+      MB[b] = FB[b] = bal;
+      MP[b] = (uint32_t)nm;
+    }
+    nm += __popc(bal);
+  }
+  const int st = (nm + 31) & ~31;
+  end -= st;
+  uint32_t* mpos = end;  // candidate of each mask
+  uint32_t* raw;
+  if (K * st <= send - sm) {
+    raw = sm;
+  } else {
+    end -= (size_t)K * st;
+    raw = end;
+  }
+  ROLLED for (int i = lane; i < K * st; i += 32) raw[i] = 0u;
+  // Sums per vertex: the table's entries, or (more vertices than it has) an
+  // array of four words each.
+  const MergeTab t = this_tab();
+  const bool wide = nL > kSlots;
+  uint32_t* first = t.lead;  // 0x7fffffff - the first P candidate, or 0
+  uint32_t* info = t.info;
+  unsigned long long* key64 = nullptr;
+  if (wide) {
+    end -= 4 * ((nL + 1) & ~1);
+    first = end;
+    info = first + ((nL + 1) & ~1);
+    key64 = reinterpret_cast<unsigned long long*>(info + ((nL + 1) & ~1));
+    ROLLED for (int i = lane; i < 4 * ((nL + 1) & ~1); i += 32) first[i] = 0u;
   }
   __syncwarp();
+  ROLLED for (int w = lane; w < nw; w += 32) {
+    const uint32_t o = MP[w];
+    int k = 0;
+    ROLLED for (uint32_t b = MB[w]; b; b &= b - 1) mpos[o + k++] = (uint32_t)(w * 32 + __ffs(b) - 1);
+  }
+  __syncwarp();
+  ROLLED for (int e0 = 0; e0 < ed.n; e0 += 64) {
+    int id[2], ci[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int e = e0 + 32 * u + lane;
+      id[u] = e < ed.n ? ed.ids[e] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      ci[u] = id[u] >= 0 ? ed.tab[ed.rows ? id[u] : id[u] >> 7] - ed.bias : -1;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = ci[u];
+      if (i < 0) continue;
+      const int r = ed.rows ? ed.rows[e0 + 32 * u + lane] : id[u] & 127;
+      const uint32_t w = MB[i >> 5], bit = 1u << (i & 31);
+      if (w & bit) {
+        const uint32_t d = MP[i >> 5] + __popc(w & (bit - 1u));
+        atomicOr(&raw[(size_t)(r >> 5) * st + d], 1u << (r & 31));
+      } else if (i < nq) {
+        atomicOr(&info[r], kInfoQ);
+      } else {
+        atomicMax(&first[r], 0x7fffffffu - (uint32_t)i);
+        const uint64_t k = keys[vidx[i]];
+        if (wide) {
+          atomicAdd(&key64[r], (unsigned long long)k);
+        } else {
+          const uint32_t lo = (uint32_t)k;
+          const uint32_t old = atomicAdd(&t.lo[r], lo);
+          atomicAdd(&t.hi[r], (uint32_t)(k >> 32) + (old + lo < lo ? 1u : 0u));
+        }
+        atomicAdd(&info[r], 1u);
+      }
+    }
+  }
+  __threadfence_block();
+  __syncwarp();
+  int nqs = 0;  // vertices whose only candidates are Q
+  ROLLED for (int r0 = 0; r0 < nL; r0 += 32) {
+    const int r = r0 + lane;
+    const uint32_t v = r < nL ? first[r] : 0u;
+    if (v) {
+      const uint32_t i = 0x7fffffffu - v;
+      atomicOr(&FB[i >> 5], 1u << (i & 31));
+    }
+    nqs += __popc(__ballot_sync(kFull, r < nL && !v && (info[r] & kInfoQ)));
+  }
+  __syncwarp();
+  int nf = 0;
+  ROLLED for (int w0 = 0; w0 < nw; w0 += 32) {
+    const int w = w0 + lane;
+    int tot;
+    const int ex = excl_scan(w < nw ? __popc(FB[w]) : 0, &tot);
+    if (w < nw) FP[w] = (uint32_t)(nf + ex);
+    nf += tot;
+  }
+  __syncwarp();
+  // Classes before candidate i, the Q-only vertices' (they stand after the
+  // other Q classes) left out.
+  const auto rank = [&](int i) {
+    return i >= n ? nf : (int)FP[i >> 5] + __popc(FB[i >> 5] & ((1u << (i & 31)) - 1u));
+  };
+  const int nqm = rank(nq);
+  *nend = rank(*nend) + nqs;
+  const ClsList l = cls_list_at(at, nf + nqs, K);
+  ROLLED for (int d = lane; d < nm; d += 32) {
+    const int i = (int)mpos[d];
+    const int f = rank(i) + (i >= nq ? nqs : 0);
+    ROLLED for (int w = 0; w < K; ++w) l.m[(size_t)w * l.stride + f] = raw[(size_t)w * st + d];
+    l.info[f] = i < nq ? kInfoQ : kInfoP | 1u;
+    // Only P candidates' keys can enter an R that is counted.
+    l.key[f] = i < nq ? 0ULL : keys[vidx[i]];
+  }
+  int oq = nqm;
+  ROLLED for (int r0 = 0; r0 < nL; r0 += 32) {
+    const int r = r0 + lane;
+    const uint32_t v = r < nL ? first[r] : 0u;
+    const uint32_t fl = r < nL ? info[r] : 0u;
+    const unsigned bal = __ballot_sync(kFull, !v && fl != 0u);
+    if (v || fl) {
+      const int f = v ? rank((int)(0x7fffffffu - v)) + nqs : oq + __popc(bal & lanemask_lt());
+      ROLLED for (int w = 0; w < K; ++w)
+        l.m[(size_t)w * l.stride + f] = w == (r >> 5) ? 1u << (r & 31) : 0u;
+      l.info[f] = fl | (v ? kInfoP : 0u);
+      l.key[f] = wide ? key64[r] : (uint64_t)t.lo[r] | ((uint64_t)t.hi[r] << 32);
+      if (!wide) first[r] = info[r] = t.lo[r] = t.hi[r] = 0u;
+    }
+    oq += __popc(bal);
+  }
+  __syncwarp();
+  return l;
 }
 
 // ---------------------------------------------------------------------------
@@ -937,70 +1993,82 @@ struct T1 {
   uint64_t sRtask, nRtask;
 };
 
-// Selects L positions with Llevel == lvl, calling fn(pos) over rows of aadj.
-template <typename Fn>
-__device__ __forceinline__ void t1_rows_at_level(Warp& W, const T1& t, int lvl, Fn fn) {
-  const int32_t* llevel = W.A(W.sl.llevel);
-  const int32_t* aoff = W.A(W.sl.aoff);
-  const int lane = (int)lane_id();
-  // Compact the selected rows of each 32-chunk, then walk them flat.
-  for (int c0 = 0; c0 < t.nL; c0 += 32) {
-    int l = c0 + lane;
-    bool sel = l < t.nL && llevel[l] == lvl;
-    unsigned bal = __ballot_sync(kFull, sel);
-    int nsel = __popc(bal);
-    if (nsel == 0) continue;
-    // Lane j takes the j-th selected row of the chunk (nsel <= 32, so the
-    // row index flat_rows passes to row_of is this lane's own id).
-    int myrow = -1;
-    {
-      unsigned m = bal;
-      for (int k = 0; k < lane && m; ++k) m &= m - 1;
-      if (lane < nsel) myrow = c0 + __ffs(m) - 1;
-    }
-    flat_rows(
-        nsel,
-        [&](int, int& beg, int& len) {
-          beg = aoff[myrow];
-          len = aoff[myrow + 1] - beg;
-        },
-        fn);
-  }
-}
+// What a walk over rows does at each entry's candidate p.
+enum T1Op {
+  kOpAdd,      // count it
+  kOpSub,      // take its count back
+  kOpRestore,  // count it, and mark it touched if its bound is at least `level`
+  kOpRetire,   // retire it below `level` unless touched (or x itself)
+  kOpFree,     // touched: free again
+  kOpSetBit,   // its bit in bits
+  kOpClearBit, // its word in bits to zero
+};
 
-// Selects the L positions of candidate x's row (cadj) with llevel == lvl,
-// calling fn(pos) over their rows of aadj: the rows a push of x keeps, walked
-// without a pass over all of L.
-template <typename Fn>
-__device__ __forceinline__ void t1_rows_of(Warp& W, int x, int lvl, Fn fn) {
-  const int32_t* llevel = W.A(W.sl.llevel);
-  const int32_t* aoff = W.A(W.sl.aoff);
-  const int32_t* coff = W.A(W.sl.coff);
-  const int32_t* cadj = W.A(W.sl.cadj);
+// Walks rows of aadj: with x >= 0 the rows of candidate x's L positions (cadj)
+// whose llevel is lvl (those a push of x keeps, found without a pass over all
+// of L), else every L position with llevel == lvl.  One function for all walks
+// of a push and a pop: inlined at each of them, the walk was a third of the
+// counts tier's code.
+__device__ __noinline__ void t1_walk(int nL, int x, int lvl, int op, int level, uint32_t* bits) {
+  Warp& W = this_warp();
+  const int32_t* llevel = W.A(W.sl().llevel);
+  const int32_t* aoff = W.A(W.sl().aoff);
+  const int32_t* aadj = W.A(W.sl().aadj);
+  const int32_t* cadj = W.A(W.sl().cadj);
+  int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
   const int lane = (int)lane_id();
-  const int rb = coff[x], re = coff[x + 1];
-  for (int c0 = rb; c0 < re; c0 += 32) {
+  int rb = 0, re = nL;
+  if (x >= 0) {
+    const int32_t* coff = W.A(W.sl().coff);
+    rb = coff[x];
+    re = coff[x + 1];
+  }
+  const int xx = x;
+  ROLLED for (int c0 = rb; c0 < re; c0 += 32) {
     const int j = c0 + lane;
-    const int l = j < re ? cadj[j] : 0;
-    const bool sel = j < re && llevel[l] == lvl;
-    const unsigned bal = __ballot_sync(kFull, sel);
+    const int l = j < re ? (x >= 0 ? cadj[j] : j) : 0;
+    const unsigned bal = __ballot_sync(kFull, j < re && llevel[l] == lvl);
     const int nsel = __popc(bal);
     if (nsel == 0) continue;
-    int myrow = -1;
-    {
-      unsigned m = bal;
-      for (int k = 0; k < lane && m; ++k) m &= m - 1;
-      if (lane < nsel) myrow = __shfl_sync(kFull, l, __ffs(m) - 1);
-      else __shfl_sync(kFull, l, 0);
-    }
+    // Lane k takes the k-th selected row of the chunk.
+    unsigned m = bal;
+    ROLLED for (int k = 0; k < lane && m; ++k) m &= m - 1;
+    const int row = __shfl_sync(kFull, l, m ? __ffs(m) - 1 : 0);
     flat_rows(
         nsel,
         [&](int, int& beg, int& len) {
-          beg = aoff[myrow];
-          len = aoff[myrow + 1] - beg;
+          beg = aoff[row];
+          len = aoff[row + 1] - beg;
         },
-        fn);
+        [&](bool valid, int pos) {
+          const int p = valid ? aadj[pos] : -1;
+          const int b = p >= 0 && op >= kOpRestore && op <= kOpFree ? bound[p] : 0;
+          return ((long long)b << 32) | (unsigned)p;
+        },
+        [&](bool, int, int, long long v) {
+          const int p = (int)v, b = (int)(v >> 32);
+          if (p < 0) return;
+          switch (op) {
+            case kOpAdd: atomicAdd(&ncnt[p], 1); break;
+            case kOpSub: atomicSub(&ncnt[p], 1); break;
+            case kOpRestore:
+              atomicAdd(&ncnt[p], 1);
+              if (b >= level) bound[p] = kTouched;
+              break;
+            case kOpRetire:
+              if (p != xx && b >= level && b != kTouched) bound[p] = level - 1;
+              break;
+            case kOpFree:
+              if (b == kTouched) bound[p] = kFree;
+              break;
+            case kOpSetBit: atomicOr(&bits[p >> 5], 1u << (p & 31)); break;
+            default: bits[p >> 5] = 0u; break;
+          }
+        });
   }
+  __threadfence_block();
+  __syncwarp();
 }
 
 // finder_pop (src/IterFinderGpu.h:266-303) of candidate x at `level`, walking
@@ -1011,49 +2079,28 @@ __device__ __forceinline__ void t1_rows_of(Warp& W, int x, int lvl, Fn fn) {
 // rows has count 0 at this level and every level below it, so no push, scan,
 // maximality test or later pop at or below this level reads its bound, and
 // the pop one level up treats every bound >= level-1 alike.
-__device__ void t1_pop(Warp& W, const T1& t, int x, int level) {
-  int32_t* llevel = W.A(W.sl.llevel);
-  int32_t* ncnt = W.A(W.sl.ncnt);
-  int32_t* bound = W.A(W.sl.bound);
-  const int32_t* aadj = W.A(W.sl.aadj);
-  const int32_t* coff = W.A(W.sl.coff);
-  const int32_t* cadj = W.A(W.sl.cadj);
+__device__ __noinline__ void t1_pop(int nL, int x, int level) {
+  Warp& W = this_warp();
+  int32_t* llevel = W.A(W.sl().llevel);
+  int32_t* bound = W.A(W.sl().bound);
+  const int32_t* coff = W.A(W.sl().coff);
+  const int32_t* cadj = W.A(W.sl().cadj);
   const int lane = (int)lane_id();
-  const bool prune = W.p.prune != 0;
   // restore counts over L_parent \ L_child and mark touched candidates
-  t1_rows_at_level(W, t, level - 1, [&](bool valid, int, int pos) {
-    if (!valid) return;
-    int p = aadj[pos];
-    if (p < 0) return;
-    atomicAdd(&ncnt[p], 1);
-    if (bound[p] >= level) bound[p] = kTouched;
-  });
-  __syncwarp();
-  if (prune) {
+  t1_walk(nL, -1, level - 1, kOpRestore, level, nullptr);
+  if (s_blk.prune) {
     // Candidates of the kept rows that no removed row met are retired at this
     // level (a candidate in several kept rows is visited several times: the
     // write is the same each time, and touched ones are left for the pass
     // below).
-    t1_rows_of(W, x, level, [&](bool valid, int, int pos) {
-      if (!valid) return;
-      const int p = aadj[pos];
-      if (p < 0 || p == x) return;
-      const int b = bound[p];
-      if (b >= level && b != kTouched) bound[p] = level - 1;
-    });
-    __syncwarp();
+    t1_walk(nL, x, level, kOpRetire, level, nullptr);
     // touched candidates -> free
-    t1_rows_at_level(W, t, level - 1, [&](bool valid, int, int pos) {
-      if (!valid) return;
-      const int p = aadj[pos];
-      if (p >= 0 && bound[p] == kTouched) bound[p] = kFree;
-    });
-    __syncwarp();
+    t1_walk(nL, -1, level - 1, kOpFree, level, nullptr);
   }
   if (lane == 0) bound[x] = kFree;
   __syncwarp();
   // the kept rows go back to the level above (deeper levels are popped already)
-  for (int j = coff[x] + lane; j < coff[x + 1]; j += 32) {
+  ROLLED for (int j = coff[x] + lane; j < coff[x + 1]; j += 32) {
     const int l = cadj[j];
     if (llevel[l] == level) llevel[l] = level - 1;
   }
@@ -1063,23 +2110,40 @@ __device__ void t1_pop(Warp& W, const T1& t, int x, int level) {
 // Hands the child sub-problem of a maximal push (x at `level`, |L_new| = kept)
 // to tier 2.  Candidates: C entries live below this level with
 // 0 < count < kept; Q = those before x.
-__device__ void t1_handoff(Warp& W, const T1& t, int x, int level, int kept, uint64_t sR,
-                           uint64_t nR) {
+// Declined (false, nothing done) if the warp's arena may not hold it.
+__device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, uint64_t sR,
+                                        uint64_t nR) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
-  const int32_t* llevel = W.A(W.sl.llevel);
-  const int32_t* ncnt = W.A(W.sl.ncnt);
-  const int32_t* bound = W.A(W.sl.bound);
-  const int32_t* cv = W.A(W.sl.cv);
-  const uint64_t* ckey = W.A64(W.sl.ckey);
-  int32_t* sidx = W.A(W.sl.sidx);
-  int32_t* lp = W.A(W.sl.lp);
-  uint64_t* lkey = W.A64(W.sl.lkey);
-  uint64_t* subkey = W.A64(W.sl.sub_v);
-  const int32_t* aoff = W.A(W.sl.aoff);
-  const int32_t* aadj = W.A(W.sl.aadj);
+  const int32_t* llevel = W.A(W.sl().llevel);
+  const int32_t* ncnt = W.A(W.sl().ncnt);
+  const int32_t* bound = W.A(W.sl().bound);
+  const int32_t* cv = W.A(W.sl().cv);
+  const uint64_t* ckey = W.A64(W.sl().ckey);
+  int32_t* sidx = W.A(W.sl().sidx);
+  int32_t* lp = W.A(W.sl().lp);
+  uint64_t* lkey = W.A64(W.sl().lkey);
+  const int32_t* aoff = W.A(W.sl().aoff);
+  const int32_t* aadj = W.A(W.sl().aadj);
+  const auto selected = [&](int i) {
+    return i < t.nC && bound[i] > level && ncnt[i] > 0 && ncnt[i] < kept;
+  };
+  int nsub = 0, nq = 0;
+  ROLLED for (int i = lane; i < t.nC; i += 32) {
+    const bool sel = selected(i);
+    nsub += sel;
+    nq += sel && i < x;  // candidates before x are Q
+  }
+  nsub = (int)__reduce_add_sync(kFull, (unsigned)nsub);
+  nq = (int)__reduce_add_sync(kFull, (unsigned)nq);
+  const int K = words_k(kept);
+  if (nsub > 0 && cls_need(nsub, K, cls_levels(kept, nsub - nq)) +
+                          cls_build_words(nsub, nsub, K, kept) + cls_stride(nsub) >
+                      W.sub_words())
+    return false;
   // L_sub positions
   int n = 0;
-  for (int c0 = 0; c0 < t.nL; c0 += 32) {
+  ROLLED for (int c0 = 0; c0 < t.nL; c0 += 32) {
     int l = c0 + lane;
     bool sel = l < t.nL && llevel[l] == level;
     unsigned bal = __ballot_sync(kFull, sel);
@@ -1087,36 +2151,31 @@ __device__ void t1_handoff(Warp& W, const T1& t, int x, int level, int kept, uin
       int j = n + __popc(bal & lanemask_lt());
       lp[j] = l;
       lkey[j] = W.gp->ukey[t.L[l]];
-      if (W.p.emit) W.A(W.sl.lid)[j] = t.L[l];
+      if (s_blk.emit) W.A(W.sl().lid)[j] = t.L[l];
     }
     n += __popc(bal);
   }
-  // candidates
-  int nsub = 0, nq = 0;
-  for (int c0 = 0; c0 < t.nC; c0 += 32) {
-    int i = c0 + lane;
-    bool sel = false;
-    if (i < t.nC) {
-      int c = ncnt[i];
-      sel = bound[i] > level && c > 0 && c < kept;
-      sidx[i] = -1;
-    }
-    unsigned bal = __ballot_sync(kFull, sel);
-    if (sel) {
-      int s = nsub + __popc(bal & lanemask_lt());
-      sidx[i] = s;
-      subkey[s] = ckey[i];
-    }
-    nsub += __popc(bal);
-    // candidates before x are Q
-    unsigned before = __ballot_sync(kFull, sel && i < x);
-    nq += __popc(before);
-  }
-  __syncwarp();
   if (nsub > 0) {
-    const int K = words_k(n), RS = rec_stride(K);
-    uint32_t* rec = reinterpret_cast<uint32_t*>(W.A(W.sl.masks));
-    init_records(rec, K, nsub);
+    uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub));
+    uint32_t* cpos = at;  // C index of each candidate
+    at += cls_stride(nsub);
+    int o = 0;
+    ROLLED for (int c0 = 0; c0 < t.nC; c0 += 32) {
+      const int i = c0 + lane;
+      const bool sel = selected(i);
+      const unsigned bal = __ballot_sync(kFull, sel);
+      if (sel) {
+        const int s = o + __popc(bal & lanemask_lt());
+        sidx[i] = s;
+        cpos[s] = (uint32_t)i;
+      } else if (i < t.nC) {
+        sidx[i] = -1;
+      }
+      o += __popc(bal);
+    }
+    __syncwarp();
+    int nend = nsub, ne = 0;
+    int32_t* ent = W.A(W.sl().ent);
     flat_rows(
         n,
         [&](int r, int& beg, int& len) {
@@ -1124,17 +2183,20 @@ __device__ void t1_handoff(Warp& W, const T1& t, int x, int level, int kept, uin
           beg = aoff[l];
           len = aoff[l + 1] - beg;
         },
-        [&](bool valid, int r, int pos) {
-          if (!valid) return;
-          int p = aadj[pos];
-          if (p < 0) return;
-          int s = sidx[p];
-          if (s >= 0) atomicOr(&rec[(size_t)s * RS + 1 + (r >> 5)], 1u << (r & 31));
+        [&](bool valid, int pos) { return valid ? aadj[pos] : -1; },
+        [&](bool, int r, int, int p) {
+          const unsigned be = __ballot_sync(kFull, p >= 0);
+          if (p >= 0) ent[ne + __popc(be & lanemask_lt())] = (p << 7) | r;
+          ne += __popc(be);
         });
     __syncwarp();
-    tier2(W, n, nsub, nq, nsub, sR, nR);
+    const ClsList l = cls_build(at, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)), nsub, nq, K, n,
+                                &nend, nullptr, ckey, reinterpret_cast<int32_t*>(cpos),
+                                ClsEdges{ent, nullptr, sidx, ne, 0});
+    tier2(W, l, n, nend, sR, nR);
   }
   __syncwarp();
+  return true;
 }
 
 // A push at `level` whose child L (the `kept` rows, marked llevel == level)
@@ -1147,28 +2209,29 @@ __device__ void t1_handoff(Warp& W, const T1& t, int x, int level, int kept, uin
 // candidate of bound >= level is FREE before the push, and candidates not
 // adjacent to the kept rows are either touched (stay FREE) or irrelevant
 // below this level (count 0), so only candidates adjacent to the kept rows
-// change.
-__device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept, uint64_t sL) {
+// change.  Declined (false, nothing done) if the warp's arena may not hold the
+// child.
+__device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int kept, uint64_t sL) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
-  int32_t* llevel = W.A(W.sl.llevel);
-  const int32_t* ncnt = W.A(W.sl.ncnt);
-  int32_t* bound = W.A(W.sl.bound);
-  const int32_t* cv = W.A(W.sl.cv);
-  const int32_t* coff = W.A(W.sl.coff);
-  const int32_t* cadj = W.A(W.sl.cadj);
-  const int32_t* aoff = W.A(W.sl.aoff);
-  const int32_t* aadj = W.A(W.sl.aadj);
-  int32_t* cc = W.A(W.sl.fill);   // child counts, all-zero between pushes
-  int32_t* sidx = W.A(W.sl.sidx); // -1 between pushes
-  int32_t* tl = W.A(W.sl.tlist);
-  int32_t* lp = W.A(W.sl.lp);
-  uint64_t* lkey = W.A64(W.sl.lkey);
-  uint64_t* subkey = W.A64(W.sl.sub_v);
+  int32_t* llevel = W.A(W.sl().llevel);
+  const int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
+  const int32_t* cv = W.A(W.sl().cv);
+  const int32_t* coff = W.A(W.sl().coff);
+  const int32_t* cadj = W.A(W.sl().cadj);
+  const int32_t* aoff = W.A(W.sl().aoff);
+  const int32_t* aadj = W.A(W.sl().aadj);
+  int32_t* cc = W.A(W.sl().fill);   // child counts, all-zero between pushes
+  int32_t* sidx = W.A(W.sl().sidx); // -1 between pushes
+  int32_t* tl = W.A(W.sl().tlist);
+  int32_t* lp = W.A(W.sl().lp);
+  uint64_t* lkey = W.A64(W.sl().lkey);
   // kept rows -> lp[0..kept), with their hash keys
   int n = 0;
   {
     int rb = coff[x], re = coff[x + 1];
-    for (int b0 = rb; b0 < re; b0 += 32) {
+    ROLLED for (int b0 = rb; b0 < re; b0 += 32) {
       int j = b0 + lane;
       int l = j < re ? cadj[j] : 0;
       bool sel = j < re && llevel[l] == level;
@@ -1178,7 +2241,7 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
         lp[q] = l;
         if (q < 32 * kKMax) {
           lkey[q] = W.gp->ukey[t.L[l]];
-          if (W.p.emit) W.A(W.sl.lid)[q] = t.L[l];
+          if (s_blk.emit) W.A(W.sl().lid)[q] = t.L[l];
         }
       }
       n += __popc(bal);
@@ -1188,56 +2251,49 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
   // Child counts over the kept rows.  tl = candidates met (each once);
   // ent = every (candidate, row) entry met, packed p << 7 | r (r < 128), so
   // that the child's masks come from one linear pass instead of a second walk.
-  int32_t* ent = W.A(W.sl.ent);
-  int32_t* tcls = W.A(W.sl.tcls);
-  const uint64_t* ckey = W.A64(W.sl.ckey);
+  int32_t* ent = W.A(W.sl().ent);
+  int32_t* tcls = W.A(W.sl().tcls);
+  const uint64_t* ckey = W.A64(W.sl().ckey);
   int nt = 0, ne = 0;
   int kent = 0;  // entries of the kept rows
-  for (int q = lane; q < n; q += 32) kent += aoff[lp[q] + 1] - aoff[lp[q]];
-  kent = warp_sum(kent);
+  ROLLED for (int q = lane; q < n; q += 32) kent += aoff[lp[q] + 1] - aoff[lp[q]];
+  kent = warp_sum64(kent);
   const int cwords = (t.nC + 31) >> 5;
-  if (use_gseen(W, kent, cwords)) {
-    // fire-and-forget counts and touch bits; the touched list from the bitmap
-    flat_rows(
-        n,
-        [&](int r, int& beg, int& len) {
-          int l = lp[r];
-          beg = aoff[l];
-          len = aoff[l + 1] - beg;
-        },
-        [&](bool valid, int r, int pos) {
-          int p = valid ? aadj[pos] : -1;
-          if (p >= 0) {
+  // (with `scan`: fire-and-forget counts and touch bits, and the touched list
+  // from the bitmap)
+  const bool scan = use_gseen(W, kent, cwords);
+  if (!scan) clear_seen(W, cwords);
+  flat_rows(
+      n,
+      [&](int r, int& beg, int& len) {
+        int l = lp[r];
+        beg = aoff[l];
+        len = aoff[l + 1] - beg;
+      },
+      [&](bool valid, int pos) { return valid ? aadj[pos] : -1; },
+      [&](bool, int r, int, int p) {
+        const unsigned lt = lanemask_lt();
+        bool first = false;
+        if (p >= 0) {
+          if (scan) {
             atomicAdd(&cc[p], 1);
-            atomicOr(&W.gseen[p >> 5], 1u << (p & 31));
+            atomicOr(&W.gseen()[p >> 5], 1u << (p & 31));
+          } else {
+            first = count_first(W, cc, p);
           }
-          const unsigned be = __ballot_sync(kFull, p >= 0);
-          if (p >= 0) ent[ne + __popc(be & lanemask_lt())] = (p << 7) | r;
-          ne += __popc(be);
-        });
+        }
+        const unsigned bal = __ballot_sync(kFull, first);
+        if (first) tl[nt + __popc(bal & lt)] = p;
+        nt += __popc(bal);
+        const unsigned be = __ballot_sync(kFull, p >= 0);
+        if (p >= 0) ent[ne + __popc(be & lt)] = (p << 7) | r;
+        ne += __popc(be);
+      });
+  if (scan) {
     __threadfence_block();
     __syncwarp();
-    nt = collect_bits(W.gseen, cwords, tl, t.nC);
+    nt = collect_bits(W.gseen(), cwords, tl, t.nC);
   } else {
-    flat_rows(
-        n,
-        [&](int r, int& beg, int& len) {
-          int l = lp[r];
-          beg = aoff[l];
-          len = aoff[l + 1] - beg;
-        },
-        [&](bool valid, int r, int pos) {
-          int p = valid ? aadj[pos] : -1;
-          bool first = false;
-          if (p >= 0) first = count_first(W, cc, p);
-          const unsigned lt = lanemask_lt();
-          unsigned bal = __ballot_sync(kFull, first);
-          if (first) tl[nt + __popc(bal & lt)] = p;
-          nt += __popc(bal);
-          unsigned be = __ballot_sync(kFull, p >= 0);
-          if (p >= 0) ent[ne + __popc(be & lt)] = (p << 7) | r;
-          ne += __popc(be);
-        });
     counts_done(W, tl, nt);
   }
   // R of the child, maximality, and each touched candidate's class (0 none,
@@ -1246,7 +2302,7 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
   bool ism = true;
   uint64_t sR = 0;
   unsigned long long nR = 0;
-  int ncand = 0, nqc = 0;
+  int ncand = 0, nqc = 0, nmul = 0;
 #pragma unroll 4
   for (int q = lane; q < nt; q += 32) {
     const int p = tl[q];
@@ -1261,48 +2317,43 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
       cls = p < x ? 1 : 2;
       ++ncand;
       nqc += cls == 1;
+      nmul += c >= 2;
     }
     tcls[q] = cls;
   }
   ism = __all_sync(kFull, ism);
-  ncand = warp_sum(ncand);
-  nqc = warp_sum(nqc);
-  sR = warp_sum(sR) + t.sRtask;
-  nR = warp_sum(nR) + t.nRtask;
+  ncand = (int)__reduce_add_sync(kFull, (unsigned)ncand);
+  nqc = (int)__reduce_add_sync(kFull, (unsigned)nqc);
+  nmul = (int)__reduce_add_sync(kFull, (unsigned)nmul);
+  const int K = words_k(n);
+  const int eff = min(ncand, nmul + kept);  // classes of the child, at most
+  const int levels = cls_levels(kept, ncand - nqc);
+  if (ism && kept > 1 && ncand > 0 &&
+      cls_need(eff, K, levels) + cls_build_words(ncand, eff, K, kept) + 2 * cls_stride(ncand) >
+          W.sub_words()) {
+    ROLLED for (int q = lane; q < nt; q += 32) cc[tl[q]] = 0;
+    __syncwarp();
+    return false;
+  }
+  sR = warp_sum64(sR) + t.sRtask;
+  nR = warp_sum64(nR) + t.nRtask;
   if (ism) {
-    W.cnt += 1;
-    W.hash += biclique_hash(*W.gp, sL, (uint64_t)kept, sR, nR);
-    if (W.p.emit) emit_list(W.ctl, emit_dst(W.p), W.gid, n, t.L, lp);
+    acc(W.cnt, 1);
+    acc(W.hash, biclique_hash(*W.gp, sL, (uint64_t)kept, sR, nR));
+    if (s_blk.emit) emit_list(s_blk.ctl, emit_dst(*s_blk.p), W.gid, n, t.L, lp);
   } else {
-    W.nonmax += 1;
+    acc(W.nonmax, 1);
   }
   __syncwarp();
   if (ism && kept > 1 && ncand > 0) {
-    // Destination: an export slot when idle warps want work and the child is
-    // big enough by GMBE's split test, else this warp's scratch.
-    const int K = words_k(n), RS = rec_stride(K);
-    int slot = -1;
-    if (slot_fits(W, ncand, K) && should_export(W, ncand - nqc, n, W.p.eager_share != 0)) {
-      slot = lane == 0 ? slot_alloc_for(W, ncand, K) : 0;
-      slot = __shfl_sync(kFull, slot, 0);
-    }
-    uint32_t* rec = reinterpret_cast<uint32_t*>(W.A(W.sl.masks));
-    int32_t* sp = nullptr;
-    if (slot >= 0) {
-      sp = slot_ptr(W, slot);
-      rec = reinterpret_cast<uint32_t*>(sp + kSlotRec);
-      subkey = slot_subkey(sp, K, ncand);
-      uint64_t* lk = reinterpret_cast<uint64_t*>(sp + kSlotLkey);
-      for (int b = lane; b < n; b += 32) lk[b] = lkey[b];
-      if (W.p.emit) {
-        int32_t* li = sp + kSlotLid;
-        const int32_t* lid = W.A(W.sl.lid);
-        for (int b = lane; b < n; b += 32) li[b] = lid[b];
-      }
-    }
     // child indices: Q from the front, P from the back
+    uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub));
+    int32_t* cpos = reinterpret_cast<int32_t*>(at);  // C index of each child candidate
+    at += cls_stride(ncand);
+    int32_t* ccnt = reinterpret_cast<int32_t*>(at);  // its count in the kept rows
+    at += cls_stride(ncand);
     int nq = 0, np = 0;
-    for (int b0 = 0; b0 < nt; b0 += 32) {
+    ROLLED for (int b0 = 0; b0 < nt; b0 += 32) {
       int q = b0 + lane;
       const int cls = q < nt ? tcls[q] : 0;
       const int p = q < nt ? tl[q] : 0;
@@ -1313,31 +2364,44 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
       if (cls == 2) s = ncand - 1 - (np + __popc(bp & lanemask_lt()));
       if (s >= 0) {
         sidx[p] = s;
-        subkey[s] = ckey[p];
+        cpos[s] = p;
+        ccnt[s] = cc[p];
       }
       nq += __popc(bq);
       np += __popc(bp);
     }
     __syncwarp();
-    init_records(rec, K, ncand);
-#pragma unroll 4
-    for (int e = lane; e < ne; e += 32) {
-      const int pk = ent[e];
-      const int si = sidx[pk >> 7];
-      const int r = pk & 127;
-      if (si >= 0) atomicOr(&rec[(size_t)si * RS + 1 + (r >> 5)], 1u << (r & 31));
+    int nend = ncand;
+    const ClsList l = cls_build(at, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)), ncand, nqc, K,
+                                n, &nend, ccnt, ckey, cpos, ClsEdges{ent, nullptr, sidx, ne, 0});
+    // To an idle warp when some want work and the child is big enough by
+    // GMBE's split test, else it runs here.
+    int slot = -1;
+    if (slot_fits(W, l.n, K, levels) && should_export(W, ncand - nqc, n, s_blk.eager_share != 0)) {
+      slot = lane == 0 ? slot_alloc_for(W, l.n, K) : 0;
+      slot = __shfl_sync(kFull, slot, 0);
     }
-    __syncwarp();
     if (slot >= 0) {
-      if (lane == 0) {
-        uint32_t L0[4];
-        full_mask(L0, n);
-        slot_header(sp, K, ncand, nq, L0, sR, nR, W.gid);
+      int32_t* sp = slot_ptr(W, slot);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(sp + kSlotList);
+      const int words = (int)cls_list_words(l.n, K);
+      ROLLED for (int i = lane; i < words; i += 32) dst[i] = l.m[i];
+      uint64_t* lk = reinterpret_cast<uint64_t*>(sp + kSlotLk);
+      ROLLED for (int b = lane; b < n; b += 32) lk[b] = lkey[b];
+      if (s_blk.emit) {
+        int32_t* li = sp + kSlotLid;
+        const int32_t* lid = W.A(W.sl().lid);
+        ROLLED for (int b = lane; b < n; b += 32) li[b] = lid[b];
       }
-      if (!slot_publish(W, slot)) tier2_from_slot(W, slot);  // ring full: run it here
-    } else {
-      tier2(W, n, ncand, nq, ncand, sR, nR);
+      if (lane < K) sp[kSlotL + lane] = (int32_t)first_bits(n, lane);
+      if (lane == 0) slot_header(sp, K, l.n, n, sR, nR, W.gid);
+      if (!slot_publish(slot, 0)) {  // ring full
+        if (lane == 0) slot_free(W, slot);
+        __syncwarp();
+        slot = -1;
+      }
     }
+    if (slot < 0) tier2(W, l, n, nend, sR, nR);
   }
   __syncwarp();
   // state after finder_pop(x, level), then clear the child scratch
@@ -1348,8 +2412,9 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
     cc[p] = 0;
     sidx[p] = -1;
   }
-  for (int q = lane; q < n; q += 32) llevel[lp[q]] = level - 1;
+  ROLLED for (int q = lane; q < n; q += 32) llevel[lp[q]] = level - 1;
   __syncwarp();
+  return true;
 }
 
 // Levels 2 .. kLevelBits + 1 of the counts tier keep a bitmap of the
@@ -1357,8 +2422,8 @@ __device__ void t1_sparse_push(Warp& W, const T1& t, int x, int level, int kept,
 // live candidate and a recount walk its words instead of every candidate.
 __device__ __forceinline__ uint32_t* level_bits(const Warp& W, int level) {
   if (level < 2 || level > kLevelBits + 1) return nullptr;
-  return reinterpret_cast<uint32_t*>(W.A(W.sl.lbits)) +
-         (size_t)(level - 2) * (size_t)((W.sl.capC + 31) >> 5);
+  return reinterpret_cast<uint32_t*>(W.A(W.sl().lbits)) +
+         (size_t)(level - 2) * (size_t)((W.sl().capC + 31) >> 5);
 }
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
@@ -1374,7 +2439,7 @@ __device__ __forceinline__ int t1_next_live(const int32_t* bound, const int32_t*
                                             const uint32_t* bits, int start, int end, int level) {
   const int lane = (int)lane_id();
   if (!bits) {
-    for (int b0 = start; b0 < end; b0 += 32) {
+    ROLLED for (int b0 = start; b0 < end; b0 += 32) {
       const int i = b0 + lane;
       const bool ok = i < end && bound[i] > level - 1 && ncnt[i] != 0;
       const unsigned bal = __ballot_sync(kFull, ok);
@@ -1384,7 +2449,7 @@ __device__ __forceinline__ int t1_next_live(const int32_t* bound, const int32_t*
   }
   if (start >= end) return -1;
   const int w0 = start >> 5, wend = (end + 31) >> 5;
-  for (int wb = w0; wb < wend; wb += 32) {
+  ROLLED for (int wb = w0; wb < wend; wb += 32) {
     const int w = wb + lane;
     uint32_t m = w < wend ? bits[w] : 0u;
     if (w == w0) m &= ~0u << (start & 31);
@@ -1421,23 +2486,24 @@ constexpr int kFrameHdr = 16;
 // Whether a counts-tier child of `kept` rows (`kent` entries) may be shared
 // out now: slots exist, every warp has room for it, warps wait for work.
 __device__ __forceinline__ bool t1_export_wanted(Warp& W, int kept, long long kent) {
-  if (!W.p.share_counts || (W.nslot == 0 && W.nbig == 0)) return false;
-  if (kept > W.import_l || kent > (long long)W.import_s) return false;
-  return export_demand(W) != 0;
+  if (!s_blk.share_counts || (s_blk.nslot == 0 && s_blk.nbig == 0)) return false;
+  if (kept > s_blk.import_l || kent > (long long)s_blk.import_s) return false;
+  return export_demand() != 0;
 }
 
-__device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, long long kent,
-                              uint64_t sR, uint64_t nR, const uint32_t* nbits) {
+__device__ __noinline__ bool t1_try_export(const T1 t, int x, int level, int kept, long long kent,
+                                           uint64_t sR, uint64_t nR, const uint32_t* nbits) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
-  const int32_t* bound = W.A(W.sl.bound);
-  const int32_t* ncnt = W.A(W.sl.ncnt);
-  const int32_t* cv = W.A(W.sl.cv);
-  const int32_t* coff = W.A(W.sl.coff);
-  const int32_t* cadj = W.A(W.sl.cadj);
-  const int32_t* llevel = W.A(W.sl.llevel);
+  const int32_t* bound = W.A(W.sl().bound);
+  const int32_t* ncnt = W.A(W.sl().ncnt);
+  const int32_t* cv = W.A(W.sl().cv);
+  const int32_t* coff = W.A(W.sl().coff);
+  const int32_t* cadj = W.A(W.sl().cadj);
+  const int32_t* llevel = W.A(W.sl().llevel);
   const int cwords = (t.nC + 31) >> 5;
   int m = 0, mq = 0;
-  for (int w0 = 0; w0 < cwords; w0 += 32) {
+  ROLLED for (int w0 = 0; w0 < cwords; w0 += 32) {
     const int w = w0 + lane;
     uint32_t b = w < cwords ? nbits[w] : 0u;
     while (b) {
@@ -1449,16 +2515,16 @@ __device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, 
       b &= b - 1;
     }
   }
-  m = warp_sum(m);
-  mq = warp_sum(mq);
-  if (m == 0 || m > W.import_cap || !should_export(W, m - mq, kept)) return false;
+  m = (int)__reduce_add_sync(kFull, (unsigned)m);
+  mq = (int)__reduce_add_sync(kFull, (unsigned)mq);
+  if (m == 0 || m > s_blk.import_cap || !should_export(W, m - mq, kept)) return false;
   const long long words = kFrameHdr + (long long)kept + m;
   int slot = -1;
   if (lane == 0) {
     if (words <= kSlotWords) slot = slot_alloc(W);
     if (slot < 0 && words <= kBigSlotWords) {
-      const int b = bits_alloc(W.big_bits, W.nbig);
-      if (b >= 0) slot = W.nslot + b;
+      const int b = bits_alloc(s_blk.big_bits, s_blk.nbig);
+      if (b >= 0) slot = s_blk.nslot + b;
     }
   }
   slot = __shfl_sync(kFull, slot, 0);
@@ -1466,7 +2532,7 @@ __device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, 
   int32_t* sp = slot_ptr(W, slot);
   // L' ids: the kept rows, from x's row of cadj
   int nl = 0;
-  for (int j0 = coff[x]; j0 < coff[x + 1]; j0 += 32) {
+  ROLLED for (int j0 = coff[x]; j0 < coff[x + 1]; j0 += 32) {
     const int j = j0 + lane;
     const int l = j < coff[x + 1] ? cadj[j] : 0;
     const bool sel = j < coff[x + 1] && llevel[l] == level;
@@ -1477,18 +2543,18 @@ __device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, 
   // C' ids in index order: lane k takes word k of each round
   int32_t* cdst = sp + kFrameHdr + kept;
   int o = 0;
-  for (int w0 = 0; w0 < cwords; w0 += 32) {
+  ROLLED for (int w0 = 0; w0 < cwords; w0 += 32) {
     const int w = w0 + lane;
     uint32_t b = w < cwords ? nbits[w] : 0u;
     uint32_t keep = 0u;
-    for (uint32_t bb = b; bb; bb &= bb - 1) {
+    ROLLED for (uint32_t bb = b; bb; bb &= bb - 1) {
       const int bit = __ffs(bb) - 1;
       const int p = (w << 5) + bit;
       if (bound[p] > level && ncnt[p] < kept) keep |= 1u << bit;
     }
     int tot;
-    int at = o + warp_excl_scan(__popc(keep), &tot);
-    for (; keep; keep &= keep - 1) cdst[at++] = cv[(w << 5) + __ffs(keep) - 1];
+    int at = o + excl_scan(__popc(keep), &tot);
+    ROLLED for (; keep; keep &= keep - 1) cdst[at++] = cv[(w << 5) + __ffs(keep) - 1];
     o += tot;
   }
   if (lane == 0) {
@@ -1499,8 +2565,8 @@ __device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, 
     *reinterpret_cast<uint64_t*>(sp + 4) = sR;
     sp[6] = (int32_t)nR;
   }
-  if (slot_publish(W, slot, 1)) {
-    W.splits += 1;
+  if (slot_publish(slot, 1)) {
+    acc(W.splits, 1);
     return true;
   }
   if (lane == 0) slot_free(W, slot);
@@ -1508,26 +2574,27 @@ __device__ bool t1_try_export(Warp& W, const T1& t, int x, int level, int kept, 
   return false;
 }
 
-__device__ void tier1_run(Warp& W, const T1& t) {
+__device__ __noinline__ void tier1_run(const T1 t) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
-  int32_t* llevel = W.A(W.sl.llevel);
-  int32_t* ncnt = W.A(W.sl.ncnt);
-  int32_t* bound = W.A(W.sl.bound);
-  int32_t* stack = W.A(W.sl.stack);
-  int32_t* lent = W.A(W.sl.lent);
-  const uint64_t* ckey = W.A64(W.sl.ckey);
-  const int32_t* coff = W.A(W.sl.coff);
-  const int32_t* cadj = W.A(W.sl.cadj);
-  const int32_t* aoff = W.A(W.sl.aoff);
-  const int32_t* aadj = W.A(W.sl.aadj);
-  const bool emitting = W.p.emit != nullptr;
+  int32_t* llevel = W.A(W.sl().llevel);
+  int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
+  int32_t* stack = W.A(W.sl().stack);
+  int32_t* lent = W.A(W.sl().lent);
+  const uint64_t* ckey = W.A64(W.sl().ckey);
+  const int32_t* coff = W.A(W.sl().coff);
+  const int32_t* cadj = W.A(W.sl().cadj);
+  const int32_t* aoff = W.A(W.sl().aoff);
+  const int32_t* aadj = W.A(W.sl().aadj);
+  const bool emitting = s_blk.emit != nullptr;
   const int t2max = W.gp->tier2_max_l;
   const int cwords = (t.nC + 31) >> 5;
 
   // The level bitmaps start clear (a task that ended early may leave bits).
-  for (int lv = 2; lv <= kLevelBits + 1; ++lv) {
+  ROLLED for (int lv = 2; lv <= kLevelBits + 1; ++lv) {
     uint32_t* b = level_bits(W, lv);
-    for (int w = lane; w < cwords; w += 32) b[w] = 0u;
+    ROLLED for (int w = lane; w < cwords; w += 32) b[w] = 0u;
   }
   if (lane == 0) {
     stack[0] = t.nq;
@@ -1539,18 +2606,18 @@ __device__ void tier1_run(Warp& W, const T1& t) {
   while (level != 0) {
     // The stop flag is a global load the whole warp waits for: look at it on
     // the first step and every 64th after.
-    if ((steps++ & 63u) == 0u && must_stop(W)) return;
+    if ((steps++ & 63u) == 0u && must_stop()) return;
     const int end = level == 1 ? t.nend : t.nC;  // the first level may push a part only
     int cur = t1_next_live(bound, ncnt, level_bits(W, level), stack[level - 1], end, level);
     if (cur >= 0) {
       // ---- finder_push (src/IterFinderGpu.h:206-264) ----
-      W.pushes += 1;
+      acc(W.pushes, 1);
       int kept = 0;
       uint64_t sL = 0;
       long long kent = 0;                 // entries of the kept rows
       unsigned long long best = ~0ULL;    // (row length << 32) | position of the shortest kept row
       int rb = coff[cur], re = coff[cur + 1];
-      for (int j = rb + lane; j < re; j += 32) {
+      ROLLED for (int j = rb + lane; j < re; j += 32) {
         int l = cadj[j];
         if (llevel[l] == level - 1) {
           llevel[l] = level;
@@ -1561,13 +2628,12 @@ __device__ void tier1_run(Warp& W, const T1& t) {
           best = min(best, ((unsigned long long)(unsigned)len << 32) | (unsigned)l);
         }
       }
-      kept = warp_sum(kept);
-      sL = warp_sum(sL);
-      kent = warp_sum(kent);
+      kept = (int)__reduce_add_sync(kFull, (unsigned)kept);
+      sL = warp_sum64(sL);
+      kent = warp_sum64(kent);
       best = warp_min_u64(best);
       __syncwarp();
-      if (W.p.prune && kept <= t2max) {
-        t1_sparse_push(W, t, cur, level, kept, sL);
+      if (s_blk.prune && kept <= t2max && t1_sparse_push(t, cur, level, kept, sL)) {
         if (lane == 0) stack[level - 1] = cur + 1;
         __syncwarp();
         continue;
@@ -1579,7 +2645,7 @@ __device__ void tier1_run(Warp& W, const T1& t) {
       const long long clear_cost = pbits ? (long long)cwords : (long long)t.nC;
       if (clear_cost + kent < rent) {
         if (pbits) {
-          for (int w = lane; w < cwords; w += 32) {
+          ROLLED for (int w = lane; w < cwords; w += 32) {
             uint32_t m = pbits[w];
             while (m) {
               ncnt[(w << 5) + __ffs(m) - 1] = 0;
@@ -1587,20 +2653,12 @@ __device__ void tier1_run(Warp& W, const T1& t) {
             }
           }
         } else {
-          for (int i = lane; i < t.nC; i += 32) ncnt[i] = 0;
+          ROLLED for (int i = lane; i < t.nC; i += 32) ncnt[i] = 0;
         }
         __syncwarp();
-        t1_rows_of(W, cur, level, [&](bool valid, int, int pos) {
-          if (!valid) return;
-          int p = aadj[pos];
-          if (p >= 0) atomicAdd(&ncnt[p], 1);
-        });
+        t1_walk(t.nL, cur, level, kOpAdd, level, nullptr);
       } else {
-        t1_rows_at_level(W, t, level - 1, [&](bool valid, int, int pos) {
-          if (!valid) return;
-          int p = aadj[pos];
-          if (p >= 0) atomicSub(&ncnt[p], 1);
-        });
+        t1_walk(t.nL, -1, level - 1, kOpSub, level, nullptr);
       }
       __syncwarp();
       // Maximality (src/IterFinderGpu.h:252-261): a candidate covering the new
@@ -1612,7 +2670,7 @@ __device__ void tier1_run(Warp& W, const T1& t) {
       {
         const int lstar = (int)(best & 0xffffffffu);
         const int mb = aoff[lstar], me = aoff[lstar + 1];
-        for (int j = mb + lane; j < me; j += 32) {
+        ROLLED for (int j = mb + lane; j < me; j += 32) {
           const int i = aadj[j];
           if (i >= 0 && ncnt[i] == kept) {
             sR += ckey[i];
@@ -1624,46 +2682,36 @@ __device__ void tier1_run(Warp& W, const T1& t) {
         }
       }
       ism = __all_sync(kFull, ism);
-      sR = warp_sum(sR) + t.sRtask;
-      nR = warp_sum(nR) + t.nRtask;
+      sR = warp_sum64(sR) + t.sRtask;
+      nR = warp_sum64(nR) + t.nRtask;
       if (ism) {
-        W.cnt += 1;
-        W.hash += biclique_hash(*W.gp, sL, (uint64_t)kept, sR, nR);
+        acc(W.cnt, 1);
+        acc(W.hash, biclique_hash(*W.gp, sL, (uint64_t)kept, sR, nR));
         if (emitting)
-          emit_level(W.ctl, emit_dst(W.p), W.gid, kept, t.nL, llevel, level, t.L);
+          emit_level(s_blk.ctl, emit_dst(*s_blk.p), W.gid, kept, t.nL, llevel, level, t.L);
       } else {
-        W.nonmax += 1;
+        acc(W.nonmax, 1);
       }
       __syncwarp();
       if (ism && kept > 1) {
-        if (kept <= t2max) {
-          t1_handoff(W, t, cur, level, kept, sR, nR);
-        } else {
+        if (kept > t2max || !t1_handoff(t, cur, level, kept, sR, nR)) {
           uint32_t* nbits = level_bits(W, level + 1);
           // The candidates the kept rows meet, as a bitmap: the next level's
           // own one, or (deeper levels) the warp's global touch bitmap, built
           // only when the child may be shared out.
           uint32_t* cbits = nbits;
           const bool want = t1_export_wanted(W, kept, kent);
-          if (!cbits && want) cbits = W.gseen;
+          if (!cbits && want) cbits = W.gseen();
           if (cbits) {
-            t1_rows_of(W, cur, level, [&](bool valid, int, int pos) {
-              if (!valid) return;
-              const int p = aadj[pos];
-              if (p >= 0) atomicOr(&cbits[p >> 5], 1u << (p & 31));
-            });
+            t1_walk(t.nL, cur, level, kOpSetBit, level, cbits);
             __threadfence_block();
             __syncwarp();
           }
           const bool exported =
-              want && cbits && t1_try_export(W, t, cur, level, kept, kent, sR, nR, cbits);
+              want && cbits && t1_try_export(t, cur, level, kept, kent, sR, nR, cbits);
           if (cbits && (exported || cbits != nbits)) {
             // back to clear: a shared-out child's level bitmap, or the touch bitmap
-            t1_rows_of(W, cur, level, [&](bool valid, int, int pos) {
-              if (!valid) return;
-              const int p = aadj[pos];
-              if (p >= 0) cbits[p >> 5] = 0u;
-            });
+            t1_walk(t.nL, cur, level, kOpClearBit, level, cbits);
             __syncwarp();
           }
           if (exported) {
@@ -1682,7 +2730,7 @@ __device__ void tier1_run(Warp& W, const T1& t) {
       }
       if (lane == 0) stack[level - 1] = cur + 1;
       __syncwarp();
-      t1_pop(W, t, cur, level);
+      t1_pop(t.nL, cur, level);
     } else {
       --level;
       if (level > 0) {
@@ -1690,14 +2738,10 @@ __device__ void tier1_run(Warp& W, const T1& t) {
         __syncwarp();
         uint32_t* cbits = level_bits(W, level + 1);
         if (cbits) {  // the finished level's bitmap back to clear
-          t1_rows_of(W, cur, level, [&](bool valid, int, int pos) {
-            if (!valid) return;
-            const int p = aadj[pos];
-            if (p >= 0) cbits[p >> 5] = 0u;
-          });
+          t1_walk(t.nL, cur, level, kOpClearBit, level, cbits);
           __syncwarp();
         }
-        t1_pop(W, t, cur, level);
+        t1_pop(t.nL, cur, level);
         if (lane == 0) stack[level - 1] = cur + 1;
         __syncwarp();
       }
@@ -1705,11 +2749,15 @@ __device__ void tier1_run(Warp& W, const T1& t) {
   }
 }
 
+__device__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count);
+__device__ void t1_transpose(int entries, int nC);
+
 // Runs a counts-tier child exported by t1_try_export: the frame is rebuilt
 // from the vertex lists (local adjacency from the graph's U -> V rows, the
 // counts of each candidate inside L'), then the counts tier runs it from its
 // first level.  The child's own biclique was counted by the exporter.
-__device__ void tier1_from_slot(Warp& W, int slot) {
+__device__ __noinline__ void tier1_from_slot(int slot) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
   int32_t* sp = slot_ptr(W, slot);
   volatile const int32_t* vh = sp;
@@ -1717,52 +2765,54 @@ __device__ void tier1_from_slot(Warp& W, int slot) {
   const int32_t gid = vh[3];
   const uint64_t sR = (uint64_t)(uint32_t)vh[4] | ((uint64_t)(uint32_t)vh[5] << 32);
   const uint64_t nR = (uint32_t)vh[6];
-  int32_t* lv = W.A(W.sl.lv);
-  int32_t* cv = W.A(W.sl.cv);
-  const bool fits = n <= W.sl.capL && m <= W.sl.capC;
+  int32_t* lv = W.A(W.sl().lv);
+  int32_t* cv = W.A(W.sl().cv);
+  const bool fits = n <= W.sl().capL && m <= W.sl().capC;
   if (fits) {
     const unsigned* src = reinterpret_cast<const unsigned*>(sp + kFrameHdr);
-    for (int i = lane; i < n; i += 32) lv[i] = (int32_t)__ldcg(src + i);
-    for (int i = lane; i < m; i += 32) cv[i] = (int32_t)__ldcg(src + n + i);
+    ROLLED for (int i = lane; i < n; i += 32) lv[i] = (int32_t)__ldcg(src + i);
+    ROLLED for (int i = lane; i < m; i += 32) cv[i] = (int32_t)__ldcg(src + n + i);
   }
   __syncwarp();
   if (lane == 0) slot_free(W, slot);
   __syncwarp();
   if (!fits) {
-    set_status(W.ctl, kStCapacity, ((unsigned long long)4 << 32) | (unsigned)m);
+    set_status(s_blk.ctl, kStCapacity, ((unsigned long long)4 << 32) | (unsigned)m);
     return;
   }
+  __syncwarp();
   W.gid = gid;
   W.gp = graph_at(W, gid);
+  __syncwarp();
   const DevGraph& g = *W.gp;
-  int32_t* map = W.A(W.sl.map);
-  int32_t* aoff = W.A(W.sl.aoff);
-  int32_t* aadj = W.A(W.sl.aadj);
-  int32_t* ent = W.A(W.sl.ent);
-  int32_t* ncnt = W.A(W.sl.ncnt);
-  int32_t* bound = W.A(W.sl.bound);
-  int32_t* coff = W.A(W.sl.coff);
-  int32_t* fill = W.A(W.sl.fill);
-  int32_t* cadj = W.A(W.sl.cadj);
-  int32_t* sidx = W.A(W.sl.sidx);
-  int32_t* llevel = W.A(W.sl.llevel);
-  uint64_t* ckey = W.A64(W.sl.ckey);
+  int32_t* map = W.A(W.sl().map);
+  int32_t* aoff = W.A(W.sl().aoff);
+  int32_t* aadj = W.A(W.sl().aadj);
+  int32_t* ent = W.A(W.sl().ent);
+  int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
+  int32_t* coff = W.A(W.sl().coff);
+  int32_t* fill = W.A(W.sl().fill);
+  int32_t* cadj = W.A(W.sl().cadj);
+  int32_t* sidx = W.A(W.sl().sidx);
+  int32_t* llevel = W.A(W.sl().llevel);
+  uint64_t* ckey = W.A64(W.sl().ckey);
   uint64_t t0 = globaltimer_ns();
   int run = 0;
-  for (int c0 = 0; c0 < n; c0 += 32) {
+  ROLLED for (int c0 = 0; c0 < n; c0 += 32) {
     const int l = c0 + lane;
     const int d = l < n ? g.rev_off[lv[l] + 1] - g.rev_off[lv[l]] : 0;
     int tot;
-    const int ex = warp_excl_scan(d, &tot);
+    const int ex = excl_scan(d, &tot);
     if (l < n) aoff[l] = run + ex;
     run += tot;
   }
   if (lane == 0) aoff[n] = run;
-  if (run > W.sl.capS) {
-    set_status(W.ctl, kStCapacity, ((unsigned long long)5 << 32) | (unsigned)run);
+  if (run > W.sl().capS) {
+    set_status(s_blk.ctl, kStCapacity, ((unsigned long long)5 << 32) | (unsigned)run);
     return;
   }
-  for (int i = lane; i < m; i += 32) {
+  ROLLED for (int i = lane; i < m; i += 32) {
     map[cv[i]] = i + 1;
     ncnt[i] = 0;
     bound[i] = kFree;
@@ -1770,57 +2820,18 @@ __device__ void tier1_from_slot(Warp& W, int slot) {
     sidx[i] = -1;
     ckey[i] = g.vkey[cv[i]];
   }
-  for (int l = lane; l < n; l += 32) llevel[l] = 0;
+  ROLLED for (int l = lane; l < n; l += 32) llevel[l] = 0;
   __threadfence_block();
   __syncwarp();
-  flat_rows(
-      n,
-      [&](int r, int& beg, int& len) {
-        const int u = lv[r];
-        beg = g.rev_off[u];
-        len = g.rev_off[u + 1] - beg;
-      },
-      [&](bool valid, int r, int pos) {
-        if (!valid) return;
-        const int u = lv[r];
-        const int off = aoff[r] + (pos - g.rev_off[u]);
-        const int p = map[__ldg(g.rev_col + pos)] - 1;
-        aadj[off] = p;
-        ent[off] = r;
-        if (p >= 0) atomicAdd(&ncnt[p], 1);
-      });
+  lay_out_rows(lv, n, run, false);
+  ROLLED for (int e = lane; e < run; e += 32) {
+    const int p = map[aadj[e]] - 1;
+    aadj[e] = p;
+    if (p >= 0) atomicAdd(&ncnt[p], 1);
+  }
   __threadfence_block();
   __syncwarp();
-  {
-    int acc = 0;
-    for (int c0 = 0; c0 < m; c0 += 32) {
-      const int i = c0 + lane;
-      const int c = i < m ? ncnt[i] : 0;
-      int tot;
-      const int ex = warp_excl_scan(c, &tot);
-      if (i < m) coff[i] = acc + ex;
-      acc += tot;
-    }
-    if (lane == 0) coff[m] = acc;
-  }
-  __syncwarp();
-  for (int j0 = 0; j0 < run; j0 += 128) {
-    int pp[4], rr[4], ss[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int j = j0 + k * 32 + lane;
-      pp[k] = j < run ? aadj[j] : -1;
-      rr[k] = j < run ? ent[j] : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) ss[k] = pp[k] >= 0 ? atomicAdd(&fill[pp[k]], 1) : 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (pp[k] >= 0) cadj[coff[pp[k]] + ss[k]] = rr[k];
-  }
-  __syncwarp();
-  for (int i = lane; i < m; i += 32) fill[i] = 0;
-  __syncwarp();
+  t1_transpose(run, m);
   T1 t1;
   t1.L = lv;
   t1.nL = n;
@@ -1831,11 +2842,11 @@ __device__ void tier1_from_slot(Warp& W, int slot) {
   t1.nRtask = nR;
   const uint64_t t1s = globaltimer_ns();
   const uint64_t t2_before = W.ns_t2;
-  tier1_run(W, t1);
-  W.ns_t1 += (globaltimer_ns() - t1s) - (W.ns_t2 - t2_before);
+  tier1_run(t1);
+  acc(W.ns_t1, (globaltimer_ns() - t1s) - (W.ns_t2 - t2_before));
   (void)t0;
   __syncwarp();
-  for (int i = lane; i < m; i += 32) map[cv[i]] = 0;
+  ROLLED for (int i = lane; i < m; i += 32) map[cv[i]] = 0;
   __syncwarp();
 }
 
@@ -1852,28 +2863,29 @@ __device__ __forceinline__ unsigned long long slot_free_tag(unsigned long long g
   return 2ULL * (gp / (unsigned long long)cap);
 }
 
-__device__ bool queue_pop(Warp& W, Task* out) {
+__device__ __noinline__ bool queue_pop(Task* out) {
+  Warp& W = this_warp();
   // lane 0 only
-  EnumCtl* ctl = W.ctl;
+  EnumCtl* ctl = s_blk.ctl;
   volatile unsigned long long* vh = &ctl->q_head;
   volatile unsigned long long* vt = &ctl->q_tail;
   unsigned long long h = *vh;
   if (h >= *vt) return false;
   if (atomicCAS(&ctl->q_head, h, h + 1) != h) return false;
-  const int cap = W.p.queue_cap;
+  const int cap = s_blk.p->queue_cap;
   unsigned long long slot = h % (unsigned long long)cap;
-  volatile unsigned long long* st = W.q_seq + slot;
+  volatile unsigned long long* st = s_blk.q_seq + slot;
   const unsigned long long full = slot_free_tag(h, cap) + 1;
   int64_t spins = 0;
   while (*st != full) {
-    if (++spins > W.p.slot_spin_limit) {
+    if (++spins > s_blk.p->slot_spin_limit) {
       set_status(ctl, kStQueue, h);
       return false;
     }
     __nanosleep(64);
   }
   __threadfence();
-  volatile int32_t* src = reinterpret_cast<volatile int32_t*>(W.q_tasks + slot);
+  volatile int32_t* src = reinterpret_cast<volatile int32_t*>(s_blk.q_tasks + slot);
   out->v[0] = src[0];
   out->v[1] = src[1];
   out->v[2] = src[2];
@@ -1882,7 +2894,7 @@ __device__ bool queue_pop(Warp& W, Task* out) {
   out->part = src[5];
   out->parts = src[6];
   __threadfence();
-  atomicExch(W.q_seq + slot, full + 1);  // free for round h/cap + 1
+  atomicExch(s_blk.q_seq + slot, full + 1);  // free for round h/cap + 1
   atomicAdd(&ctl->q_used, (unsigned long long)-1LL);
   return true;
 }
@@ -1892,8 +2904,8 @@ __device__ bool queue_pop(Warp& W, Task* out) {
 template <typename Make>
 __device__ bool queue_push_n(Warp& W, unsigned long long n, Make make) {
   const int lane = (int)lane_id();
-  EnumCtl* ctl = W.ctl;
-  const int cap = W.p.queue_cap;
+  EnumCtl* ctl = s_blk.ctl;
+  const int cap = s_blk.p->queue_cap;
   unsigned long long pos = 0;
   int ok = 0;
   if (lane == 0) {
@@ -1910,15 +2922,15 @@ __device__ bool queue_push_n(Warp& W, unsigned long long n, Make make) {
   ok = __shfl_sync(kFull, ok, 0);
   if (!ok) return false;
   pos = __shfl_sync(kFull, pos, 0);
-  for (unsigned long long i = lane; i < n; i += 32) {
+  ROLLED for (unsigned long long i = lane; i < n; i += 32) {
     unsigned long long gp = pos + i;
     unsigned long long slot = gp % (unsigned long long)cap;
-    volatile unsigned long long* st = W.q_seq + slot;
+    volatile unsigned long long* st = s_blk.q_seq + slot;
     const unsigned long long free_tag = slot_free_tag(gp, cap);
     int64_t spins = 0;
     bool ready = true;
     while (*st != free_tag) {
-      if (++spins > W.p.slot_spin_limit) {
+      if (++spins > s_blk.p->slot_spin_limit) {
         set_status(ctl, kStQueue, gp);
         ready = false;
         break;
@@ -1926,17 +2938,18 @@ __device__ bool queue_push_n(Warp& W, unsigned long long n, Make make) {
       __nanosleep(64);
     }
     if (!ready) continue;  // the run is aborting; the slot stays unwritten
-    W.q_tasks[slot] = make((int)i);
+    s_blk.q_tasks[slot] = make((int)i);
     __threadfence();
-    atomicExch(W.q_seq + slot, free_tag + 1);
+    atomicExch(s_blk.q_seq + slot, free_tag + 1);
   }
   __syncwarp();
   return true;
 }
 
 // Pushes children task + {cv[i]} for i in [nq, nC); false if the ring is full.
-__device__ bool queue_push_children(Warp& W, const Task& t, int k, int nq, int nC) {
-  const int32_t* cv = W.A(W.sl.cv);
+__device__ __noinline__ bool queue_push_children(const Task& t, int k, int nq, int nC) {
+  Warp& W = this_warp();
+  const int32_t* cv = W.A(W.sl().cv);
   return queue_push_n(W, (unsigned long long)(nC - nq), [&](int i) {
     Task c = t;
     c.v[k] = cv[nq + i];
@@ -1946,7 +2959,8 @@ __device__ bool queue_push_children(Warp& W, const Task& t, int k, int nq, int n
 }
 
 // Pushes parts 1 .. m-1 of root task t; false if the ring is full.
-__device__ bool queue_push_parts(Warp& W, const Task& t, int m) {
+__device__ __noinline__ bool queue_push_parts(const Task& t, int m) {
+  Warp& W = this_warp();
   return queue_push_n(W, (unsigned long long)(m - 1), [&](int i) {
     Task c = t;
     c.part = i + 1;
@@ -1959,13 +2973,14 @@ __device__ bool queue_push_parts(Warp& W, const Task& t, int m) {
 // big warps claim from (the other warps' scratch cannot hold the root).
 // They count as pending before the record becomes visible.  False if the
 // record list is full (the root then runs whole).
-__device__ bool big_parts_push(Warp& W, int v, int m) {
+__device__ __noinline__ bool big_parts_push(int v, int m) {
+  Warp& W = this_warp();
   int ok = 0;
   if (lane_id() == 0) {
-    const unsigned long long i = atomicAdd(&W.ctl->n_big_parts, 1ULL);
-    if (i < (unsigned long long)W.p.big_parts_cap) {
-      atomicAdd(&W.ctl->pending, (unsigned long long)(m - 1));
-      int32_t* r = W.p.big_parts + 4 * i;
+    const unsigned long long i = atomicAdd(&s_blk.ctl->n_big_parts, 1ULL);
+    if (i < (unsigned long long)s_blk.p->big_parts_cap) {
+      atomicAdd(&s_blk.ctl->pending, (unsigned long long)(m - 1));
+      int32_t* r = s_blk.p->big_parts + 4 * i;
       r[0] = v;
       r[1] = m;
       r[2] = 1;  // part 0 runs on this warp
@@ -1978,12 +2993,13 @@ __device__ bool big_parts_push(Warp& W, int v, int m) {
 }
 
 // Claims a part of a listed big root (lane 0 of a big warp).
-__device__ bool big_parts_claim(Warp& W, Task* t) {
-  EnumCtl* c = W.ctl;
+__device__ __noinline__ bool big_parts_claim(Task* t) {
+  Warp& W = this_warp();
+  EnumCtl* c = s_blk.ctl;
   const unsigned long long n = min(*(volatile unsigned long long*)&c->n_big_parts,
-                                   (unsigned long long)W.p.big_parts_cap);
-  for (unsigned long long i = *(volatile unsigned long long*)&c->big_parts_head; i < n; ++i) {
-    int32_t* r = W.p.big_parts + 4 * i;
+                                   (unsigned long long)s_blk.p->big_parts_cap);
+  ROLLED for (unsigned long long i = *(volatile unsigned long long*)&c->big_parts_head; i < n; ++i) {
+    int32_t* r = s_blk.p->big_parts + 4 * i;
     if (*(volatile int32_t*)&r[3] == 0) continue;  // being written
     const int m = *(volatile int32_t*)&r[1];
     if (*(volatile int32_t*)&r[2] < m) {
@@ -2007,8 +3023,8 @@ __device__ bool big_parts_claim(Warp& W, Task* t) {
 // Pushes one task (lane-uniform); false if the ring is full.
 __device__ bool queue_push_one(Warp& W, const Task& t) {
   const int lane = (int)lane_id();
-  EnumCtl* ctl = W.ctl;
-  const int cap = W.p.queue_cap;
+  EnumCtl* ctl = s_blk.ctl;
+  const int cap = s_blk.p->queue_cap;
   int ok = 0;
   if (lane == 0) {
     unsigned long long used = atomicAdd(&ctl->q_used, 1ULL);
@@ -2019,12 +3035,12 @@ __device__ bool queue_push_one(Warp& W, const Task& t) {
       graph_spawned(W, 1ULL);
       unsigned long long gp = atomicAdd(&ctl->q_tail, 1ULL);
       unsigned long long slot = gp % (unsigned long long)cap;
-      volatile unsigned long long* st = W.q_seq + slot;
+      volatile unsigned long long* st = s_blk.q_seq + slot;
       const unsigned long long free_tag = slot_free_tag(gp, cap);
       int64_t spins = 0;
       ok = 1;
       while (*st != free_tag) {
-        if (++spins > W.p.slot_spin_limit) {
+        if (++spins > s_blk.p->slot_spin_limit) {
           set_status(ctl, kStQueue, gp);
           ok = 2;
           break;
@@ -2032,9 +3048,9 @@ __device__ bool queue_push_one(Warp& W, const Task& t) {
         __nanosleep(64);
       }
       if (ok == 1) {
-        W.q_tasks[slot] = t;
+        s_blk.q_tasks[slot] = t;
         __threadfence();
-        atomicExch(W.q_seq + slot, free_tag + 1);
+        atomicExch(s_blk.q_seq + slot, free_tag + 1);
       }
     }
   }
@@ -2042,17 +3058,118 @@ __device__ bool queue_push_one(Warp& W, const Task& t) {
   return ok != 0;  // 2: the run is aborting; the task counts as handed over
 }
 
+// Lays the two-hop multiset of L out in order: the V ids met into aadj, each
+// one's L position into ent, nL rows of the graph's U -> V lists end to end.
+// With `count`, counts every id in the dense map on the way and lists the ids
+// met (each once, at most capC of them) in `touched`; returns their number.
+__device__ __noinline__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count) {
+  Warp& W = this_warp();
+  const int lane = (int)lane_id();
+  const DevGraph& g = *W.gp;
+  int32_t* map = W.A(W.sl().map);
+  int32_t* touched = W.A(W.sl().touched);
+  int32_t* aadj = W.A(W.sl().aadj);
+  int32_t* ent = W.A(W.sl().ent);
+  const int capC = W.sl().capC;
+  const int vwords = (g.nV + 31) >> 5;
+  const int32_t* rev_off = g.rev_off;
+  const int32_t* rev_col = g.rev_col;
+  uint32_t* gseen = W.gseen();
+  // Large set-up without the shared bitmap: fire-and-forget counts and touch
+  // bits, then the touched list in id order from the bitmap.
+  const bool scan = count && use_gseen(W, entries, vwords);
+  if (count && !scan) clear_seen(W, vwords);
+  int nt = 0;
+  flat_rows(
+      nL,
+      [&](int r, int& beg, int& len) {
+        const int u = L[r];
+        beg = rev_off[u];
+        len = rev_off[u + 1] - beg;
+      },
+      [&](bool valid, int pos) { return valid ? __ldg(rev_col + pos) : 0; },
+      [&](bool valid, int r, int k, int w) {
+        bool isnew = false;
+        if (valid) {
+          aadj[k] = w;
+          ent[k] = r;
+          if (scan) {
+            atomicAdd(&map[w], 1);
+            atomicOr(&gseen[w >> 5], 1u << (w & 31));
+          } else if (count) {
+            isnew = count_first(W, map, w);
+          }
+        }
+        const unsigned bal = __ballot_sync(kFull, isnew);
+        const int at = nt + __popc(bal & lanemask_lt());
+        if (isnew && at < capC) touched[at] = w;
+        nt += __popc(bal);
+      });
+  if (scan) {
+    __threadfence_block();
+    __syncwarp();
+    nt = collect_bits(gseen, vwords, touched, capC);
+  } else if (count) {
+    counts_done(W, touched, min(nt, capC));
+  }
+  __syncwarp();
+  return nt;
+}
+
+// The transpose of the local adjacency: cadj lists, from coff[i], the L
+// positions of candidate i (aadj: candidate of each entry, ent: its position;
+// fill: all-zero, and again so on return).  Every lane has four slot
+// reservations in flight before it uses any.
+__device__ __noinline__ void t1_transpose(int entries, int nC) {
+  Warp& W = this_warp();
+  const int lane = (int)lane_id();
+  const int32_t* aadj = W.A(W.sl().aadj);
+  const int32_t* ent = W.A(W.sl().ent);
+  const int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* coff = W.A(W.sl().coff);
+  int32_t* fill = W.A(W.sl().fill);
+  int32_t* cadj = W.A(W.sl().cadj);
+  int run = 0;
+  ROLLED for (int c0 = 0; c0 < nC; c0 += 32) {
+    const int i = c0 + lane;
+    int tot;
+    const int ex = excl_scan(i < nC ? ncnt[i] : 0, &tot);
+    if (i < nC) coff[i] = run + ex;
+    run += tot;
+  }
+  if (lane == 0) coff[nC] = run;
+  __syncwarp();
+  ROLLED for (int j0 = 0; j0 < entries; j0 += 128) {
+    int pp[4], rr[4], ss[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = j0 + k * 32 + lane;
+      pp[k] = j < entries ? aadj[j] : -1;
+      rr[k] = j < entries ? ent[j] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ss[k] = pp[k] >= 0 ? atomicAdd(&fill[pp[k]], 1) : 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (pp[k] >= 0) cadj[coff[pp[k]] + ss[k]] = rr[k];
+  }
+  __syncwarp();
+  ROLLED for (int i = lane; i < nC; i += 32) fill[i] = 0;
+  __syncwarp();
+}
+
 // ---------------------------------------------------------------------------
 // Task set-up (IterFinderWithMultipleVertex) and dispatch.
-__device__ void run_task(Warp& W, const Task& t) {
+__device__ __noinline__ void run_task(const Task& t) {
+  Warp& W = this_warp();
   const int lane = (int)lane_id();
   const DevGraph& g = *W.gp;
   int k = 1;
   while (k < 4 && t.v[k] >= 0) ++k;
   const int last = t.v[k - 1];
-  int32_t* map = W.A(W.sl.map);
-  int32_t* touched = W.A(W.sl.touched);
-  int32_t* lv = W.A(W.sl.lv);
+  int32_t* map = W.A(W.sl().map);
+  int32_t* touched = W.A(W.sl().touched);
+  int32_t* lv = W.A(W.sl().lv);
 
   // ---- L = common neighbours of the task vertices ----
   const int32_t* L;
@@ -2063,7 +3180,7 @@ __device__ void run_task(Warp& W, const Task& t) {
   } else {
     // Intersect: probe the smallest row against the others.
     int best = 0, bestlen = 0x7fffffff;
-    for (int i = 0; i < k; ++i) {
+    ROLLED for (int i = 0; i < k; ++i) {
       int len = g.row_off[t.v[i] + 1] - g.row_off[t.v[i]];
       if (len < bestlen) {
         bestlen = len;
@@ -2072,11 +3189,11 @@ __device__ void run_task(Warp& W, const Task& t) {
     }
     const int32_t* sm = g.col + g.row_off[t.v[best]];
     int n = 0;
-    for (int b0 = 0; b0 < bestlen; b0 += 32) {
+    ROLLED for (int b0 = 0; b0 < bestlen; b0 += 32) {
       int j = b0 + lane;
       bool in = j < bestlen;
       int u = in ? __ldg(sm + j) : 0;
-      for (int i = 0; i < k && in; ++i) {
+      ROLLED for (int i = 0; i < k && in; ++i) {
         if (i == best) continue;
         const int32_t* row = g.col + g.row_off[t.v[i]];
         in = contains_sorted(row, g.row_off[t.v[i] + 1] - g.row_off[t.v[i]], u);
@@ -2090,16 +3207,16 @@ __device__ void run_task(Warp& W, const Task& t) {
     nL = n;
   }
   if (nL == 0) return;
-  if (nL > W.sl.capL) {
-    set_status(W.ctl, kStCapacity, ((unsigned long long)1 << 32) | (unsigned)nL);
+  if (nL > W.sl().capL) {
+    set_status(s_blk.ctl, kStCapacity, ((unsigned long long)1 << 32) | (unsigned)nL);
     return;
   }
 
   // ---- two-hop multiset: counts in the per-warp dense map ----
-  int32_t* aoff = W.A(W.sl.aoff);
+  int32_t* aoff = W.A(W.sl().aoff);
   {
     int run = 0;
-    for (int c0 = 0; c0 < nL; c0 += 32) {
+    ROLLED for (int c0 = 0; c0 < nL; c0 += 32) {
       int l = c0 + lane;
       int d = 0;
       if (l < nL) {
@@ -2107,69 +3224,32 @@ __device__ void run_task(Warp& W, const Task& t) {
         d = g.rev_off[u + 1] - g.rev_off[u];
       }
       int tot;
-      int ex = warp_excl_scan(d, &tot);
+      int ex = excl_scan(d, &tot);
       if (l < nL) aoff[l] = run + ex;
       run += tot;
     }
     if (lane == 0) aoff[nL] = run;
-    if (run > W.sl.capS) {
-      set_status(W.ctl, kStCapacity, ((unsigned long long)2 << 32) | (unsigned)run);
+    if (run > W.sl().capS) {
+      set_status(s_blk.ctl, kStCapacity, ((unsigned long long)2 << 32) | (unsigned)run);
       return;
     }
   }
   __syncwarp();
-  int nt = 0;
-  const int vwords = (g.nV + 31) >> 5;
-  if (use_gseen(W, aoff[nL], vwords)) {
-    // Large set-up without the shared bitmap: fire-and-forget counts and
-    // touch bits, then the touched list in id order from the bitmap.
-    flat_rows(
-        nL,
-        [&](int r, int& beg, int& len) {
-          int u = L[r];
-          beg = g.rev_off[u];
-          len = g.rev_off[u + 1] - beg;
-        },
-        [&](bool valid, int, int pos) {
-          if (!valid) return;
-          const int w = __ldg(g.rev_col + pos);
-          atomicAdd(&map[w], 1);
-          atomicOr(&W.gseen[w >> 5], 1u << (w & 31));
-        });
-    __threadfence_block();
-    __syncwarp();
-    nt = collect_bits(W.gseen, vwords, touched, W.sl.capC);
-  } else {
-    flat_rows(
-        nL,
-        [&](int r, int& beg, int& len) {
-          int u = L[r];
-          beg = g.rev_off[u];
-          len = g.rev_off[u + 1] - beg;
-        },
-        [&](bool valid, int, int pos) {
-          int w = valid ? __ldg(g.rev_col + pos) : 0;
-          bool isnew = valid && count_first(W, map, w);
-          unsigned bal = __ballot_sync(kFull, isnew);
-          if (isnew && nt + __popc(bal & lanemask_lt()) < W.sl.capC)
-            touched[nt + __popc(bal & lanemask_lt())] = w;
-          nt += __popc(bal);
-        });
-    counts_done(W, touched, min(nt, W.sl.capC));
-  }
-  if (nt > W.sl.capC) {
+  const int entries = aoff[nL];
+  const int nt = lay_out_rows(L, nL, entries, true);
+  if (nt > W.sl().capC) {
     // Vertices beyond the touched list's room keep counts: clear the whole
     // map (the launch is failing; this keeps the invariant for the record).
-    set_status(W.ctl, kStCapacity, ((unsigned long long)3 << 32) | (unsigned)nt);
-    for (int i = lane; i < g.nV; i += 32) map[i] = 0;
+    set_status(s_blk.ctl, kStCapacity, ((unsigned long long)3 << 32) | (unsigned)nt);
+    ROLLED for (int i = lane; i < g.nV; i += 32) map[i] = 0;
     __syncwarp();
     return;
   }
 
   // ---- classify: R (count == |L|), Q (w < last), P (w > last) ----
-  int32_t* cv = W.A(W.sl.cv);
-  int32_t* ncnt = W.A(W.sl.ncnt);
-  int32_t* bound = W.A(W.sl.bound);
+  int32_t* cv = W.A(W.sl().cv);
+  int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
   uint64_t sR = 0;
   unsigned long long nR = 0;
   int nq = 0, np = 0, nend = 0;
@@ -2180,17 +3260,18 @@ __device__ void run_task(Warp& W, const Task& t) {
   // pushes the candidates of this part; those before it act as Q, those after
   // it stay candidates of the children.
   int part = t.part, parts = t.parts;
-  int cntQ = 0, cntPre = 0, cntIn = 0;
+  int cntQ = 0, cntPre = 0, cntIn = 0, cntM = 0;
   {
     int cntC = 0;
     bool r_below = false;
-    for (int b0 = 0; b0 < nt; b0 += 32) {
+    ROLLED for (int b0 = 0; b0 < nt; b0 += 32) {
       int i = b0 + lane;
       bool valid = i < nt;
       int w = valid ? touched[i] : 0;
       int c = valid ? map[w] : 0;
       bool isC = valid && c != nL;
       cntC += __popc(__ballot_sync(kFull, isC));
+      cntM += __popc(__ballot_sync(kFull, isC && c >= 2));
       cntQ += __popc(__ballot_sync(kFull, isC && w < last));
       r_below |= __ballot_sync(kFull, valid && c == nL && w < last) != 0u;
     }
@@ -2198,21 +3279,21 @@ __device__ void run_task(Warp& W, const Task& t) {
     const int np_all = cntC - cntQ;
     // A heavy maximal root is split into parts before its C is laid out.
     // Its first level costs about |P| pushes, each a pass over all of C.
-    if (k == 1 && parts == 0 && !r_below && W.p.range_work > 0 &&
-        np_all >= 2 * W.p.range_chunk &&
-        (long long)np_all * cntC > (long long)W.p.range_work) {
-      const int m = min((np_all + W.p.range_chunk - 1) / W.p.range_chunk, kMaxParts);
+    if (k == 1 && parts == 0 && !r_below && s_blk.p->range_work > 0 &&
+        np_all >= 2 * s_blk.p->range_chunk &&
+        (long long)np_all * cntC > (long long)s_blk.p->range_work) {
+      const int m = min((np_all + s_blk.p->range_chunk - 1) / s_blk.p->range_chunk, kMaxParts);
       // A listed big root's parts go to big warps only; other roots' parts
       // fit every warp and take the common queue.
-      const bool big_root = W.p.n_big_warps > 0 && W.p.big_flag[last];
-      if (big_root ? big_parts_push(W, last, m) : queue_push_parts(W, t, m)) {
+      const bool big_root = s_blk.p->n_big_warps > 0 && s_blk.p->big_flag[last];
+      if (big_root ? big_parts_push(last, m) : queue_push_parts(t, m)) {
         part = 0;
         parts = m;
-        W.splits += 1;
+        acc(W.splits, 1);
       }
     }
     if (parts > 1) {
-      for (int b0 = 0; b0 < nt; b0 += 32) {
+      ROLLED for (int b0 = 0; b0 < nt; b0 += 32) {
         int i = b0 + lane;
         bool valid = i < nt;
         int w = valid ? touched[i] : 0;
@@ -2227,7 +3308,7 @@ __device__ void run_task(Warp& W, const Task& t) {
   }
   {
     int oQ = 0, oPre = cntQ, oIn = cntQ + cntPre, oPost = cntQ + cntPre + cntIn;
-    for (int b0 = 0; b0 < nt; b0 += 32) {
+    ROLLED for (int b0 = 0; b0 < nt; b0 += 32) {
       int i = b0 + lane;
       bool valid = i < nt;
       int w = valid ? touched[i] : 0;
@@ -2271,8 +3352,8 @@ __device__ void run_task(Warp& W, const Task& t) {
     W.shape = (unsigned long long)(unsigned)nC | ((unsigned long long)(part & 0xffff) << 32) |
               ((unsigned long long)(parts & 0xffff) << 48);
   }
-  sR = warp_sum(sR);
-  nR = warp_sum(nR);
+  sR = warp_sum64(sR);
+  nR = warp_sum64(nR);
   viol_first = warp_min_i(viol_first);
   __syncwarp();
 
@@ -2283,7 +3364,7 @@ __device__ void run_task(Warp& W, const Task& t) {
       ism = false;  // R[0] != root
     } else {
       // Every R vertex below `last` must already cover L_parent.
-      int32_t* lp = W.A(W.sl.lp);
+      int32_t* lp = W.A(W.sl().lp);
       const int32_t* Lpar;
       int nLp;
       if (k == 2) {
@@ -2293,11 +3374,11 @@ __device__ void run_task(Warp& W, const Task& t) {
         const int32_t* r0 = g.col + g.row_off[t.v[0]];
         int len0 = g.row_off[t.v[0] + 1] - g.row_off[t.v[0]];
         int n = 0;
-        for (int b0 = 0; b0 < len0; b0 += 32) {
+        ROLLED for (int b0 = 0; b0 < len0; b0 += 32) {
           int j = b0 + lane;
           bool in = j < len0;
           int u = in ? __ldg(r0 + j) : 0;
-          for (int i = 1; i < k - 1 && in; ++i)
+          ROLLED for (int i = 1; i < k - 1 && in; ++i)
             in = contains_sorted(g.col + g.row_off[t.v[i]],
                                  g.row_off[t.v[i] + 1] - g.row_off[t.v[i]], u);
           unsigned bal = __ballot_sync(kFull, in);
@@ -2308,7 +3389,7 @@ __device__ void run_task(Warp& W, const Task& t) {
         Lpar = lp;
         nLp = n;
       }
-      for (int b0 = 0; b0 < nt && ism; b0 += 32) {
+      ROLLED for (int b0 = 0; b0 < nt && ism; b0 += 32) {
         int i = b0 + lane;
         int w = i < nt ? touched[i] : 0;
         bool cand = i < nt && w < last && map[w] == 0;  // R vertex below last
@@ -2319,7 +3400,7 @@ __device__ void run_task(Warp& W, const Task& t) {
           bal &= bal - 1;
           int ww = __shfl_sync(kFull, w, src);
           bool trivially = false;
-          for (int q = 0; q < k - 1; ++q) trivially |= (t.v[q] == ww);
+          ROLLED for (int q = 0; q < k - 1; ++q) trivially |= (t.v[q] == ww);
           if (trivially) continue;
           const int32_t* rw = g.col + g.row_off[ww];
           int dw = g.row_off[ww + 1] - g.row_off[ww];
@@ -2330,7 +3411,7 @@ __device__ void run_task(Warp& W, const Task& t) {
             break;
           }
           bool all = true;
-          for (int j0 = 0; j0 < nLp && all; j0 += 32) {
+          ROLLED for (int j0 = 0; j0 < nLp && all; j0 += 32) {
             int j = j0 + lane;
             bool in = j >= nLp || contains_sorted(rw, dw, Lpar[j]);
             all = __all_sync(kFull, in);
@@ -2341,19 +3422,19 @@ __device__ void run_task(Warp& W, const Task& t) {
     }
   }
   if (!ism) {
-    W.nonmax += 1;
-    for (int i = lane; i < nt; i += 32) map[touched[i]] = 0;
+    acc(W.nonmax, 1);
+    ROLLED for (int i = lane; i < nt; i += 32) map[touched[i]] = 0;
     __syncwarp();
     return;
   }
   // the task's own biclique (once: parts after the first skip it)
   if (part == 0) {
     uint64_t sL = 0;
-    for (int l = lane; l < nL; l += 32) sL += g.ukey[L[l]];
-    sL = warp_sum(sL);
-    W.cnt += 1;
-    W.hash += biclique_hash(g, sL, (uint64_t)nL, sR, nR);
-    if (W.p.emit) emit_list(W.ctl, emit_dst(W.p), W.gid, nL, L, nullptr);
+    ROLLED for (int l = lane; l < nL; l += 32) sL += g.ukey[L[l]];
+    sL = warp_sum64(sL);
+    acc(W.cnt, 1);
+    acc(W.hash, biclique_hash(g, sL, (uint64_t)nL, sR, nR));
+    if (s_blk.emit) emit_list(s_blk.ctl, emit_dst(*s_blk.p), W.gid, nL, L, nullptr);
   }
   bool done = nL <= 1 || np == 0;
   // ---- split (src/IterFinderGpu.cu:835-858) ----
@@ -2362,116 +3443,59 @@ __device__ void run_task(Warp& W, const Task& t) {
   if (!done && k < 4) {
     long long rest = np;
     bool split;
-    if (W.p.vertex_split)
+    if (s_blk.p->vertex_split)
       split = (rest > W.gp->bound_height || nL > W.gp->bound_height) &&
               rest * (long long)nL > (long long)W.gp->bound_size;
     else
-      split = k == 1 && parts <= 1 && W.p.root_split > 0 &&
-              rest * (long long)nL > (long long)W.p.root_split;
+      split = k == 1 && parts <= 1 && s_blk.p->root_split > 0 &&
+              rest * (long long)nL > (long long)s_blk.p->root_split;
     if (split) {
-      if (queue_push_children(W, t, k, nq, nC)) {
-        W.splits += 1;
+      if (queue_push_children(t, k, nq, nC)) {
+        acc(W.splits, 1);
         done = true;
       }
     }
   }
   if (!done) {
-    if (nL <= W.gp->tier2_max_l && nC <= W.gp->direct_max_c) {
-      // ---- tier 2 directly: masks of every candidate over all of L ----
-      uint64_t* lkey = W.A64(W.sl.lkey);
-      uint64_t* subkey = W.A64(W.sl.sub_v);
-      int32_t* lid = W.A(W.sl.lid);
-      for (int l = lane; l < nL; l += 32) lkey[l] = g.ukey[L[l]];
-      if (W.p.emit)
-        for (int l = lane; l < nL; l += 32) lid[l] = L[l];
-      for (int i = lane; i < nC; i += 32) subkey[i] = g.vkey[cv[i]];
-      const int K = words_k(nL), RS = rec_stride(K);
-      uint32_t* rec = reinterpret_cast<uint32_t*>(W.A(W.sl.masks));
-      init_records(rec, K, nC);
-      flat_rows(
-          nL,
-          [&](int r, int& beg, int& len) {
-            int u = L[r];
-            beg = g.rev_off[u];
-            len = g.rev_off[u + 1] - beg;
-          },
-          [&](bool valid, int r, int pos) {
-            if (!valid) return;
-            int p = map[__ldg(g.rev_col + pos)] - 1;
-            if (p >= 0) atomicOr(&rec[(size_t)p * RS + 1 + (r >> 5)], 1u << (r & 31));
-          });
-      __syncwarp();
-      tier2(W, nL, nC, nq, nend, sR, nR);
+    const int K = words_k(nL);
+    const int eff = s_blk.prune ? min(nC, cntM + nL) : nC;
+    if (nL <= W.gp->tier2_max_l && nC <= W.gp->direct_max_c &&
+        cls_need(eff, K, cls_levels(nL, nC - nq)) + cls_build_words(nC, eff, K, nL) + 96LL * K <=
+            W.root_words()) {
+      // ---- tier 2 directly ----
+      uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_root));
+      uint64_t* lkey = reinterpret_cast<uint64_t*>(at);
+      int32_t* lid = reinterpret_cast<int32_t*>(at + 64 * K);
+      ROLLED for (int l = lane; l < nL; l += 32) lkey[l] = g.ukey[L[l]];
+      if (s_blk.emit)
+        ROLLED for (int l = lane; l < nL; l += 32) lid[l] = L[l];
+      uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end));
+      const ClsList cl = cls_build(
+          at + 96 * K, end, nC, nq, K, nL, &nend, ncnt, g.vkey, cv,
+          ClsEdges{W.A(W.sl().aadj), W.A(W.sl().ent), map, entries, 1});
+      cls_run(cl, first_bits(nL, lane), nend, lkey, lid, sR, nR,
+              cl.m + cls_list_words(cl.n, cl.K), end);
     } else {
       // ---- tier 1: local adjacency ----
       {
-        uint64_t* ckey = W.A64(W.sl.ckey);  // hash key per candidate, for the pushes
-        for (int i = lane; i < nC; i += 32) ckey[i] = g.vkey[cv[i]];
+        uint64_t* ckey = W.A64(W.sl().ckey);  // hash key per candidate, for the pushes
+        ROLLED for (int i = lane; i < nC; i += 32) ckey[i] = g.vkey[cv[i]];
       }
-      int32_t* llevel = W.A(W.sl.llevel);
-      int32_t* aadj = W.A(W.sl.aadj);
-      int32_t* coff = W.A(W.sl.coff);
-      int32_t* fill = W.A(W.sl.fill);
-      int32_t* cadj = W.A(W.sl.cadj);
-      int32_t* sidx = W.A(W.sl.sidx);
-      int32_t* ent = W.A(W.sl.ent);  // free until the first sparse push
-      for (int l = lane; l < nL; l += 32) llevel[l] = 0;
-      // aadj: L row -> C index (or -1 for R), rows sized by degree
-      flat_rows(
-          nL,
-          [&](int r, int& beg, int& len) {
-            int u = L[r];
-            beg = g.rev_off[u];
-            len = g.rev_off[u + 1] - beg;
-          },
-          [&](bool valid, int r, int pos) {
-            if (!valid) return;
-            int u = L[r];
-            int off = aoff[r] + (pos - g.rev_off[u]);
-            aadj[off] = map[__ldg(g.rev_col + pos)] - 1;
-            ent[off] = r;  // the entry's row, for the transpose below
-          });
-      // coff = exclusive scan of the initial counts; fill = 0; sidx = -1
-      {
-        int run = 0;
-        for (int c0 = 0; c0 < nC; c0 += 32) {
-          int i = c0 + lane;
-          int c = i < nC ? ncnt[i] : 0;
-          int tot;
-          int ex = warp_excl_scan(c, &tot);
-          if (i < nC) {
-            coff[i] = run + ex;
-            fill[i] = 0;
-            sidx[i] = -1;
-          }
-          run += tot;
-        }
-        if (lane == 0) coff[nC] = run;
+      int32_t* llevel = W.A(W.sl().llevel);
+      int32_t* aadj = W.A(W.sl().aadj);
+      int32_t* fill = W.A(W.sl().fill);
+      int32_t* sidx = W.A(W.sl().sidx);
+      ROLLED for (int l = lane; l < nL; l += 32) llevel[l] = 0;
+      // aadj: L row -> C index (or -1 for R)
+#pragma unroll 4
+      for (int e = lane; e < entries; e += 32) aadj[e] = map[aadj[e]] - 1;
+      ROLLED for (int i = lane; i < nC; i += 32) {
+        fill[i] = 0;
+        sidx[i] = -1;
       }
       __syncwarp();
-      // cadj: C index -> L positions.  A linear pass over the entries: each
-      // lane has four slot reservations in flight before it uses any.
-      {
-        const int S = aoff[nL];
-        for (int j0 = 0; j0 < S; j0 += 128) {
-          int pp[4], rr[4], ss[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int j = j0 + k * 32 + lane;
-            pp[k] = j < S ? aadj[j] : -1;
-            rr[k] = j < S ? ent[j] : 0;
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) ss[k] = pp[k] >= 0 ? atomicAdd(&fill[pp[k]], 1) : 0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (pp[k] >= 0) cadj[coff[pp[k]] + ss[k]] = rr[k];
-        }
-      }
-      __syncwarp();
-      // fill doubles as the sparse push's child-count array: back to zero.
-      for (int i = lane; i < nC; i += 32) fill[i] = 0;
-      __syncwarp();
+      // (fill doubles as the sparse push's child-count array: left all-zero)
+      t1_transpose(entries, nC);
       T1 t1;
       t1.L = L;
       t1.nL = nL;
@@ -2482,12 +3506,12 @@ __device__ void run_task(Warp& W, const Task& t) {
       t1.nRtask = nR;
       uint64_t t1s = globaltimer_ns();
       uint64_t t2_before = W.ns_t2;
-      tier1_run(W, t1);
-      W.ns_t1 += (globaltimer_ns() - t1s) - (W.ns_t2 - t2_before);
+      tier1_run(t1);
+      acc(W.ns_t1, (globaltimer_ns() - t1s) - (W.ns_t2 - t2_before));
     }
   }
   __syncwarp();
-  for (int i = lane; i < nt; i += 32) map[touched[i]] = 0;
+  ROLLED for (int i = lane; i < nt; i += 32) map[touched[i]] = 0;
   __syncwarp();
 }
 
@@ -2515,14 +3539,15 @@ __device__ __forceinline__ int graph_of_position(const long long* prefix, int n,
 // A warp that saw the head below the tail just before another moved it past
 // its graph claims nothing (that graph was exhausted), so the quiet test
 // (pending == 0, head >= tail) loses no root.
-__device__ bool serve_claim_root(Warp& W, Task* t) {
-  const ServeLink& L = W.p.serve;
+__device__ __noinline__ bool serve_claim_root(Task* t) {
+  Warp& W = this_warp();
+  const ServeLink& L = s_blk.p->serve;
   volatile ServeCtl* sc = L.sctl;
   if (sc->arr_head >= sc->arr_tail) return false;
   // A launch that is ending takes no new roots: the host relaunches for them.
-  if (*(volatile int32_t*)&W.ctl->closing) return false;
-  atomicAdd(&W.ctl->pending, 1ULL);
-  for (int tries = 0; tries < 64; ++tries) {
+  if (*(volatile int32_t*)&s_blk.ctl->closing) return false;
+  atomicAdd(&s_blk.ctl->pending, 1ULL);
+  ROLLED for (int tries = 0; tries < 64; ++tries) {
     const unsigned long long h = sc->arr_head;
     if (h >= sc->arr_tail) break;
     const uint32_t blk = *(volatile const uint32_t*)&L.arr_blk[h % (unsigned long long)L.arr_cap];
@@ -2538,15 +3563,16 @@ __device__ bool serve_claim_root(Warp& W, Task* t) {
     }
     atomicCAS((unsigned long long*)&L.sctl->arr_head, h, h + 1);
   }
-  atomicAdd(&W.ctl->pending, (unsigned long long)-1LL);
+  atomicAdd(&s_blk.ctl->pending, (unsigned long long)-1LL);
   return false;
 }
 
 // Serving: one task of graph `gid` finished (lane 0, after its results were
 // added).  The task that brings the graph's pending count to zero writes the
 // graph's completion record for the host.
-__device__ void serve_task_done(Warp& W, int32_t gid) {
-  const ServeLink& L = W.p.serve;
+__device__ __noinline__ void serve_task_done(int32_t gid) {
+  Warp& W = this_warp();
+  const ServeLink& L = s_blk.p->serve;
   ServeGraph* sg = serve_graph(W, gid);
   if (atomicAdd(&sg->pending, (unsigned long long)-1LL) != 1ULL) return;
   __threadfence();
@@ -2560,7 +3586,7 @@ __device__ void serve_task_done(Warp& W, int32_t gid) {
   d->non_maximal = nm;
   // Every task of the graph reserved its records before it finished, so the
   // reservation counter now lies past all of them.
-  d->emit_end = *(volatile unsigned long long*)&W.ctl->emit_pos;
+  d->emit_end = *(volatile unsigned long long*)&s_blk.ctl->emit_pos;
   __threadfence_system();
   d->seq = pos + 1;
 }
@@ -2579,43 +3605,60 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
   // Two tiers: the first n_big_warps warps hold the big layout, then the
   // launch's layout follows for every other warp.
   const bool big = kTiers && warp_global < p.n_big_warps;
-  Warp W{p, (kTiers && big) ? p.big_sl : sl};
-  W.ctl = ctl;
-  W.q_tasks = q_tasks;
-  W.q_seq = q_seq;
-  W.slots = pool.slots;
-  W.bigslots = pool.big;
-  W.big_bits = pool.big_bits;
-  W.nbig = pool.nbig;
-  W.import_cap = pool.import_cap;
-  W.import_l = pool.import_l;
-  W.import_s = pool.import_s;
-  W.slot_bits = pool.bits;
-  W.nslot = pool.nslot;
-  if (!kTiers)
-    W.base = scratch + (size_t)warp_global * (size_t)sl.words_per_warp;
-  else
-    W.base = big ? scratch + (size_t)warp_global * (size_t)p.big_sl.words_per_warp
-                 : scratch + (size_t)p.n_big_warps * (size_t)p.big_sl.words_per_warp +
-                       (size_t)(warp_global - p.n_big_warps) * (size_t)sl.words_per_warp;
-  extern __shared__ uint32_t enum_smem[];
-  W.seen = sl.seen_words && p.touch_scan <= 0
-               ? enum_smem + (size_t)(threadIdx.x >> 5) * sl.seen_words
-               : nullptr;
-  W.gseen = reinterpret_cast<uint32_t*>(W.base + W.sl.gseen);
-  if (W.seen) {
-    for (int i = lane; i < sl.seen_words; i += 32) W.seen[i] = 0u;
-    __syncwarp();
+  Warp& W = this_warp();
+  if (threadIdx.x == 0) {
+    s_blk.p = &p;
+    s_blk.ctl = ctl;
+    s_blk.q_tasks = q_tasks;
+    s_blk.q_seq = q_seq;
+    s_blk.graphs = graphs;
+    s_blk.slots = pool.slots;
+    s_blk.slot_bits = pool.bits;
+    s_blk.bigslots = pool.big;
+    s_blk.big_bits = pool.big_bits;
+    s_blk.emit = p.emit;
+    s_blk.deadline = p.time_limit_ns > 0 ? t_start + (uint64_t)p.time_limit_ns : 0;
+    s_blk.import_words = pool.import_words;
+    s_blk.nslot = pool.nslot;
+    s_blk.nbig = pool.nbig;
+    s_blk.import_cap = pool.import_cap;
+    s_blk.import_l = pool.import_l;
+    s_blk.import_s = pool.import_s;
+    s_blk.prune = p.prune;
+    s_blk.server = p.server;
+    s_blk.share_min_work = p.share_min_work;
+    s_blk.slot_records = p.slot_records;
+    s_blk.eager_share = p.eager_share;
+    s_blk.share_counts = p.share_counts;
+    s_blk.touch_scan = p.touch_scan;
+    s_blk.smem_words = sl.smem_words;
+    s_blk.lookout = 0;
+    s_sl[0] = sl;
+    if (kTiers) s_sl[1] = p.big_sl;
   }
-  W.graphs = graphs;
-  W.gp = graphs;
-  W.gid = 0;
-  W.cnt = W.hash = W.nonmax = W.splits = 0;
-  W.ns_t1 = W.ns_t2 = W.n_t2 = 0;
-  W.pushes = W.shape = 0;
-  W.deadline = p.time_limit_ns > 0 ? t_start + (uint64_t)p.time_limit_ns : 0;
-  W.dem = 0;
-  W.dem_t = -(1LL << 62);
+  // Shared memory of a warp: the first-touch bitmap of counting passes and the
+  // bitmap tier take turns in it (clear_seen).
+  uint32_t* smem =
+      reinterpret_cast<uint32_t*>(enum_smem4) + (size_t)(threadIdx.x >> 5) * sl.smem_words;
+  ROLLED for (int i = lane; i < sl.smem_words; i += 32) smem[i] = 0u;
+  if (lane == 0) {
+    if (!kTiers)
+      W.base = scratch + (size_t)warp_global * (size_t)sl.words_per_warp;
+    else
+      W.base = big ? scratch + (size_t)warp_global * (size_t)p.big_sl.words_per_warp
+                   : scratch + (size_t)p.n_big_warps * (size_t)p.big_sl.words_per_warp +
+                         (size_t)(warp_global - p.n_big_warps) * (size_t)sl.words_per_warp;
+    W.tier = big ? 1 : 0;
+    W.seen = sl.seen_words && p.touch_scan <= 0 ? smem : nullptr;
+    W.gp = graphs;
+    W.gid = 0;
+    W.cnt = W.hash = W.nonmax = W.splits = 0;
+    W.ns_t1 = W.ns_t2 = W.n_t2 = 0;
+    W.pushes = W.shape = 0;
+    W.dem = 0;
+    W.dem_t = -(1LL << 62);
+  }
+  __syncthreads();
   uint64_t ns_idle = 0, n_tasks = 0, max_task = 0, max_info = 0, max_split = 0;
   uint64_t max_pushes = 0, max_shape = 0;
   int32_t max_gid = 0;
@@ -2625,17 +3668,17 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
   while (true) {
     int ab = 0;
     if (lane == 0 && p.server) ab = *(volatile int32_t*)&p.serve.sctl->stop;  // shutting down
-    if (__shfl_sync(kFull, ab, 0) || must_stop(W)) break;
+    if (__shfl_sync(kFull, ab, 0) || must_stop()) break;
     Task t;
     int have = 0;
     if (lane == 0) {
-      have = queue_pop(W, &t) ? 1 : 0;
+      have = queue_pop(&t) ? 1 : 0;
       if (!have && p.server) {
-        have = serve_claim_root(W, &t) ? 1 : 0;
+        have = serve_claim_root(&t) ? 1 : 0;
       } else if (!have) {
         // A big warp first takes parts of big roots, then the roots no other
         // warp has room for.
-        if (kTiers && big && p.big_parts_cap > 0) have = big_parts_claim(W, &t) ? 1 : 0;
+        if (kTiers && big && p.big_parts_cap > 0) have = big_parts_claim(&t) ? 1 : 0;
         if (!have && kTiers && big &&
             *(volatile long long*)&ctl->next_big < (long long)p.n_big_roots) {
           atomicAdd(&ctl->pending, 1ULL);
@@ -2689,11 +3732,11 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
       if (t.v[0] >= 0) {
         W.gid = t.graph;
         W.gp = graph_at(W, t.graph);
-        run_task(W, t);
+        run_task(t);
       } else if (t.v[1] == 1) {
-        tier1_from_slot(W, -2 - t.v[0]);  // an exported counts-tier child (sets the graph)
+        tier1_from_slot(-2 - t.v[0]);  // an exported counts-tier child (sets the graph)
       } else {
-        tier2_from_slot(W, -2 - t.v[0]);  // an exported bitmap sub-problem (sets the graph)
+        tier2_from_slot(-2 - t.v[0]);  // an exported bitmap sub-problem (sets the graph)
       }
       __syncwarp();
       // Results go to the task's graph.
@@ -2702,8 +3745,8 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
         if (W.cnt) atomicAdd(&r[0], W.cnt);
         if (W.hash) atomicAdd(&r[1], W.hash);
         if (W.nonmax) atomicAdd(&r[2], W.nonmax);
+        W.cnt = W.hash = W.nonmax = 0;
       }
-      W.cnt = W.hash = W.nonmax = 0;
       uint64_t te = globaltimer_ns();
       busy_ns += te - tb;
       last_done_ns = te - t_start;
@@ -2719,7 +3762,7 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
       }
       if (lane == 0) {
         __threadfence();
-        if (p.server) serve_task_done(W, W.gid);
+        if (p.server) serve_task_done(W.gid);
         atomicAdd(&ctl->pending, (unsigned long long)-1LL);
       }
       idle_since = 0;
@@ -2769,7 +3812,29 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
       if (lane == 0) set_status(ctl, kStTimeout, now - idle_since);
       break;
     }
-    __nanosleep(256);
+    // Until something may have changed.  One idle warp of the block looks at
+    // the queue, the others at the block's own flag in shared memory until they
+    // take the lookout over: thousands of warps reading the launch's counters
+    // kept one L2 slice busy and held up everyone's memory traffic (a half-size
+    // grid was a third faster).
+    if (lane == 0) {
+      bool look = false;
+      ROLLED for (int r = 0; r < 16; ++r) {
+        if (!look) look = atomicCAS(&s_blk.lookout, 0, 1) == 0;
+        if (look) {
+          const unsigned long long h = *(volatile unsigned long long*)&ctl->q_head;
+          const unsigned long long q = *(volatile unsigned long long*)&ctl->q_tail;
+          if (h < q || *(volatile unsigned long long*)&ctl->pending == 0ULL) break;
+          if (p.server) {
+            volatile ServeCtl* sc = p.serve.sctl;
+            if (sc->arr_head < sc->arr_tail) break;
+          }
+        }
+        __nanosleep(look ? 200 : 400);
+      }
+      if (look) atomicExch(&s_blk.lookout, 0);
+    }
+    __syncwarp();
   }
   __syncwarp();
   if (lane == 0) {

@@ -18,6 +18,8 @@ constexpr int kEnumThreads = kEnumWarps * 32;  // threads per block
 // Blocks per SM the register allocation is made for (launch bounds).
 constexpr int kEnumMinBlocks = GMBE_ENUM_MIN_BLOCKS;
 constexpr int kKMax = 4;                       // bitmap words of the tier-2 sub-problem
+constexpr int kChildMax = 128;                 // largest child that is merged on the way to its list
+constexpr int kSmemWords = 2488;               // shared memory words of a warp
 constexpr int kLevelBits = 8;                  // counts-tier levels with a candidate bitmap
 
 // One persistent launch over p.n_graphs graphs: graphs[i] describes graph i,
@@ -45,7 +47,7 @@ constexpr int32_t kSlotMaxRecords = 8064;
 constexpr int kSeenMaxWords = 3584;
 // Dynamic shared memory of a launch with layout sl.
 inline size_t enum_smem_bytes(const ScratchLayout& sl) {
-  return (size_t)sl.seen_words * sizeof(uint32_t) * kEnumWarps;
+  return (size_t)sl.smem_words * sizeof(uint32_t) * kEnumWarps;
 }
 // |P|*|L| from which a child is shared out while many warps wait for work.
 constexpr int32_t kShareMinWorkDefault = 256;

@@ -126,7 +126,9 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
   if (capC >= (1 << 24))
     return set_error(MBE_ERR_CAPACITY, "graph too large for the no-allocation pool");
   ScratchLayout sl = make_layout(nV, capC, capL, capS);
-  sl.seen_words = 0;  // first touches by global atomics: this launch uses no dynamic shared memory
+  // First touches by global atomics; shared memory for the bitmap tier only.
+  sl.seen_words = 0;
+  sl.smem_words = kSmemWords;
 
   // Pool partition: control block, split ring, per-block timing, hash keys,
   // then as many 16-warp blocks of per-warp scratch as fit.
@@ -158,10 +160,9 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
                      "holds %zu bytes in total (use mbe_enumerate for graphs this large)",
                      per_block, kEnumWarps, kNoAllocPoolBytes);
   int sms = 0, occ = 0;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mbe_enum_kernel, kEnumThreads, 0)) !=
-          cudaSuccess)
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return set_error(MBE_ERR_CUDA, "device query: %s", cudaGetErrorString(e));
+  if (int rc0 = enum_blocks_per_sm(false, enum_smem_bytes(sl), &occ)) return rc0;
   int blocks = std::min(fit_blocks, std::max(1, sms * occ));
   if (prm.blocks > 0) blocks = std::min(blocks, prm.blocks);
   const int warps = blocks * kEnumWarps;
@@ -226,7 +227,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
   none.nslot = 0;  // no sub-problem export out of the static pool
   ep.vertex_split = 1;
   noalloc_init<<<1, 32, 0, st>>>(dg, d_graph, d_prefix, d_gres);
-  mbe_enum_kernel<<<blocks, kEnumThreads, 0, st>>>(d_graph, d_prefix, d_gres, ep, sl, ctl, q_tasks,
+  mbe_enum_kernel<<<blocks, kEnumThreads, enum_smem_bytes(sl), st>>>(d_graph, d_prefix, d_gres, ep, sl, ctl, q_tasks,
                                                    q_seq, none, scratch, exit_ns);
   noalloc_finish<<<1, 32, 0, st>>>(ctl, d_gres, d_out);
   if ((e = cudaGetLastError()) != cudaSuccess)

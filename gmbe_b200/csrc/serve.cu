@@ -272,6 +272,7 @@ int launch(mbe_server* s) {
   pool.slots = s->d_slots;
   pool.bits = s->d_slot_bits;
   pool.nslot = s->nslot;
+  pool.import_words = s->sl.ar_end - s->sl.ar_root;
   mbe_enum_kernel<<<s->blocks, kEnumThreads, enum_smem_bytes(s->sl), s->s_run>>>(
       reinterpret_cast<const DevGraph*>(s->d_arena), nullptr, nullptr, s->ep, s->sl, s->d_ctl,
       s->d_q_tasks, s->d_q_seq, pool, s->d_scratch, nullptr);
