@@ -2417,6 +2417,135 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
   return true;
 }
 
+// A push at `level` that keeps one or two rows (la; lb, or -1), whole: what
+// t1_sparse_push would do, without counts, an entry list or a sub-problem.
+// With pruning on, the child of two rows has candidates on one row each; its
+// pushes keep that row alone, one push per row that has a P candidate (the
+// others of the row are retired with it), non-maximal exactly if the row has a
+// Q candidate.  So the rows are walked and summed up: row a's candidates are
+// marked in cc, row b's walk tells the common ones (R of the push) from its
+// own, row a's second walk sees the rest.  Each walk keeps kNarrow rounds of
+// loads in flight, for a push is a chain of them and one warp's pushes are a
+// root's critical path.
+//
+// On the 300,000-edge graph three fifths of a heavy root's first-level pushes
+// keep one or two rows (3,042 of 5,028).  Whole calls, before -> after: that
+// graph 50.2 -> 48.5 ms, one shard of the large graph (rows of 10^5 entries)
+// 915 -> 839 ms.
+constexpr int kNarrow = 4;
+__device__ __noinline__ void t1_narrow_push(const T1 t, int x, int level, int la, int lb,
+                                            uint64_t sL) {
+  Warp& W = this_warp();
+  const int lane = (int)lane_id();
+  int32_t* llevel = W.A(W.sl().llevel);
+  const int32_t* ncnt = W.A(W.sl().ncnt);
+  int32_t* bound = W.A(W.sl().bound);
+  const int32_t* aoff = W.A(W.sl().aoff);
+  const int32_t* aadj = W.A(W.sl().aadj);
+  const uint64_t* ckey = W.A64(W.sl().ckey);
+  int32_t* cc = W.A(W.sl().fill);  // all-zero between pushes
+  const bool two = lb >= 0;
+  if (two) {
+    const int end = aoff[la + 1];
+#pragma unroll 4
+    for (int j = aoff[la] + lane; j < end; j += 32) {
+      const int p = aadj[j];
+      if (p >= 0) cc[p] = 1;
+    }
+    __syncwarp();
+  }
+  bool ism = true;
+  uint64_t sR = 0;       // R of the push
+  unsigned nR = 0;
+  uint64_t key[2];       // R of the child's push that keeps row b (0), row a (1)
+  unsigned np[2], nq[2];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    key[s] = 0;
+    np[s] = nq[s] = 0;
+    if (s == 0 && !two) continue;
+    const int row = s == 0 ? lb : la;
+    const int end = aoff[row + 1];
+    ROLLED for (int j0 = aoff[row] + lane; j0 < end; j0 += 32 * kNarrow) {
+      int p[kNarrow], b[kNarrow], nc[kNarrow], m[kNarrow];
+      uint64_t k[kNarrow];
+#pragma unroll
+      for (int u = 0; u < kNarrow; ++u) p[u] = j0 + 32 * u < end ? aadj[j0 + 32 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < kNarrow; ++u) {
+        if (p[u] < 0) continue;
+        b[u] = bound[p[u]];
+        nc[u] = ncnt[p[u]];
+        k[u] = ckey[p[u]];
+        m[u] = two ? cc[p[u]] : 1;  // row b: 1 in row a too; row a: 2 in row b too
+      }
+#pragma unroll
+      for (int u = 0; u < kNarrow; ++u) {
+        if (p[u] < 0) continue;
+        const bool live = b[u] >= level;
+        if (two) {
+          if (s == 0 && m[u]) cc[p[u]] = 2;
+          if (s == 1) cc[p[u]] = 0;
+          if (s == 1 && m[u] == 2) continue;  // common: done with row b
+        }
+        const bool covers = !two || (s == 0 && m[u]);
+        if (covers) {
+          sR += k[u];
+          ++nR;
+          ism = ism && !(live && p[u] < x);
+        } else if (live) {
+          if (p[u] < x) {
+            ++nq[s];
+          } else {
+            key[s] += k[u];
+            ++np[s];
+          }
+        }
+        // finder_pop: retired if it meets no removed row
+        if (live && p[u] != x && nc[u] == (covers && two ? 2 : 1)) bound[p[u]] = level - 1;
+      }
+    }
+    __syncwarp();
+  }
+  ism = __all_sync(kFull, ism);
+  if (ism) {
+    sR = warp_sum64(sR) + t.sRtask;
+    const uint64_t nRs = __reduce_add_sync(kFull, nR) + t.nRtask;
+    acc(W.cnt, 1);
+    acc(W.hash, biclique_hash(*W.gp, sL, two ? 2 : 1, sR, nRs));
+    int32_t* lp = W.A(W.sl().lp);
+    if (s_blk.emit) {
+      if (lane <= (int)two) lp[lane] = lane < (int)two ? lb : la;
+      __syncwarp();
+      emit_list(s_blk.ctl, emit_dst(*s_blk.p), W.gid, two ? 2 : 1, t.L, lp);
+    }
+    if (two) {
+      const uint64_t ka = W.gp->ukey[t.L[la]];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const unsigned n = __reduce_add_sync(kFull, np[s]);
+        if (n == 0) continue;
+        acc(W.pushes, 1ULL << 32);
+        if (__any_sync(kFull, nq[s] != 0)) {
+          acc(W.nonmax, 1);
+          continue;
+        }
+        const uint64_t ks = warp_sum64(key[s]);
+        acc(W.cnt, 1);
+        acc(W.hash, biclique_hash(*W.gp, s == 0 ? sL - ka : ka, 1, sR + ks, nRs + n));
+        if (s_blk.emit) emit_list(s_blk.ctl, emit_dst(*s_blk.p), W.gid, 1, t.L, lp + s);
+      }
+    }
+  } else {
+    acc(W.nonmax, 1);
+  }
+  if (lane == 0) {
+    llevel[la] = level - 1;
+    if (two) llevel[lb] = level - 1;
+  }
+  __syncwarp();
+}
+
 // Levels 2 .. kLevelBits + 1 of the counts tier keep a bitmap of the
 // candidates the level's L meets (count != 0 there): the scan for the next
 // live candidate and a recount walk its words instead of every candidate.
@@ -2616,6 +2745,7 @@ __device__ __noinline__ void tier1_run(const T1 t) {
       uint64_t sL = 0;
       long long kent = 0;                 // entries of the kept rows
       unsigned long long best = ~0ULL;    // (row length << 32) | position of the shortest kept row
+      int first = INT_MAX, last = -1;     // the first and the last kept row
       int rb = coff[cur], re = coff[cur + 1];
       ROLLED for (int j = rb + lane; j < re; j += 32) {
         int l = cadj[j];
@@ -2626,10 +2756,21 @@ __device__ __noinline__ void tier1_run(const T1 t) {
           const int len = aoff[l + 1] - aoff[l];
           kent += len;
           best = min(best, ((unsigned long long)(unsigned)len << 32) | (unsigned)l);
+          last = max(last, l);
+          first = min(first, l);
         }
       }
       kept = (int)__reduce_add_sync(kFull, (unsigned)kept);
       sL = warp_sum64(sL);
+      if (s_blk.prune && kept <= min(t2max, 2)) {
+        __syncwarp();
+        first = __reduce_min_sync(kFull, first);
+        last = __reduce_max_sync(kFull, last);
+        t1_narrow_push(t, cur, level, first, kept == 2 ? last : -1, sL);
+        if (lane == 0) stack[level - 1] = cur + 1;
+        __syncwarp();
+        continue;
+      }
       kent = warp_sum64(kent);
       best = warp_min_u64(best);
       __syncwarp();
