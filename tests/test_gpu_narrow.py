@@ -50,3 +50,35 @@ def test_narrow_pushes_match_oracle(nL, lens, extra):
                     assert r.non_maximal == plain, (order, params)
             r, found = G.enumerate_emit(1 << 20)
             assert len(found) == want.count and r.set_hash == want.set_hash
+
+
+@pytest.mark.parametrize("nL,singles,extra", [
+    (40, 100, 3),      # fewer entries than a compaction starts from
+    (40, 170, 12),     # about that many
+    (40, 1000, 60),    # several compactions in one task
+    (200, 5000, 300),
+])
+def test_retired_entries_dropped_match_oracle(nL, singles, extra):
+    """Most candidates on two hub rows and on nothing else: the first push that
+    keeps such a row retires them, and the rows are compacted under the pushes
+    that follow (counts tier, also for short L: bitmap_max_l)."""
+    import gmbe_b200 as gm
+    rng = np.random.default_rng(nL + singles)
+    adj = [np.arange(nL, dtype=np.int32)]
+    adj += [np.array([i % 7 == 0], np.int32) for i in range(singles)]
+    for _ in range(extra):
+        rest = 2 + rng.choice(nL - 2, size=int(rng.integers(1, 12)), replace=False)
+        hubs = np.nonzero(rng.random(2) < 0.7)[0]
+        adj.append(np.sort(np.concatenate([hubs, rest])).astype(np.int32))
+    ro = np.zeros(len(adj) + 1, np.int32)
+    ro[1:] = np.cumsum([len(r) for r in adj])
+    g = (ro, np.concatenate(adj).astype(np.int32), nL)
+    for order in (0, 1):
+        want = oracle.gmbe(*g, uvtrans=0, order=order)
+        with gm.Graph.from_csr(*g, uvtrans=0, order=order) as G:
+            for params in (dict(), dict(bitmap_max_l=1), dict(bitmap_max_l=16),
+                           dict(bitmap_max_l=16, share_min_work=1), dict(direct_max_c=1),
+                           dict(direct_max_c=1, range_split_work=100, range_chunk=8),
+                           dict(bitmap_max_l=4, touch_scan=1)):
+                r = G.enumerate(wait_limit_ns=30 * 10**9, **params)
+                assert (r.count, r.set_hash) == (want.count, want.set_hash), (order, params)
