@@ -2929,7 +2929,10 @@ __device__ __noinline__ void tier1_run(const T1 t) {
       }
       __syncwarp();
       if (ism && kept > 1) {
-        if (kept > t2max || !t1_handoff(t, cur, level, kept, sR, nR)) {
+        // (Pruning on, a child the sparse push declined is not handed over
+        // either: the hand-off keeps no counts of its candidates, by which the
+        // class list is built then, and leaves its indices in sidx.)
+        if (kept > t2max || s_blk.prune || !t1_handoff(t, cur, level, kept, sR, nR)) {
           uint32_t* nbits = level_bits(W, level + 1);
           // The candidates the kept rows meet, as a bitmap: the next level's
           // own one, or (deeper levels) the warp's global touch bitmap, built
