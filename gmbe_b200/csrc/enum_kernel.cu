@@ -958,14 +958,33 @@ __device__ __noinline__ bool leaf_export(uint32_t m, uint64_t key, uint32_t cnt,
   return false;
 }
 
-// What a walk adds to its warp's totals, in registers.
+// What a walk adds to its warp's totals, in registers.  The two counts go to
+// the 64-bit totals at every look at the stop flag: a step adds one to one of
+// them at most and some loop of the walk looks whenever `steps` passes a
+// multiple of kLookSteps, so that they stay at or below it, however many
+// bicliques the sub-problem has.
+constexpr uint32_t kLookSteps = 4096;
 struct Tally {
   unsigned long long hl;  // this lane's part of the hash sum
-  uint32_t cnt, nonmax;   // bicliques found, pushes rejected
+  uint32_t cnt, nonmax;   // bicliques found, pushes rejected, since the last look
   uint32_t steps;
   int swapped;
   int share_floor;        // |P|*|L| from which a child may be shared out
 };
+__device__ __forceinline__ void tally_fold(Tally& y) {
+  Warp& W = this_warp();
+  acc(W.cnt, y.cnt);
+  acc(W.nonmax, y.nonmax);
+  acc(W.pushes, (unsigned long long)(y.cnt + y.nonmax) << 32);
+  y.cnt = y.nonmax = 0u;
+}
+// Counts a step; whether the walk should stop.  `every`: steps between looks, a
+// divisor of kLookSteps.
+__device__ __forceinline__ bool tally_step(Tally& y, uint32_t every) {
+  if ((++y.steps & (every - 1u)) != 0u) return false;
+  tally_fold(y);
+  return must_stop();
+}
 
 // Walks a leaf sub-problem (lid: the internal U id of each L bit, for
 // emission); false if the launch is stopping.
@@ -993,7 +1012,7 @@ __device__ __forceinline__ bool leaf_run(Tally& y, const Leaf& f, const int32_t*
       if (depth == 0) lim = f.lim;
       continue;
     }
-    if ((++y.steps & 4095u) == 0u && must_stop()) return false;
+    if (tally_step(y, kLookSteps)) return false;
     // ---- push (finder_push) of class c, and what its pop leaves ----
     const int c = __ffs(t) - 1;
     const uint32_t cb = t & (0u - t);
@@ -1634,7 +1653,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
       if (!cls_leave(c, L, curw)) break;
       continue;
     }
-    if ((++y.steps & 1023u) == 0u && must_stop()) break;
+    if (tally_step(y, 1024u)) break;
     curw = cpos >> 5;
     const int K = c.l.K;
     const uint32_t mc = lane < K ? c.l.m[(size_t)lane * c.l.stride + cpos] : 0u;
@@ -1748,11 +1767,9 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     }
   }
   hash += warp_sum64(y.hl);
+  tally_fold(y);
   Warp& W = this_warp();
   acc(W.hash, hash);
-  acc(W.cnt, y.cnt);
-  acc(W.nonmax, y.nonmax);
-  acc(W.pushes, (unsigned long long)(y.cnt + y.nonmax) << 32);
   acc(W.ns_t2, globaltimer_ns() - t0);
   acc(W.n_t2, 1);
   __syncwarp();
