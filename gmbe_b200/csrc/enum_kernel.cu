@@ -2650,16 +2650,17 @@ __device__ __forceinline__ int t1_next_live(const int32_t* bound, const int32_t*
 // |Q'|, graph, sR (2 words), |R|}, then L' ids, then C' ids.
 constexpr int kFrameHdr = 16;
 
-// Whether a counts-tier child of `kept` rows (`kent` entries) may be shared
-// out now: slots exist, every warp has room for it, warps wait for work.
+// Whether a counts-tier child of `kept` rows (`kent` entries left in them) may
+// be shared out now: slots exist, every warp has room for that much, warps wait
+// for work.
 __device__ __forceinline__ bool t1_export_wanted(Warp& W, int kept, long long kent) {
   if (!s_blk.share_counts || (s_blk.nslot == 0 && s_blk.nbig == 0)) return false;
   if (kept > s_blk.import_l || kent > (long long)s_blk.import_s) return false;
   return export_demand() != 0;
 }
 
-__device__ __noinline__ bool t1_try_export(const T1 t, int x, int level, int kept, long long kent,
-                                           uint64_t sR, uint64_t nR, const uint32_t* nbits) {
+__device__ __noinline__ bool t1_try_export(const T1 t, int x, int level, int kept, uint64_t sR,
+                                           uint64_t nR, const uint32_t* nbits) {
   Warp& W = this_warp();
   const int lane = (int)lane_id();
   const int32_t* bound = W.A(W.sl().bound);
@@ -2685,6 +2686,17 @@ __device__ __noinline__ bool t1_try_export(const T1 t, int x, int level, int kep
   m = (int)__reduce_add_sync(kFull, (unsigned)m);
   mq = (int)__reduce_add_sync(kFull, (unsigned)mq);
   if (m == 0 || m > s_blk.import_cap || !should_export(W, m - mq, kept)) return false;
+  if (s_blk.import_s < W.sl().capS) {
+    // The importer lays the graph's whole rows out; those here may have lost
+    // entries since (t1_compact).
+    const int32_t* rev_off = W.gp->rev_off;
+    long long whole = 0;
+    ROLLED for (int j = coff[x] + lane; j < coff[x + 1]; j += 32) {
+      const int l = cadj[j];
+      if (llevel[l] == level) whole += rev_off[t.L[l] + 1] - rev_off[t.L[l]];
+    }
+    if (warp_sum64(whole) > (unsigned long long)s_blk.import_s) return false;
+  }
   const long long words = kFrameHdr + (long long)kept + m;
   int slot = -1;
   if (lane == 0) {
@@ -2963,7 +2975,7 @@ __device__ __noinline__ void tier1_run(const T1 t) {
             __syncwarp();
           }
           const bool exported =
-              want && cbits && t1_try_export(t, cur, level, kept, kent, sR, nR, cbits);
+              want && cbits && t1_try_export(t, cur, level, kept, sR, nR, cbits);
           if (cbits && (exported || cbits != nbits)) {
             // back to clear: a shared-out child's level bitmap, or the touch bitmap
             t1_walk(t.nL, cur, level, kOpClearBit, level, cbits);
