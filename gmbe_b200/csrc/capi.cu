@@ -172,7 +172,7 @@ ScratchLayout make_layout(int32_t nV, int32_t capC, int32_t capL, int32_t capS) 
   s.ckey = take(2 * C);
   s.tlist = take(C);
   s.ar_sub = off;
-  take(13 * C + 9696);
+  take(cls_sub_words(C));
   s.ar_end = off;
   s.words_per_warp = off;
   const int64_t seen = ((int64_t)nV + 31) / 32;

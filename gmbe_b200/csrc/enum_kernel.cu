@@ -164,10 +164,6 @@ struct Warp {
   }
   // This warp's first-touch bitmap in global memory.
   __device__ __forceinline__ uint32_t* gseen() const;
-  // Arena words of a sub-problem that starts at a root or a slot, or below a
-  // counts-tier push.
-  __device__ __forceinline__ long long root_words() const;
-  __device__ __forceinline__ long long sub_words() const;
 };
 
 __shared__ Block s_blk;
@@ -184,8 +180,6 @@ __device__ __forceinline__ const ScratchLayout& Warp::sl() const { return s_sl[t
 __device__ __forceinline__ uint32_t* Warp::gseen() const {
   return reinterpret_cast<uint32_t*>(base + sl().gseen);
 }
-__device__ __forceinline__ long long Warp::root_words() const { return sl().ar_end - sl().ar_root; }
-__device__ __forceinline__ long long Warp::sub_words() const { return sl().ar_end - sl().ar_sub; }
 // Adds to one of the warp's accumulators (v: the same in every lane).
 __device__ __forceinline__ void acc(unsigned long long& a, unsigned long long v) {
   if (lane_id() == 0) a += v;
@@ -455,12 +449,6 @@ struct ClsList {
   int n, stride, K;
 };
 
-__host__ __device__ __forceinline__ long long cls_stride(long long n) { return (n + 31) & ~31LL; }
-// Words of a list of n classes with K-word masks (a multiple of 32).
-__host__ __device__ __forceinline__ long long cls_list_words(long long n, int K) {
-  return cls_stride(n) * (K + 3);
-}
-
 __device__ __forceinline__ ClsList cls_list_at(uint32_t* base, int n, int K) {
   ClsList l;
   l.n = n;
@@ -472,38 +460,32 @@ __device__ __forceinline__ ClsList cls_list_at(uint32_t* base, int n, int K) {
   return l;
 }
 
-// One level of the walk while a deeper one runs, in the warp's arena: the
-// list it works on and where its live, Q and P bits (a bit per class) are; its
-// L words follow.
+// One level of the walk while a deeper one runs, in the warp's arena: the list
+// it works on, its live bits (a bit per class), and the class it pushed last;
+// its L words follow.  The list's own Q and P bits serve every level on it:
+// classes are pushed in order, so that at each level, of the live ones, those
+// up to the last pushed one are Q and the rest are what they were when the list
+// was made (q_bits, p_bits).  So a level costs one bit a class, and the scratch
+// holds a level per L vertex of the widest child (cls_sub_words).  With Q and P
+// bits at every level it held half of them, and wider children went down the
+// counts tier instead: 900 candidates below a row of 140 vertices, 800 of them
+// below one of 128, 17 ms on one B200 against 63 with the other warps' help and
+// 156 without.
 struct ClsFrame {
   ClsList l;
   const uint64_t* lk;  // hash key of each L bit
   const int32_t* lid;  // internal U id of each L bit (emission only)
   uint64_t sR;         // R of the push that opened the level
   ClsFrame* prev;
-  uint32_t* A;         // live, Q and P bits
+  uint32_t* A;         // live bits
+  const uint32_t* QP;  // the list's Q bits, then its P bits
   uint32_t *top, *stop;  // first free word above the level: arena, shared memory
   uint32_t nR;
   int nend;            // classes [0, nend) may be pushed here
-  int curw;            // word the scan for the next candidate stands at
+  int last;            // the last pushed class (-1: none; a level on its parent's
+                       // list starts from the parent's)
 };
-constexpr int kFrameWords = (int)((sizeof(ClsFrame) / 4 + 3) & ~3u);
-__host__ __device__ __forceinline__ long long cls_frame_words(long long n, int K) {
-  return kFrameWords + 3 * ((((n + 31) >> 5) + 1) & ~1LL) + ((K + 1) & ~1);
-}
-// Most levels of a sub-problem: a level's L and its classes to push are both
-// fewer than those of the level above.
-__host__ __device__ __forceinline__ int cls_levels(int kn, int np) {
-  return kn < np + 1 ? kn : np + 1;
-}
-// Words a sub-problem of n classes, K words and so many levels may need: its
-// list, two words of bits per 32 classes that a push makes, a frame per level
-// (a level that finds no room for a list of its own works on the one above it
-// with bits of its own), and room for the keys of a leaf's L bits.
-__host__ __device__ __forceinline__ long long cls_need(long long n, int K, int levels) {
-  return cls_list_words(n, K) + 4 * ((n + 63) >> 6) + (long long)levels * cls_frame_words(n, K) +
-         512;
-}
+static_assert(sizeof(ClsFrame) <= 4 * kFrameWords, "frame size");
 
 __device__ __forceinline__ int words_k(int n) {
   int w = (n + 31) >> 5;
@@ -565,7 +547,7 @@ __device__ int slot_alloc_for(Warp& W, int n, int K) {
 // Whether a child of n classes and so many levels can be exported at all:
 // some kind of slot holds it, and every warp of the launch can run it.
 __device__ __forceinline__ bool slot_fits(const Warp& W, int n, int K, int levels) {
-  if (s_blk.nslot == 0 || cls_need(n, K, levels) + 96LL * K > s_blk.import_words) return false;
+  if (s_blk.nslot == 0 || cls_need(n, K, levels) + cls_key_words(K) > s_blk.import_words) return false;
   return regular_fits(W, n, K) || (s_blk.nbig > 0 && n <= big_slot_cap(K));
 }
 
@@ -1072,19 +1054,29 @@ struct ClsCur {             // the level being walked, in shared memory
   ClsList l;
   const uint64_t* lk;
   const int32_t* lid;
-  uint32_t* A;              // live bits; Q and P bits follow, nwp words each
+  uint32_t* A;              // live bits
+  const uint32_t* QP;       // the list's Q bits, then its P bits (nwp words each)
   uint32_t *S, *C;          // bits of the child being made, and of the covering classes
   ClsFrame* fr;
   uint32_t *top, *stop;     // first free word of the arena, and of the shared one
   const int32_t* leaf_lid;  // of the leaf being walked (emission)
   uint64_t sR;
   uint32_t nR;
-  int nw, nwp;              // words of A, Q, P
+  int nw, nwp;              // words of the bit strings (nwp: the even number from nw)
   int nend;
 };
 static_assert(sizeof(ClsCur) <= 40 * 4, "shared memory layout");
 __device__ __forceinline__ ClsCur& this_cur() {
   return *reinterpret_cast<ClsCur*>(this_smem() + kSmCur);
+}
+
+// Word w of a level's Q and P bits, the live classes' at least, while class `at`
+// is being pushed.
+__device__ __forceinline__ uint32_t q_bits(const ClsCur& c, int at, int w) {
+  return c.QP[w] | (c.QP[c.nwp + w] & first_bits(at, w));
+}
+__device__ __forceinline__ uint32_t p_bits(const ClsCur& c, int at, int w) {
+  return c.QP[c.nwp + w] & ~first_bits(at + 1, w);
 }
 
 // Visits four words of classes at a time, those whose bit is set in `live`
@@ -1122,12 +1114,12 @@ struct SweepOut {
 
 // One push's sweep over the level's live classes.  lnw and rmw (lane w: word
 // w) are the new L and the L vertices it leaves; cpos is the pushed class,
-// which stays live, and is in Q and no longer in P from here on.  Bits C: the
-// classes covering the new L; bits S: the child's.
+// which stays live.  Bits C: the classes covering the new L; bits S: the
+// child's.
 __device__ __forceinline__ SweepOut cls_sweep(const ClsCur& c, uint32_t lnw, uint32_t rmw,
                                               int cpos) {
   const int lane = (int)lane_id();
-  const int K = c.l.K, st = c.l.stride, nw = c.nw, nwp = c.nwp;
+  const int K = c.l.K, st = c.l.stride, nw = c.nw;
   const uint32_t* m = c.l.m;
   uint32_t* A = c.A;
   const bool prune = s_blk.prune != 0;
@@ -1136,8 +1128,8 @@ __device__ __forceinline__ SweepOut cls_sweep(const ClsCur& c, uint32_t lnw, uin
     const int wl = sb + lane;
     const bool in = wl < nw;
     const uint32_t aw = in ? A[wl] : 0u;
-    uint32_t qw = in ? A[nwp + wl] : 0u;
-    uint32_t pw = in ? A[2 * nwp + wl] : 0u;
+    const uint32_t qw = in ? q_bits(c, cpos, wl) : 0u;
+    const uint32_t pw = in ? p_bits(c, cpos, wl) : 0u;
     uint32_t sel = 0u, out = 0u, cv = 0u;
     uint32_t miss[4] = {0u, 0u, 0u, 0u}, meet[4] = {0u, 0u, 0u, 0u}, leave[4] = {0u, 0u, 0u, 0u};
     cls_words4(
@@ -1169,16 +1161,7 @@ __device__ __forceinline__ SweepOut cls_sweep(const ClsCur& c, uint32_t lnw, uin
     sel &= aw & ~cv;
     bad |= cv & qw;
     if (in) {
-      uint32_t an = prune ? aw & out : aw;
-      if (wl == (cpos >> 5)) {
-        const uint32_t bit = 1u << (cpos & 31);
-        an |= bit;
-        qw |= bit;
-        pw &= ~bit;
-        A[nwp + wl] = qw;
-        A[2 * nwp + wl] = pw;
-      }
-      if (prune) A[wl] = an;
+      if (prune) A[wl] = (aw & out) | (wl == (cpos >> 5) ? 1u << (cpos & 31) : 0u);
       c.S[wl] = sel;
       c.C[wl] = cv;
     }
@@ -1239,15 +1222,15 @@ __device__ __noinline__ void cls_pack_keys(const uint64_t* slk, const int32_t* s
   __syncwarp();
 }
 
-// Writes the child's classes (selection bits S) to list d: masks cut down to
-// ln, moved together to dK words when that is fewer (at most four then).
+// Writes the child's classes (selection bits S of the push of class cpos) to
+// list d: masks cut down to ln, moved together to dK words when that is fewer
+// (at most four then).
 __device__ __noinline__ void cls_copy_child(uint32_t lnw, uint32_t base, uint32_t* dbase, int dn,
-                                            int dK) {
+                                            int dK, int cpos) {
   const ClsCur& c = this_cur();
   const int lane = (int)lane_id();
   const ClsList d = cls_list_at(dbase, dn, dK);
   const ClsList l = c.l;
-  const uint32_t *Q = c.A + c.nwp, *P = Q + c.nwp;
   const bool pack = dK < l.K;
   int o = 0;
   ROLLED for (int b0 = 0; b0 < c.nw; b0 += 32) {
@@ -1260,8 +1243,8 @@ __device__ __noinline__ void cls_copy_child(uint32_t lnw, uint32_t base, uint32_
       const int t = o + __popc(sw & lanemask_lt());
       if (mine) {
         d.key[t] = l.key[i];
-        d.info[t] = (l.info[i] & kInfoCnt) | (((Q[b] >> lane) & 1u) ? kInfoQ : 0u) |
-                    (((P[b] >> lane) & 1u) ? kInfoP : 0u);
+        d.info[t] = (l.info[i] & kInfoCnt) | (((q_bits(c, cpos, b) >> lane) & 1u) ? kInfoQ : 0u) |
+                    (((p_bits(c, cpos, b) >> lane) & 1u) ? kInfoP : 0u);
       }
       if (pack) {
         uint32_t hi[3];
@@ -1286,7 +1269,7 @@ __device__ __noinline__ void cls_copy_child(uint32_t lnw, uint32_t base, uint32_
 
 // Hands the child just selected to an idle warp.
 __device__ __noinline__ bool cls_export(uint32_t lnw, uint32_t base, int nsel, int nselp, int kn,
-                                        uint64_t sR, uint32_t nR) {
+                                        uint64_t sR, uint32_t nR, int cpos) {
   Warp& W = this_warp();
   const ClsCur& c = this_cur();
   const int lane = (int)lane_id();
@@ -1297,7 +1280,7 @@ __device__ __noinline__ bool cls_export(uint32_t lnw, uint32_t base, int nsel, i
   slot = __shfl_sync(kFull, slot, 0);
   if (slot < 0) return false;
   int32_t* sp = slot_ptr(W, slot);
-  cls_copy_child(lnw, base, reinterpret_cast<uint32_t*>(sp + kSlotList), nsel, K);
+  cls_copy_child(lnw, base, reinterpret_cast<uint32_t*>(sp + kSlotList), nsel, K, cpos);
   uint64_t* lk = reinterpret_cast<uint64_t*>(sp + kSlotLk);
   int32_t* lid = s_blk.emit ? sp + kSlotLid : nullptr;
   if (K < cK) {
@@ -1356,14 +1339,13 @@ __device__ __forceinline__ void cls_indices(const uint32_t* S, int nw, uint32_t*
 // are the child's classes; their number is returned, they themselves go to lm
 // (masks), key and info.
 __device__ __noinline__ int cls_child(uint32_t lnw, uint32_t base, int nsel, uint32_t* lm,
-                                      uint64_t* key, uint32_t* info) {
+                                      uint64_t* key, uint32_t* info, int cpos) {
   const ClsCur& c = this_cur();
   const int lane = (int)lane_id();
   const MergeTab t = this_tab();
   uint32_t* g = this_smem() + kSmIdx;
   const bool merge = s_blk.prune != 0;
   const ClsList l = c.l;
-  const uint32_t *Qw = c.A + c.nwp, *Pw = Qw + c.nwp;
   cls_indices(c.S, c.nw, g);
   const uint32_t ln0 = __shfl_sync(kFull, lnw, 0);
   int n = 0;
@@ -1380,7 +1362,8 @@ __device__ __noinline__ int cls_child(uint32_t lnw, uint32_t base, int nsel, uin
         x = l.K == 1 ? (in ? l.m[i] & ln0 : 0u)
                      : cls_pack<false>(l.m, l.stride, l.K, lnw, base, i, in, nullptr);
         if (in) {
-          f = (((Qw[i >> 5] >> (i & 31)) & 1u) << 31) | (((Pw[i >> 5] >> (i & 31)) & 1u) << 30);
+          f = (((q_bits(c, cpos, i >> 5) >> (i & 31)) & 1u) << 31) |
+              (((p_bits(c, cpos, i >> 5) >> (i & 31)) & 1u) << 30);
           if (f & kInfoP) {
             f |= l.info[i] & kInfoCnt;
             k = l.key[i];
@@ -1435,27 +1418,32 @@ __device__ __noinline__ int cls_child(uint32_t lnw, uint32_t base, int nsel, uin
   return n;
 }
 
-// A level of its own for a list (masks at l.m): live, Q and P bits and a frame.
+// A level: live bits and a frame.  last < 0: for a fresh list (masks at l.m),
+// whose Q and P bits are made here too; else on the parent's list, where class
+// `last` was pushed, for the classes selected there.
 __device__ __noinline__ void cls_enter(ClsList l, uint32_t L, int nend, const uint64_t* lk,
                                        const int32_t* lid, uint64_t sR, uint32_t nR,
-                                       uint32_t* top, uint32_t* stop, bool own_bits) {
+                                       uint32_t* top, uint32_t* stop, int last) {
   ClsCur& c = this_cur();
   const int lane = (int)lane_id();
   const uint32_t* send = this_smem() + kSmemWords;
   ClsFrame* fr = reinterpret_cast<ClsFrame*>(top);
   const int nw = (l.n + 31) >> 5, nwp = (nw + 1) & ~1;
+  const int bits = last < 0 ? 3 * nwp : nwp;
   uint32_t* Lw = top + kFrameWords;
   top = Lw + ((l.K + 1) & ~1);
   uint32_t* A;
-  if (3 * nwp <= send - stop) {
+  if (bits <= send - stop) {
     A = stop;
-    stop += 3 * nwp;
+    stop += bits;
   } else {
     A = top;
-    top += 3 * nwp;
+    top += bits;
   }
-  uint32_t *Q = A + nwp, *P = Q + nwp;
-  if (own_bits) {  // a fresh list: everything is live, Q and P as the info words say
+  const uint32_t* QP = c.QP;
+  if (last < 0) {  // everything is live, Q and P as the info words say
+    uint32_t *Q = A + nwp, *P = Q + nwp;
+    QP = Q;
     ROLLED for (int b = 0; b < nw; ++b) {
       const int i = b * 32 + lane;
       const uint32_t f = i < l.n ? l.info[i] : 0u;
@@ -1474,14 +1462,9 @@ __device__ __noinline__ void cls_enter(ClsList l, uint32_t L, int nend, const ui
       l.m = stop;
       stop += words;
     }
-  } else {  // the parent's list: the selected classes
-    const uint32_t *S = c.S, *Qp = c.A + c.nwp, *Pp = Qp + c.nwp;
-    ROLLED for (int b = lane; b < nw; b += 32) {
-      const uint32_t s = S[b];
-      A[b] = s;
-      Q[b] = Qp[b] & s;
-      P[b] = Pp[b] & s;
-    }
+  } else {
+    const uint32_t* S = c.S;
+    ROLLED for (int b = lane; b < nw; b += 32) A[b] = S[b];
   }
   if (lane < l.K) Lw[lane] = L;
   ClsFrame* prev = c.fr;
@@ -1493,15 +1476,17 @@ __device__ __noinline__ void cls_enter(ClsList l, uint32_t L, int nend, const ui
     fr->sR = sR;
     fr->prev = prev;
     fr->A = A;
+    fr->QP = QP;
     fr->top = top;
     fr->stop = stop;
     fr->nR = nR;
     fr->nend = nend;
-    fr->curw = 0;
+    fr->last = last;
     c.l = l;
     c.lk = lk;
     c.lid = lid;
     c.A = A;
+    c.QP = QP;
     c.fr = fr;
     c.top = top;
     c.stop = stop;
@@ -1515,15 +1500,15 @@ __device__ __noinline__ void cls_enter(ClsList l, uint32_t L, int nend, const ui
 }
 
 // Back to the level above (false: there is none); its L in L (lane w: word w),
-// and where its scan stood in curw.
-__device__ __forceinline__ bool cls_leave(ClsCur& c, uint32_t& L, int& curw) {
+// and the class it pushed last in `last`.
+__device__ __forceinline__ bool cls_leave(ClsCur& c, uint32_t& L, int& last) {
   const int lane = (int)lane_id();
   const ClsFrame* fr = c.fr->prev;
   if (!fr) return false;
   __syncwarp();
   const int K = fr->l.K;
   L = lane < K ? (reinterpret_cast<const uint32_t*>(fr) + kFrameWords)[lane] : 0u;
-  curw = fr->curw;
+  last = fr->last;
   if (lane == 0) {
     c.l = fr->l;
     c.lk = fr->lk;
@@ -1531,6 +1516,7 @@ __device__ __forceinline__ bool cls_leave(ClsCur& c, uint32_t& L, int& curw) {
     c.nw = (fr->l.n + 31) >> 5;
     c.nwp = (c.nw + 1) & ~1;
     c.A = fr->A;
+    c.QP = fr->QP;
     c.fr = const_cast<ClsFrame*>(fr);
     c.top = fr->top;
     c.stop = fr->stop;
@@ -1551,14 +1537,14 @@ __device__ __noinline__ bool cls_begin(ClsList* lp, uint32_t L, int* nend, const
   uint32_t* sm = this_smem();
   ClsList l = *lp;
   uint32_t* S = top;
-  uint32_t* C = top + 2 * ((l.n + 63) >> 6);
-  top += 4 * ((l.n + 63) >> 6);
+  uint32_t* C = top + cls_bit_words(l.n);
+  top += 2 * cls_bit_words(l.n);
   if (s_blk.prune && l.n > 32) l.n = cls_merge(l.m, l.key, l.info, l.n, l.K, &l.stride, S, nend);
   *lp = l;
   if (l.n <= 32 && l.K == 1) return true;
   // The two bit strings a push makes go to the shared arena.
   uint32_t* stop = sm + kSmArena;
-  const int nwp = (((l.n + 31) >> 5) + 1) & ~1;
+  const int nwp = (int)cls_bit_words(l.n);
   if (2 * nwp <= sm + kSmemWords - stop) {
     S = stop;
     C = stop + nwp;
@@ -1571,7 +1557,7 @@ __device__ __noinline__ bool cls_begin(ClsList* lp, uint32_t L, int* nend, const
     c.C = C;
   }
   __syncwarp();
-  cls_enter(l, L, *nend, lk, lid, sR0, nR0, top, stop, true);
+  cls_enter(l, L, *nend, lk, lid, sR0, nR0, top, stop, -1);
   return false;
 }
 
@@ -1619,7 +1605,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
   }
   unsigned long long hash = 0;
   Leaf f;
-  int curw = 0;
+  int last = -1;
   bool leaf = cls_begin(&l, L, &nend, lk, lid, sR0, (uint32_t)nR0, top);
   const bool root_leaf = leaf;
   if (leaf) {
@@ -1636,11 +1622,10 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     int cpos = -1;
     {
       const uint32_t* A = c.A;
-      const int nw = c.nw, pofs = 2 * c.nwp;
-      const int e = c.nend;
-      ROLLED for (int b0 = curw; b0 < nw; b0 += 32) {
+      const int nw = c.nw, e = c.nend;
+      ROLLED for (int b0 = (last + 1) >> 5; b0 < nw; b0 += 32) {
         const int w = b0 + lane;
-        const uint32_t t = w < nw ? A[w] & A[pofs + w] & first_bits(e, w) : 0u;
+        const uint32_t t = w < nw ? A[w] & p_bits(c, last, w) & first_bits(e, w) : 0u;
         const unsigned bal = __ballot_sync(kFull, t != 0u);
         if (bal) {
           const int j = __ffs(bal) - 1;
@@ -1650,11 +1635,11 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
       }
     }
     if (cpos < 0) {
-      if (!cls_leave(c, L, curw)) break;
+      if (!cls_leave(c, L, last)) break;
       continue;
     }
     if (tally_step(y, 1024u)) break;
-    curw = cpos >> 5;
+    last = cpos;
     const int K = c.l.K;
     const uint32_t mc = lane < K ? c.l.m[(size_t)lane * c.l.stride + cpos] : 0u;
     const uint32_t lnw = L & mc, rmw = L & ~mc;
@@ -1679,7 +1664,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     }
     // A big enough child goes to an idle warp instead, at any depth, so that a
     // subtree that started here can still be shared once warps run out of work.
-    if (nselp * (long long)kn >= y.share_floor && cls_export(lnw, base, nsel, nselp, kn, sR, nR))
+    if (nselp * (long long)kn >= y.share_floor && cls_export(lnw, base, nsel, nselp, kn, sR, nR, cpos))
       continue;
     const int kc = words_k(kn);
     const int dK = kc <= kKMax && kc < K ? kc : K;
@@ -1687,12 +1672,11 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     const long long keys = pack ? 64LL * dK + (s_blk.emit ? 32LL * dK : 0) : 0;
     const bool tiny = kn <= 32 && nsel <= 32;
     uint32_t* at = c.top;
-    if (lane == 0) c.fr->curw = curw;
+    if (lane == 0) c.fr->last = cpos;
     if (!tiny && cls_need(nsel, dK, cls_levels(kn, nselp)) + keys > end - at) {
       // ---- no room: a level on the parent's list ----
-      cls_enter(c.l, lnw, c.l.n, c.lk, c.lid, sR, nR, at, c.stop, false);
+      cls_enter(c.l, lnw, c.l.n, c.lk, c.lid, sR, nR, at, c.stop, cpos);
       L = lnw;
-      curw = 0;
       continue;
     }
     const uint64_t* clk = c.lk;
@@ -1712,10 +1696,9 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
       cls_indices(c.S, c.nw, g);
       const bool in = lane < nsel;
       const int i = in ? (int)g[lane] : 0;
-      const uint32_t* Q = c.A + c.nwp;
       f.A = first_bits(nsel, 0);
-      f.Q = __ballot_sync(kFull, in && ((Q[i >> 5] >> (i & 31)) & 1u));
-      f.P = __ballot_sync(kFull, in && ((Q[c.nwp + (i >> 5)] >> (i & 31)) & 1u));
+      f.Q = __ballot_sync(kFull, in && ((q_bits(c, cpos, i >> 5) >> (i & 31)) & 1u));
+      f.P = __ballot_sync(kFull, in && ((p_bits(c, cpos, i >> 5) >> (i & 31)) & 1u));
       const bool p = (f.P >> lane) & 1u;
       f.key = p ? c.l.key[i] : 0ULL;
       f.cnt = p ? c.l.info[i] & kInfoCnt : 0u;
@@ -1732,14 +1715,14 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
       if (kn <= 32 && nsel <= kChildMax) {
         uint32_t* lm = d.m;
         if (d.stride <= this_smem() + kSmemWords - stop) lm = stop;
-        d.n = cls_child(lnw, base, nsel, lm, d.key, d.info);
+        d.n = cls_child(lnw, base, nsel, lm, d.key, d.info, cpos);
         d.stride = (d.n + 31) & ~31;
         d.m = lm;
         leaf = d.n <= 32;
         if (leaf) leaf_of_list(d, 0u, d.n, clk, sR, nR, f);
         else if (lm == stop) stop += d.stride;
       } else {
-        cls_copy_child(lnw, base, d.m, nsel, dK);
+        cls_copy_child(lnw, base, d.m, nsel, dK, cpos);
         int dend = nsel;
         if (s_blk.prune && nsel > 32)
           d.n = cls_merge(d.m, d.key, d.info, nsel, dK, &d.stride, c.S, &dend);
@@ -1749,9 +1732,9 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
         }
       }
       if (!leaf) {
-        cls_enter(d, nl, d.n, clk, clid, sR, nR, at + cls_list_words(nsel, dK), stop, true);
+        cls_enter(d, nl, d.n, clk, clid, sR, nR, at + cls_list_words(nsel, dK), stop, -1);
         L = lane < dK ? nl : 0u;
-        curw = 0;
+        last = -1;
       }
     }
     if (leaf) {
@@ -1804,7 +1787,7 @@ __device__ __noinline__ void tier2_from_slot(int slot) {
   uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_root));
   uint64_t* lkey = reinterpret_cast<uint64_t*>(at);
   int32_t* lid = reinterpret_cast<int32_t*>(at + 64 * K);
-  const ClsList l = cls_list_at(at + 96 * K, n, K);
+  const ClsList l = cls_list_at(at + cls_key_words(K), n, K);
   const int nw = (int)cls_list_words(n, K);
   const uint4* src = reinterpret_cast<const uint4*>(sp + kSlotList);
 #pragma unroll 4
@@ -1823,13 +1806,6 @@ __device__ __noinline__ void tier2_from_slot(int slot) {
   cls_run(l, L, n, lkey, lid, sR, nR, l.m + nw, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)));
 }
 
-// Words of scratch cls_build may use on top of cls_need for a list of `eff`
-// classes made of n candidates over nL vertices.
-__host__ __device__ __forceinline__ long long cls_build_words(long long n, long long eff, int K,
-                                                              int nL) {
-  return cls_stride(eff) * (K + 1) + 4 * ((n + 63) >> 5) + 4LL * nL + 64;
-}
-
 // The edges between a sub-problem's candidates and its vertices: edge e joins
 // candidate tab[ids[e]] - bias (below 0: none) and vertex rows[e]; without
 // rows, ids holds both, id << 7 | vertex.
@@ -1839,10 +1815,11 @@ struct ClsEdges {
 };
 
 // Builds the class list of n candidates, [Q | P], the first nq of them Q, over
-// nL vertices, at `at` ([at, end): at least cls_need + cls_build_words).
-// Candidate i has cnt[i] of the vertices and hash key keys[vidx[i]].  *nend:
-// candidates [0, nend) may be pushed at the first level; classes [0, nend) on
-// return.
+// nL vertices, at `at` ([at, end): at least cls_list_words + cls_build_words).
+// Candidate i has cnt[i] of the vertices and hash key keys[vidx[i]]; without
+// cnt, vidx[i] is complemented if it has one of them only.  *nend: candidates
+// [0, nend) may be pushed at the first level; classes [0, nend) on return.
+// mpos: room for n words, or null (it is taken from the end then).
 //
 // Most candidates of a root have one of its vertices only (on the 300,000-edge
 // serving graph a root has 1,565 candidates and 1,867 edges to them).  Those
@@ -1850,7 +1827,7 @@ struct ClsEdges {
 // summed up per vertex as the edges are walked, and only the others get masks.
 __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, int nq, int K, int nL,
                                           int* nend, const int32_t* cnt, const uint64_t* keys,
-                                          const int32_t* vidx, ClsEdges ed) {
+                                          const int32_t* vidx, ClsEdges ed, uint32_t* mpos) {
   const int lane = (int)lane_id();
   const bool merge = s_blk.prune != 0;
   const int nw = (n + 31) >> 5;
@@ -1870,7 +1847,8 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
 #pragma unroll 2
   for (int b = 0; b < nw; ++b) {
     const int i = b * 32 + lane;
-    const unsigned bal = __ballot_sync(kFull, i < n && (!merge || cnt[i] >= 2));
+    const unsigned bal =
+        __ballot_sync(kFull, i < n && (!merge || (cnt ? cnt[i] >= 2 : vidx[i] >= 0)));
     if (lane == 0) {
       MB[b] = FB[b] = bal;
       MP[b] = (uint32_t)nm;
@@ -1878,8 +1856,14 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
     nm += __popc(bal);
   }
   const int st = (nm + 31) & ~31;
-  end -= st;
-  uint32_t* mpos = end;  // candidate of each mask
+  if (!mpos) {
+    end -= st;
+    mpos = end;  // candidate of each mask
+  }
+  const auto key_of = [&](int i) {
+    const int v = vidx[i];
+    return keys[v < 0 ? ~v : v];
+  };
   uint32_t* raw;
   if (K * st <= send - sm) {
     raw = sm;
@@ -1888,20 +1872,11 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
     raw = end;
   }
   ROLLED for (int i = lane; i < K * st; i += 32) raw[i] = 0u;
-  // Sums per vertex: the table's entries, or (more vertices than it has) an
-  // array of four words each.
+  // Sums per vertex: the table's entries.
+  static_assert(32 * kKMax <= kSlots, "an entry per vertex");
   const MergeTab t = this_tab();
-  const bool wide = nL > kSlots;
   uint32_t* first = t.lead;  // 0x7fffffff - the first P candidate, or 0
   uint32_t* info = t.info;
-  unsigned long long* key64 = nullptr;
-  if (wide) {
-    end -= 4 * ((nL + 1) & ~1);
-    first = end;
-    info = first + ((nL + 1) & ~1);
-    key64 = reinterpret_cast<unsigned long long*>(info + ((nL + 1) & ~1));
-    ROLLED for (int i = lane; i < 4 * ((nL + 1) & ~1); i += 32) first[i] = 0u;
-  }
   __syncwarp();
   ROLLED for (int w = lane; w < nw; w += 32) {
     const uint32_t o = MP[w];
@@ -1932,14 +1907,10 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
         atomicOr(&info[r], kInfoQ);
       } else {
         atomicMax(&first[r], 0x7fffffffu - (uint32_t)i);
-        const uint64_t k = keys[vidx[i]];
-        if (wide) {
-          atomicAdd(&key64[r], (unsigned long long)k);
-        } else {
-          const uint32_t lo = (uint32_t)k;
-          const uint32_t old = atomicAdd(&t.lo[r], lo);
-          atomicAdd(&t.hi[r], (uint32_t)(k >> 32) + (old + lo < lo ? 1u : 0u));
-        }
+        const uint64_t k = key_of(i);
+        const uint32_t lo = (uint32_t)k;
+        const uint32_t old = atomicAdd(&t.lo[r], lo);
+        atomicAdd(&t.hi[r], (uint32_t)(k >> 32) + (old + lo < lo ? 1u : 0u));
         atomicAdd(&info[r], 1u);
       }
     }
@@ -1980,7 +1951,7 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
     ROLLED for (int w = 0; w < K; ++w) l.m[(size_t)w * l.stride + f] = raw[(size_t)w * st + d];
     l.info[f] = i < nq ? kInfoQ : kInfoP | 1u;
     // Only P candidates' keys can enter an R that is counted.
-    l.key[f] = i < nq ? 0ULL : keys[vidx[i]];
+    l.key[f] = i < nq ? 0ULL : key_of(i);
   }
   int oq = nqm;
   ROLLED for (int r0 = 0; r0 < nL; r0 += 32) {
@@ -1993,8 +1964,8 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
       ROLLED for (int w = 0; w < K; ++w)
         l.m[(size_t)w * l.stride + f] = w == (r >> 5) ? 1u << (r & 31) : 0u;
       l.info[f] = fl | (v ? kInfoP : 0u);
-      l.key[f] = wide ? key64[r] : (uint64_t)t.lo[r] | ((uint64_t)t.hi[r] << 32);
-      if (!wide) first[r] = info[r] = t.lo[r] = t.hi[r] = 0u;
+      l.key[f] = (uint64_t)t.lo[r] | ((uint64_t)t.hi[r] << 32);
+      first[r] = info[r] = t.lo[r] = t.hi[r] = 0u;
     }
     oq += __popc(bal);
   }
@@ -2127,9 +2098,10 @@ __device__ __noinline__ void t1_pop(int nL, int x, int level) {
 
 // Hands the child sub-problem of a maximal push (x at `level`, |L_new| = kept)
 // to tier 2.  Candidates: C entries live below this level with
-// 0 < count < kept; Q = those before x.
-// Declined (false, nothing done) if the warp's arena may not hold it.
-__device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, uint64_t sR,
+// 0 < count < kept; Q = those before x.  Pruning is off here: with it, the
+// sparse push takes every child that the bitmap tier may run (its indices, -1
+// between pushes, would not survive this one).
+__device__ __noinline__ void t1_handoff(const T1 t, int x, int level, int kept, uint64_t sR,
                                         uint64_t nR) {
   Warp& W = this_warp();
   const int lane = (int)lane_id();
@@ -2155,10 +2127,6 @@ __device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, 
   nsub = (int)__reduce_add_sync(kFull, (unsigned)nsub);
   nq = (int)__reduce_add_sync(kFull, (unsigned)nq);
   const int K = words_k(kept);
-  if (nsub > 0 && cls_need(nsub, K, cls_levels(kept, nsub - nq)) +
-                          cls_build_words(nsub, nsub, K, kept) + cls_stride(nsub) >
-                      W.sub_words())
-    return false;
   // L_sub positions
   int n = 0;
   ROLLED for (int c0 = 0; c0 < t.nL; c0 += 32) {
@@ -2175,8 +2143,8 @@ __device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, 
   }
   if (nsub > 0) {
     uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub));
-    uint32_t* cpos = at;  // C index of each candidate
-    at += cls_stride(nsub);
+    uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)) - cls_stride(nsub);
+    int32_t* cpos = reinterpret_cast<int32_t*>(end);  // C index of each candidate
     int o = 0;
     ROLLED for (int c0 = 0; c0 < t.nC; c0 += 32) {
       const int i = c0 + lane;
@@ -2185,7 +2153,7 @@ __device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, 
       if (sel) {
         const int s = o + __popc(bal & lanemask_lt());
         sidx[i] = s;
-        cpos[s] = (uint32_t)i;
+        cpos[s] = i;
       } else if (i < t.nC) {
         sidx[i] = -1;
       }
@@ -2208,13 +2176,12 @@ __device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, 
           ne += __popc(be);
         });
     __syncwarp();
-    const ClsList l = cls_build(at, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)), nsub, nq, K, n,
-                                &nend, nullptr, ckey, reinterpret_cast<int32_t*>(cpos),
-                                ClsEdges{ent, nullptr, sidx, ne, 0});
+    const ClsList l =
+        cls_build(at, end, nsub, nq, K, n, &nend, nullptr, ckey, cpos,
+                  ClsEdges{ent, nullptr, sidx, ne, 0}, reinterpret_cast<uint32_t*>(W.A(W.sl().tcls)));
     tier2(W, l, n, nend, sR, nR);
   }
   __syncwarp();
-  return true;
 }
 
 // A push at `level` whose child L (the `kept` rows, marked llevel == level)
@@ -2227,9 +2194,8 @@ __device__ __noinline__ bool t1_handoff(const T1 t, int x, int level, int kept, 
 // candidate of bound >= level is FREE before the push, and candidates not
 // adjacent to the kept rows are either touched (stay FREE) or irrelevant
 // below this level (count 0), so only candidates adjacent to the kept rows
-// change.  Declined (false, nothing done) if the warp's arena may not hold the
-// child.
-__device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int kept, uint64_t sL) {
+// change.
+__device__ __noinline__ void t1_sparse_push(const T1 t, int x, int level, int kept, uint64_t sL) {
   Warp& W = this_warp();
   const int lane = (int)lane_id();
   int32_t* llevel = W.A(W.sl().llevel);
@@ -2329,7 +2295,7 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
   bool ism = true;
   uint64_t sR = 0;
   unsigned long long nR = 0;
-  int ncand = 0, nqc = 0, nmul = 0;
+  int ncand = 0, nqc = 0;
 #pragma unroll 4
   for (int q = lane; q < nt; q += 32) {
     const int p = tl[q];
@@ -2344,24 +2310,14 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
       cls = p < x ? 1 : 2;
       ++ncand;
       nqc += cls == 1;
-      nmul += c >= 2;
     }
     tcls[q] = cls;
   }
   ism = __all_sync(kFull, ism);
   ncand = (int)__reduce_add_sync(kFull, (unsigned)ncand);
   nqc = (int)__reduce_add_sync(kFull, (unsigned)nqc);
-  nmul = (int)__reduce_add_sync(kFull, (unsigned)nmul);
   const int K = words_k(n);
-  const int eff = min(ncand, nmul + kept);  // classes of the child, at most
   const int levels = cls_levels(kept, ncand - nqc);
-  if (ism && kept > 1 && ncand > 0 &&
-      cls_need(eff, K, levels) + cls_build_words(ncand, eff, K, kept) + 2 * cls_stride(ncand) >
-          W.sub_words()) {
-    ROLLED for (int q = lane; q < nt; q += 32) cc[tl[q]] = 0;
-    __syncwarp();
-    return false;
-  }
   sR = warp_sum64(sR) + t.sRtask;
   nR = warp_sum64(nR) + t.nRtask;
   if (ism) {
@@ -2375,10 +2331,9 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
   if (ism && kept > 1 && ncand > 0) {
     // child indices: Q from the front, P from the back
     uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub));
-    int32_t* cpos = reinterpret_cast<int32_t*>(at);  // C index of each child candidate
-    at += cls_stride(ncand);
-    int32_t* ccnt = reinterpret_cast<int32_t*>(at);  // its count in the kept rows
-    at += cls_stride(ncand);
+    uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)) - cls_stride(ncand);
+    // C index of each child candidate, complemented if it meets one kept row
+    int32_t* cpos = reinterpret_cast<int32_t*>(end);
     int nq = 0, np = 0;
     ROLLED for (int b0 = 0; b0 < nt; b0 += 32) {
       int q = b0 + lane;
@@ -2391,16 +2346,16 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
       if (cls == 2) s = ncand - 1 - (np + __popc(bp & lanemask_lt()));
       if (s >= 0) {
         sidx[p] = s;
-        cpos[s] = p;
-        ccnt[s] = cc[p];
+        cpos[s] = cc[p] >= 2 ? p : ~p;
       }
       nq += __popc(bq);
       np += __popc(bp);
     }
     __syncwarp();
     int nend = ncand;
-    const ClsList l = cls_build(at, reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)), ncand, nqc, K,
-                                n, &nend, ccnt, ckey, cpos, ClsEdges{ent, nullptr, sidx, ne, 0});
+    const ClsList l =
+        cls_build(at, end, ncand, nqc, K, n, &nend, nullptr, ckey, cpos,
+                  ClsEdges{ent, nullptr, sidx, ne, 0}, reinterpret_cast<uint32_t*>(tcls));
     // To an idle warp when some want work and the child is big enough by
     // GMBE's split test, else it runs here.
     int slot = -1;
@@ -2447,7 +2402,6 @@ __device__ __noinline__ bool t1_sparse_push(const T1 t, int x, int level, int ke
   if (level == 1) acc(W.dead, __reduce_add_sync(kFull, gone));
   ROLLED for (int q = lane; q < n; q += 32) llevel[lp[q]] = level - 1;
   __syncwarp();
-  return true;
 }
 
 // A push at `level` that keeps one or two rows (la; lb, or -1), whole: what
@@ -2897,7 +2851,8 @@ __device__ __noinline__ void tier1_run(const T1 t) {
       kent = warp_sum64(kent);
       best = warp_min_u64(best);
       __syncwarp();
-      if (s_blk.prune && kept <= t2max && t1_sparse_push(t, cur, level, kept, sL)) {
+      if (s_blk.prune && kept <= t2max) {
+        t1_sparse_push(t, cur, level, kept, sL);
         if (lane == 0) stack[level - 1] = cur + 1;
         __syncwarp();
         continue;
@@ -2958,10 +2913,9 @@ __device__ __noinline__ void tier1_run(const T1 t) {
       }
       __syncwarp();
       if (ism && kept > 1) {
-        // (Pruning on, a child the sparse push declined is not handed over
-        // either: the hand-off keeps no counts of its candidates, by which the
-        // class list is built then, and leaves its indices in sidx.)
-        if (kept > t2max || s_blk.prune || !t1_handoff(t, cur, level, kept, sR, nR)) {
+        if (kept <= t2max) {
+          t1_handoff(t, cur, level, kept, sR, nR);
+        } else {
           uint32_t* nbits = level_bits(W, level + 1);
           // The candidates the kept rows meet, as a bitmap: the next level's
           // own one, or (deeper levels) the warp's global touch bitmap, built
@@ -3527,7 +3481,7 @@ __device__ __noinline__ void run_task(const Task& t) {
   // pushes the candidates of this part; those before it act as Q, those after
   // it stay candidates of the children.
   int part = t.part, parts = t.parts;
-  int cntQ = 0, cntPre = 0, cntIn = 0, cntM = 0;
+  int cntQ = 0, cntPre = 0, cntIn = 0;
   {
     int cntC = 0;
     bool r_below = false;
@@ -3538,7 +3492,6 @@ __device__ __noinline__ void run_task(const Task& t) {
       int c = valid ? map[w] : 0;
       bool isC = valid && c != nL;
       cntC += __popc(__ballot_sync(kFull, isC));
-      cntM += __popc(__ballot_sync(kFull, isC && c >= 2));
       cntQ += __popc(__ballot_sync(kFull, isC && w < last));
       r_below |= __ballot_sync(kFull, valid && c == nL && w < last) != 0u;
     }
@@ -3725,10 +3678,7 @@ __device__ __noinline__ void run_task(const Task& t) {
   }
   if (!done) {
     const int K = words_k(nL);
-    const int eff = s_blk.prune ? min(nC, cntM + nL) : nC;
-    if (nL <= W.gp->tier2_max_l && nC <= W.gp->direct_max_c &&
-        cls_need(eff, K, cls_levels(nL, nC - nq)) + cls_build_words(nC, eff, K, nL) + 96LL * K <=
-            W.root_words()) {
+    if (nL <= W.gp->tier2_max_l && nC <= W.gp->direct_max_c) {
       // ---- tier 2 directly ----
       uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_root));
       uint64_t* lkey = reinterpret_cast<uint64_t*>(at);
@@ -3738,8 +3688,8 @@ __device__ __noinline__ void run_task(const Task& t) {
         ROLLED for (int l = lane; l < nL; l += 32) lid[l] = L[l];
       uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end));
       const ClsList cl = cls_build(
-          at + 96 * K, end, nC, nq, K, nL, &nend, ncnt, g.vkey, cv,
-          ClsEdges{W.A(W.sl().aadj), W.A(W.sl().ent), map, entries, 1});
+          at + cls_key_words(K), end, nC, nq, K, nL, &nend, ncnt, g.vkey, cv,
+          ClsEdges{W.A(W.sl().aadj), W.A(W.sl().ent), map, entries, 1}, nullptr);
       cls_run(cl, first_bits(nL, lane), nend, lkey, lid, sR, nR,
               cl.m + cls_list_words(cl.n, cl.K), end);
     } else {

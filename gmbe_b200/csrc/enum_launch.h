@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "cls_sizes.h"
 #include "enum_common.cuh"
 
 namespace gmbe {
@@ -17,7 +18,6 @@ constexpr int kEnumWarps = GMBE_ENUM_WARPS;    // warps per block
 constexpr int kEnumThreads = kEnumWarps * 32;  // threads per block
 // Blocks per SM the register allocation is made for (launch bounds).
 constexpr int kEnumMinBlocks = GMBE_ENUM_MIN_BLOCKS;
-constexpr int kKMax = 4;                       // bitmap words of the tier-2 sub-problem
 constexpr int kChildMax = 128;                 // largest child that is merged on the way to its list
 constexpr int kSmemWords = 2488;               // shared memory words of a warp
 constexpr int kLevelBits = 8;                  // counts-tier levels with a candidate bitmap

@@ -32,7 +32,8 @@ def nested(nV, nL, kept, n, seed):
 
 SHAPES = [(700, 140, 100, 560), (700, 140, 100, 608), (700, 140, 100, 680),
           (900, 140, 128, 560), (900, 140, 128, 608), (900, 140, 128, 800),
-          (8000, 140, 48, 7000), (8000, 140, 48, 7800), (2500, 150, 64, 2450)]
+          (1000, 140, 128, 997), (5000, 130, 128, 4990), (8000, 140, 48, 7000),
+          (8000, 140, 48, 7800), (2500, 150, 64, 2450)]
 
 
 @pytest.mark.parametrize("nV,nL,kept,n", SHAPES)
@@ -43,12 +44,12 @@ def test_wide_children_match_oracle(nV, nL, kept, n):
         want = oracle.gmbe(*g, uvtrans=0, order=order)
         with gm.Graph.from_csr(*g, uvtrans=0, order=order) as G:
             runs = [dict(), dict(share_counts=-1), dict(share_min_work=1), dict(direct_max_c=1)]
-            if nV < 1000:  # (a tree thousands of times as large at 8,000)
+            if nV <= 1000:  # (a tree thousands of times as large at 8,000)
                 runs.append(dict(prune=0))
             for params in runs:
                 r = G.enumerate(wait_limit_ns=30 * 10**9, time_limit_ns=60 * 10**9, **params)
                 assert (r.count, r.set_hash) == (want.count, want.set_hash), (order, params)
-            if nV < 1000:
+            if nV <= 1000:
                 r, found = G.enumerate_emit(1 << 22, time_limit_ns=60 * 10**9)
                 assert len(set(found)) == len(found) == want.count
                 assert r.set_hash == want.set_hash
@@ -63,3 +64,21 @@ def test_wide_children_in_a_batch():
         per, _ = batch.run()
         assert [(r.count, r.set_hash) for r in per] == [(w.count, w.set_hash) for w in want]
     batch.free()
+
+
+# Rejected pushes with pruning off, as the engine counted them when the bitmap
+# tier walked single candidates (which tier runs a child decides the order of
+# its pushes, and with it this count).
+@pytest.mark.parametrize("nV,nL,kept,n,nonmax", [
+    (700, 140, 100, 560, 68424), (700, 140, 100, 680, 88800),
+    (900, 140, 128, 560, 82175), (900, 140, 128, 800, 112055), (1000, 140, 128, 997, 136975)])
+def test_wide_children_stay_in_the_bitmap_tier(nV, nL, kept, n, nonmax):
+    import gmbe_b200 as gm
+    g = nested(nV, nL, kept, n, seed=n)
+    with gm.Graph.from_csr(*g, uvtrans=0, order=0) as G:
+        r = G.enumerate(prune=0, wait_limit_ns=30 * 10**9)
+        assert r.non_maximal == nonmax
+        # pruning on: the first level's pushes only
+        r = G.enumerate(split_mode=1, bound_height=1 << 20, bound_size=1 << 30)
+        assert r.max_task_pushes1 < nV
+        assert r.non_maximal == G.enumerate(share_min_work=1).non_maximal
