@@ -176,8 +176,7 @@ ScratchLayout make_layout(int32_t nV, int32_t capC, int32_t capL, int32_t capS) 
   s.ar_end = off;
   s.words_per_warp = off;
   const int64_t seen = ((int64_t)nV + 31) / 32;
-  s.seen_words = seen <= kSeenMaxWords ? (int32_t)((seen + 3) & ~int64_t(3)) : 0;
-  s.smem_words = std::max(s.seen_words, kSmemWords);
+  set_seen_words(&s, seen <= kSeenMaxWords ? (int32_t)((seen + 3) & ~int64_t(3)) : 0);
   return s;
 }
 

@@ -99,7 +99,7 @@ struct ScratchLayout {
   // V vertex / candidate position); 0 = first touches found by global atomics.
   int32_t seen_words;
   // Shared memory words per warp: the larger of that bitmap and what the
-  // bitmap tier uses (kSmemWords; fewer: it runs without, and merges nothing).
+  // bitmap tier uses (at least kSmemWords: it uses them in every launch).
   int32_t smem_words;
   // A first-touch bitmap in global memory (one bit per V vertex / candidate
   // position, gseen_words words), right after the count map: large counting

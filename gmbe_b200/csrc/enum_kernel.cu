@@ -139,6 +139,7 @@ struct Block {
   int32_t prune, server, share_min_work, slot_records, eager_share, share_counts, touch_scan;
   int32_t smem_words;
   int32_t lookout;  // 1 while an idle warp of the block watches the queue
+  unsigned long long last_ns, busy_ns;  // per-block timing, at the launch's end
 };
 
 struct Warp {
@@ -169,6 +170,11 @@ struct Warp {
 __shared__ Block s_blk;
 __shared__ ScratchLayout s_sl[2];
 __shared__ Warp s_warp[kEnumWarps];
+static_assert(sizeof(Block) + 2 * sizeof(ScratchLayout) + kEnumWarps * sizeof(Warp) + 64 +
+                      kEnumWarps * sizeof(uint32_t) *
+                          (kSeenMaxWords > kSmemWords ? kSeenMaxWords : kSmemWords) <=
+                  kBlockSmemBytes,
+              "a block's shared memory (64 bytes: alignment)");
 extern __shared__ uint4 enum_smem4[];
 
 __device__ __forceinline__ Warp& this_warp() { return s_warp[threadIdx.x >> 5]; }
@@ -4074,20 +4080,19 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
   }
   if (p.record_exit) {
     // Per block: when its last task finished, and its warps' summed busy time.
-    __shared__ unsigned long long blk_last, blk_busy;
     if (threadIdx.x == 0) {
-      blk_last = 0;
-      blk_busy = 0;
+      s_blk.last_ns = 0;
+      s_blk.busy_ns = 0;
     }
     __syncthreads();
     if (lane == 0) {
-      atomicMax(&blk_last, (unsigned long long)last_done_ns);
-      atomicAdd(&blk_busy, (unsigned long long)busy_ns);
+      atomicMax(&s_blk.last_ns, (unsigned long long)last_done_ns);
+      atomicAdd(&s_blk.busy_ns, (unsigned long long)busy_ns);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      exit_ns[blockIdx.x] = blk_last;
-      exit_ns[gridDim.x + blockIdx.x] = blk_busy;
+      exit_ns[blockIdx.x] = s_blk.last_ns;
+      exit_ns[gridDim.x + blockIdx.x] = s_blk.busy_ns;
     }
   }
 }

@@ -43,8 +43,17 @@ constexpr int kSlotWordsHost = 32768;  // int32 words per sub-problem slot (128 
 // Most candidate records one slot carries (K = 1): a warp that may run
 // another warp's exported sub-problem needs room for this many candidates.
 constexpr int32_t kSlotMaxRecords = 8064;
-// Largest first-touch bitmap per warp (kEnumWarps of them fit the 227 KiB a block may use).
+// Largest first-touch bitmap per warp: kEnumWarps of them and what the kernel
+// holds in static shared memory fit the 227 KiB a block may use (the kernel
+// asserts it).
 constexpr int kSeenMaxWords = 3584;
+constexpr int kBlockSmemBytes = 227 * 1024;
+// Gives a layout a first-touch bitmap of that many words in shared memory (0:
+// none), next to the words that the bitmap tier always uses.
+inline void set_seen_words(ScratchLayout* sl, int32_t words) {
+  sl->seen_words = words;
+  sl->smem_words = words > kSmemWords ? words : kSmemWords;
+}
 // Dynamic shared memory of a launch with layout sl.
 inline size_t enum_smem_bytes(const ScratchLayout& sl) {
   return (size_t)sl.smem_words * sizeof(uint32_t) * kEnumWarps;

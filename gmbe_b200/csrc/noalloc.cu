@@ -127,8 +127,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
     return set_error(MBE_ERR_CAPACITY, "graph too large for the no-allocation pool");
   ScratchLayout sl = make_layout(nV, capC, capL, capS);
   // First touches by global atomics; shared memory for the bitmap tier only.
-  sl.seen_words = 0;
-  sl.smem_words = kSmemWords;
+  set_seen_words(&sl, 0);
 
   // Pool partition: control block, split ring, per-block timing, hash keys,
   // then as many 16-warp blocks of per-warp scratch as fit.
