@@ -276,12 +276,15 @@ int apply_tuning(const mbe_params& prm, DevGraph* dg) {
 
 int enum_blocks_per_sm(bool tiers, size_t smem, int* occ) {
   const void* fn = tiers ? (const void*)mbe_enum_kernel_tiers : (const void*)mbe_enum_kernel;
-  // The limit only ever rises: a server and single-graph launches may share
-  // the kernel from different threads, each with its own bitmap size.
+  // Always all that a block may have: servers, single-graph and no-allocation
+  // launches share the kernel from different threads, each with its own bitmap
+  // size, and one that raised the limit to its own size could lower it under
+  // another that was about to launch.
   cudaFuncAttributes fa;
   CK(cudaFuncGetAttributes(&fa, fn));
-  if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int most = kBlockSmemBytes - (int)fa.sharedSizeBytes;
+  if (fa.maxDynamicSharedSizeBytes < most)
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, fn, kEnumThreads, smem));
   if (*occ < 1) return set_error(MBE_ERR_CUDA, "enumeration kernel cannot be resident");
   return MBE_OK;

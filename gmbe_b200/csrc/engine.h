@@ -126,7 +126,7 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
 
 // Resident blocks per SM of the enumeration kernel (the two-tier variant if
 // `tiers`) with `smem` bytes of dynamic shared memory per block; also raises
-// the kernel's dynamic shared memory limit to `smem` where it is lower.
+// the kernel's dynamic shared memory limit to the most a block may have.
 int enum_blocks_per_sm(bool tiers, size_t smem, int* occ);
 
 // Whether every warp's count map is all-zero where the plan's layout has it.
