@@ -652,8 +652,7 @@ __device__ void slot_header(int32_t* sp, int K, int n, int kn, uint64_t sR, uint
 
 // Bit i of word w set below i classes: the first n bits of a bit string.
 __device__ __forceinline__ uint32_t first_bits(int n, int w) {
-  const int b = n - 32 * w;
-  return b >= 32 ? 0xffffffffu : (b <= 0 ? 0u : (1u << b) - 1u);
+  return ~__funnelshift_lc(0u, 0xffffffffu, (unsigned)max(n - 32 * w, 0));  // (clamped at 32)
 }
 
 // ---------------------------------------------------------------------------
@@ -959,19 +958,21 @@ struct Tally {
   int swapped;
   int share_floor;        // |P|*|L| from which a child may be shared out
 };
-__device__ __forceinline__ void tally_fold(Tally& y) {
+// Adds the counts to the totals; whether the walk should stop.
+__device__ __noinline__ bool tally_look(uint32_t cnt, uint32_t nonmax) {
   Warp& W = this_warp();
-  acc(W.cnt, y.cnt);
-  acc(W.nonmax, y.nonmax);
-  acc(W.pushes, (unsigned long long)(y.cnt + y.nonmax) << 32);
-  y.cnt = y.nonmax = 0u;
+  acc(W.cnt, cnt);
+  acc(W.nonmax, nonmax);
+  acc(W.pushes, (unsigned long long)(cnt + nonmax) << 32);
+  return must_stop();
 }
 // Counts a step; whether the walk should stop.  `every`: steps between looks, a
 // divisor of kLookSteps.
 __device__ __forceinline__ bool tally_step(Tally& y, uint32_t every) {
   if ((++y.steps & (every - 1u)) != 0u) return false;
-  tally_fold(y);
-  return must_stop();
+  const bool stop = tally_look(y.cnt, y.nonmax);
+  y.cnt = y.nonmax = 0u;
+  return stop;
 }
 
 // Walks a leaf sub-problem (lid: the internal U id of each L bit, for
@@ -1756,7 +1757,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     }
   }
   hash += warp_sum64(y.hl);
-  tally_fold(y);
+  tally_look(y.cnt, y.nonmax);
   Warp& W = this_warp();
   acc(W.hash, hash);
   acc(W.ns_t2, globaltimer_ns() - t0);
