@@ -1850,11 +1850,61 @@ __device__ __noinline__ void tier2_from_slot(int slot) {
 
 // The edges between a sub-problem's candidates and its vertices: edge e joins
 // candidate tab[ids[e]] - bias (below 0: none) and vertex rows[e]; without
-// rows, ids holds both, id << 7 | vertex.
+// rows, ids holds both, id << 7 | vertex.  Without ids (n = 0), they are the
+// graph's U -> V rows of the vertices L.
 struct ClsEdges {
   const int32_t *ids, *rows, *tab;
   int n, bias;
+  const int32_t* L;
 };
+
+// The candidates of a list being built that get masks (bits and ranks, MB and
+// MP), and their masks (K planes of st words).
+struct ClsRaw {
+  const uint32_t *MB, *MP;
+  uint32_t* raw;
+  int st, nq;
+};
+
+// An edge between candidate i and vertex r: a bit of the candidate's mask, or,
+// where it gets none, into the vertex's sums.
+__device__ __forceinline__ void cls_edge(const ClsRaw& b, const MergeTab& t, const uint64_t* keys,
+                                         const int32_t* vidx, int i, int r) {
+  const uint32_t w = b.MB[i >> 5], bit = 1u << (i & 31);
+  if (w & bit) {
+    const uint32_t d = b.MP[i >> 5] + __popc(w & (bit - 1u));
+    atomicOr(&b.raw[(size_t)(r >> 5) * b.st + d], 1u << (r & 31));
+  } else if (i < b.nq) {
+    atomicOr(&t.info[r], kInfoQ);
+  } else {
+    atomicMax(&t.lead[r], 0x7fffffffu - (uint32_t)i);
+    const int v = vidx[i];
+    const uint64_t k = keys[v < 0 ? ~v : v];
+    const uint32_t lo = (uint32_t)k;
+    const uint32_t old = atomicAdd(&t.lo[r], lo);
+    atomicAdd(&t.hi[r], (uint32_t)(k >> 32) + (old + lo < lo ? 1u : 0u));
+    atomicAdd(&t.info[r], 1u);
+  }
+}
+
+// All edges, from the graph's rows.
+__device__ __noinline__ void cls_edges_of_rows(ClsRaw b, const uint64_t* keys, const int32_t* vidx,
+                                               const int32_t* tab, int bias, const int32_t* L,
+                                               int nL) {
+  const MergeTab t = this_tab();
+  const int32_t *rev_off = this_warp().gp->rev_off, *rev_col = this_warp().gp->rev_col;
+  flat_rows(
+      nL,
+      [&](int r, int& beg, int& len) {
+        const int u = L[r];
+        beg = rev_off[u];
+        len = rev_off[u + 1] - beg;
+      },
+      [&](bool valid, int pos) { return valid ? tab[__ldg(rev_col + pos)] - bias : -1; },
+      [&](bool, int r, int, int i) {
+        if (i >= 0) cls_edge(b, t, keys, vidx, i, r);
+      });
+}
 
 // Builds the class list of n candidates, [Q | P], the first nq of them Q, over
 // nL vertices, at `at` ([at, end): at least cls_list_words + cls_build_words).
@@ -1926,6 +1976,8 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
     ROLLED for (uint32_t b = MB[w]; b; b &= b - 1) mpos[o + k++] = (uint32_t)(w * 32 + __ffs(b) - 1);
   }
   __syncwarp();
+  const ClsRaw b{MB, MP, raw, st, nq};
+  if (!ed.ids) cls_edges_of_rows(b, keys, vidx, ed.tab, ed.bias, ed.L, nL);
   ROLLED for (int e0 = 0; e0 < ed.n; e0 += 64) {
     int id[2], ci[2];
 #pragma unroll
@@ -1937,25 +1989,9 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
     for (int u = 0; u < 2; ++u)
       ci[u] = id[u] >= 0 ? ed.tab[ed.rows ? id[u] : id[u] >> 7] - ed.bias : -1;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = ci[u];
-      if (i < 0) continue;
-      const int r = ed.rows ? ed.rows[e0 + 32 * u + lane] : id[u] & 127;
-      const uint32_t w = MB[i >> 5], bit = 1u << (i & 31);
-      if (w & bit) {
-        const uint32_t d = MP[i >> 5] + __popc(w & (bit - 1u));
-        atomicOr(&raw[(size_t)(r >> 5) * st + d], 1u << (r & 31));
-      } else if (i < nq) {
-        atomicOr(&info[r], kInfoQ);
-      } else {
-        atomicMax(&first[r], 0x7fffffffu - (uint32_t)i);
-        const uint64_t k = key_of(i);
-        const uint32_t lo = (uint32_t)k;
-        const uint32_t old = atomicAdd(&t.lo[r], lo);
-        atomicAdd(&t.hi[r], (uint32_t)(k >> 32) + (old + lo < lo ? 1u : 0u));
-        atomicAdd(&info[r], 1u);
-      }
-    }
+    for (int u = 0; u < 2; ++u)
+      if (ci[u] >= 0)
+        cls_edge(b, t, keys, vidx, ci[u], ed.rows ? ed.rows[e0 + 32 * u + lane] : id[u] & 127);
   }
   __threadfence_block();
   __syncwarp();
@@ -2220,7 +2256,7 @@ __device__ __noinline__ void t1_handoff(const T1 t, int x, int level, int kept, 
     __syncwarp();
     const ClsList l =
         cls_build(at, end, nsub, nq, K, n, &nend, nullptr, ckey, cpos,
-                  ClsEdges{ent, nullptr, sidx, ne, 0}, reinterpret_cast<uint32_t*>(W.A(W.sl().tcls)));
+                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr}, reinterpret_cast<uint32_t*>(W.A(W.sl().tcls)));
     tier2(W, l, n, nend, sR, nR);
   }
   __syncwarp();
@@ -2399,7 +2435,7 @@ __device__ __noinline__ void t1_sparse_push(const T1 t, int x, int level, int ke
     int nend = ncand;
     const ClsList l =
         cls_build(at, end, ncand, nqc, K, n, &nend, nullptr, ckey, cpos,
-                  ClsEdges{ent, nullptr, sidx, ne, 0}, reinterpret_cast<uint32_t*>(tcls));
+                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr}, reinterpret_cast<uint32_t*>(tcls));
     // To an idle warp when some want work and the child is big enough by
     // GMBE's split test, else it runs here.
     int slot = -1;
@@ -3014,7 +3050,7 @@ __device__ __noinline__ void tier1_run(const T1 t) {
   }
 }
 
-__device__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count);
+__device__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count, bool keep);
 __device__ void t1_transpose(int entries, int nC);
 
 // Runs a counts-tier child exported by t1_try_export: the frame is rebuilt
@@ -3088,7 +3124,7 @@ __device__ __noinline__ void tier1_from_slot(int slot) {
   ROLLED for (int l = lane; l < n; l += 32) llevel[l] = 0;
   __threadfence_block();
   __syncwarp();
-  lay_out_rows(lv, n, run, false);
+  lay_out_rows(lv, n, run, false, true);
   ROLLED for (int e = lane; e < run; e += 32) {
     const int p = map[aadj[e]] - 1;
     aadj[e] = p;
@@ -3327,7 +3363,9 @@ __device__ bool queue_push_one(Warp& W, const Task& t) {
 // one's L position into ent, nL rows of the graph's U -> V lists end to end.
 // With `count`, counts every id in the dense map on the way and lists the ids
 // met (each once, at most capC of them) in `touched`; returns their number.
-__device__ __noinline__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count) {
+// Without `keep`, only that.
+__device__ __noinline__ int lay_out_rows(const int32_t* L, int nL, int entries, bool count,
+                                         bool keep) {
   Warp& W = this_warp();
   const int lane = (int)lane_id();
   const DevGraph& g = *W.gp;
@@ -3358,8 +3396,10 @@ __device__ __noinline__ int lay_out_rows(const int32_t* L, int nL, int entries, 
       [&](bool valid, int r, int k, int w) {
         bool isnew = false;
         if (valid) {
-          aadj[k] = w;
-          ent[k] = r;
+          if (keep) {
+            aadj[k] = w;
+            ent[k] = r;
+          }
           if (scan) {
             atomicAdd(&map[w], 1);
             atomicOr(&gseen[w >> 5], 1u << (w & 31));
@@ -3424,6 +3464,14 @@ __device__ __noinline__ void t1_transpose(int entries, int nC) {
   ROLLED for (int i = lane; i < nC; i += 32) fill[i] = 0;
   __syncwarp();
 }
+
+// Entries above which the set-up of a root on its way to the bitmap tier keeps
+// no copy of them.  Whole calls, a copy of all of them kept / none above the
+// line: 900 roots of about 33,000 entries 2.30 / 1.90 ms, 8,000 of 374,000 35.4 /
+// 31.9 ms.  Lower lines cost small roots the second walk over short rows:
+// 256 graphs of 20,000 to 40,000 edges 166 ms with none kept, 164.6 up to 1,024,
+// 161.7 up to 4,096, 161.4 up to 16,384.
+constexpr int kKeepEntries = 4096;
 
 // ---------------------------------------------------------------------------
 // Task set-up (IterFinderWithMultipleVertex) and dispatch.
@@ -3503,7 +3551,12 @@ __device__ __noinline__ void run_task(const Task& t) {
   }
   __syncwarp();
   const int entries = aoff[nL];
-  const int nt = lay_out_rows(L, nL, entries, true);
+  // A root that goes to the bitmap tier reads its entries once more, to set
+  // them as bits; many of them (every warp's together do not fit L2) come from
+  // the graph's rows again, which all warps share, rather than by way of this
+  // warp's scratch.
+  const bool laid_out = nL > W.gp->tier2_max_l || entries <= kKeepEntries;
+  const int nt = lay_out_rows(L, nL, entries, true, laid_out);
   if (nt > W.sl().capC) {
     // Vertices beyond the touched list's room keep counts: clear the whole
     // map (the launch is failing; this keeps the invariant for the record).
@@ -3735,7 +3788,9 @@ __device__ __noinline__ void run_task(const Task& t) {
       uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end));
       const ClsList cl = cls_build(
           at + cls_key_words(K), end, nC, nq, K, nL, &nend, ncnt, g.vkey, cv,
-          ClsEdges{W.A(W.sl().aadj), W.A(W.sl().ent), map, entries, 1}, nullptr);
+          ClsEdges{laid_out ? W.A(W.sl().aadj) : nullptr, W.A(W.sl().ent), map,
+                   laid_out ? entries : 0, 1, L},
+          nullptr);
       cls_run(cl, first_bits(nL, lane), nend, lkey, lid, sR, nR,
               cl.m + cls_list_words(cl.n, cl.K), end);
     } else {
@@ -3748,6 +3803,7 @@ __device__ __noinline__ void run_task(const Task& t) {
       int32_t* aadj = W.A(W.sl().aadj);
       int32_t* fill = W.A(W.sl().fill);
       int32_t* sidx = W.A(W.sl().sidx);
+      if (!laid_out) lay_out_rows(L, nL, entries, false, true);
       ROLLED for (int l = lane; l < nL; l += 32) llevel[l] = 0;
       // aadj: L row -> C index (or -1 for R)
 #pragma unroll 4
