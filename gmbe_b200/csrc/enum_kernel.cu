@@ -1341,22 +1341,25 @@ __device__ __noinline__ bool cls_export(uint32_t lnw, uint32_t base, int nsel, i
   return false;
 }
 
-// The leaf of a list of at most 32 one-word classes.
-__device__ __forceinline__ void leaf_of_list(const ClsList& l, uint32_t L, int nend,
-                                             const uint64_t* lk, uint64_t sR, uint32_t nR,
-                                             Leaf& f) {
+// The classes of a list of at most 32 one-word classes, a class per lane.
+__device__ __forceinline__ void leaf_of_list(const ClsList& l, Leaf& f) {
   const int lane = (int)lane_id();
   const bool in = lane < l.n;
   const uint32_t info = in ? l.info[lane] : 0u;
   f.m = in ? l.m[lane] : 0u;
   f.key = in ? l.key[lane] : 0ULL;
   f.cnt = info & kInfoCnt;
-  f.lk = (L >> lane) & 1u ? lk[lane] : 0ULL;
   f.A = first_bits(l.n, 0);
   f.Q = __ballot_sync(kFull, (info & kInfoQ) != 0u);
   f.P = __ballot_sync(kFull, (info & kInfoP) != 0u);
+}
+// Its L (keys lk), what its first level may push, and R of its root biclique.
+__device__ __forceinline__ void leaf_at(Leaf& f, uint32_t L, const uint64_t* lk, uint32_t lim,
+                                        uint64_t sR, uint32_t nR) {
+  const int lane = (int)lane_id();
   f.L = L;
-  f.lim = first_bits(nend, 0);
+  f.lk = (L >> lane) & 1u ? lk[lane] : 0ULL;
+  f.lim = lim;
   f.sR = sR;
   f.nR = nR;
 }
@@ -1662,7 +1665,8 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
   bool leaf = cls_begin(&l, L, &nend, lk, lid, sR0, (uint32_t)nR0, top);
   const bool root_leaf = leaf;
   if (leaf) {
-    leaf_of_list(l, __shfl_sync(kFull, L, 0), nend, lk, sR0, (uint32_t)nR0, f);
+    leaf_of_list(l, f);
+    leaf_at(f, __shfl_sync(kFull, L, 0), lk, first_bits(nend, 0), sR0, (uint32_t)nR0);
     if (lane == 0) c.leaf_lid = lid;
     __syncwarp();
   }
@@ -1772,7 +1776,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
         d.stride = (d.n + 31) & ~31;
         d.m = lm;
         leaf = d.n <= 32;
-        if (leaf) leaf_of_list(d, 0u, d.n, clk, sR, nR, f);
+        if (leaf) leaf_of_list(d, f);
         else if (lm == stop) stop += d.stride;
       } else {
         cls_copy_child(lnw, base, d.m, nsel, dK, cpos);
@@ -1780,7 +1784,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
         if (s_blk.prune && nsel > 32)
           d.n = cls_merge(d.m, d.key, d.info, nsel, dK, &d.stride, c.S, &dend);
         if (d.n <= 32 && dK == 1) {
-          leaf_of_list(d, __shfl_sync(kFull, nl, 0), d.n, clk, sR, nR, f);
+          leaf_of_list(d, f);
           leaf = true;
         }
       }
@@ -1791,12 +1795,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
       }
     }
     if (leaf) {
-      const uint32_t l0 = __shfl_sync(kFull, nl, 0);
-      f.L = l0;
-      f.lk = (l0 >> lane) & 1u ? clk[lane] : 0ULL;
-      f.lim = kFull;
-      f.sR = sR;
-      f.nR = nR;
+      leaf_at(f, __shfl_sync(kFull, nl, 0), clk, kFull, sR, nR);
       __syncwarp();
       if (lane == 0) c.leaf_lid = clid;
       __syncwarp();
@@ -2197,7 +2196,6 @@ __device__ __noinline__ void t1_handoff(const T1 t, int x, int level, int kept, 
   const int32_t* llevel = W.A(W.sl().llevel);
   const int32_t* ncnt = W.A(W.sl().ncnt);
   const int32_t* bound = W.A(W.sl().bound);
-  const int32_t* cv = W.A(W.sl().cv);
   const uint64_t* ckey = W.A64(W.sl().ckey);
   int32_t* sidx = W.A(W.sl().sidx);
   int32_t* lp = W.A(W.sl().lp);
@@ -2290,7 +2288,6 @@ __device__ __noinline__ void t1_sparse_push(const T1 t, int x, int level, int ke
   int32_t* llevel = W.A(W.sl().llevel);
   const int32_t* ncnt = W.A(W.sl().ncnt);
   int32_t* bound = W.A(W.sl().bound);
-  const int32_t* cv = W.A(W.sl().cv);
   const int32_t* coff = W.A(W.sl().coff);
   const int32_t* cadj = W.A(W.sl().cadj);
   const int32_t* aoff = W.A(W.sl().aoff);
@@ -3109,7 +3106,6 @@ __device__ __noinline__ void tier1_from_slot(int slot) {
   int32_t* sidx = W.A(W.sl().sidx);
   int32_t* llevel = W.A(W.sl().llevel);
   uint64_t* ckey = W.A64(W.sl().ckey);
-  uint64_t t0 = globaltimer_ns();
   int run = 0;
   ROLLED for (int c0 = 0; c0 < n; c0 += 32) {
     const int l = c0 + lane;
@@ -3156,7 +3152,6 @@ __device__ __noinline__ void tier1_from_slot(int slot) {
   const uint64_t t2_before = W.ns_t2;
   tier1_run(t1);
   acc(W.ns_t1, (globaltimer_ns() - t1s) - (W.ns_t2 - t2_before));
-  (void)t0;
   __syncwarp();
   ROLLED for (int i = lane; i < m; i += 32) map[cv[i]] = 0;
   __syncwarp();
