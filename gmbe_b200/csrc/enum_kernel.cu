@@ -1860,12 +1860,12 @@ __device__ __noinline__ void tier2_from_slot(int slot) {
 
 // The edges between a sub-problem's candidates and its vertices: edge e joins
 // candidate tab[ids[e]] - bias (below 0: none) and vertex rows[e]; without
-// rows, ids holds both, id << 7 | vertex.  Without ids (n = 0), they are the
-// graph's U -> V rows of the vertices L.
+// rows, ids holds both, id << 7 | vertex.  Without ids (n = 0), vertex r's are
+// the ids col[off[L[r]] .. off[L[r] + 1]) (below 0: none).
 struct ClsEdges {
   const int32_t *ids, *rows, *tab;
   int n, bias;
-  const int32_t* L;
+  const int32_t *L, *off, *col;
 };
 
 // The candidates of a list being built that get masks (bits and ranks, MB and
@@ -1897,21 +1897,20 @@ __device__ __forceinline__ void cls_edge(const ClsRaw& b, const MergeTab& t, con
   }
 }
 
-// All edges, from the graph's rows.
+// All edges of rows that are not laid out.
 __device__ __noinline__ void cls_edges_of_rows(ClsRaw b, const uint64_t* keys, const int32_t* vidx,
-                                               const int32_t* tab, int bias, const int32_t* L,
-                                               int nL) {
+                                               ClsEdges ed, int nL) {
   const MergeTab t = this_tab();
-  const int32_t *rev_off = this_warp().gp->rev_off, *rev_col = this_warp().gp->rev_col;
-  flat_rows(
+  flat_rows2(
       nL,
       [&](int r, int& beg, int& len) {
-        const int u = L[r];
-        beg = rev_off[u];
-        len = rev_off[u + 1] - beg;
+        const int u = ed.L[r];
+        beg = ed.off[u];
+        len = ed.off[u + 1] - beg;
       },
-      [&](bool valid, int pos) { return valid ? tab[__ldg(rev_col + pos)] - bias : -1; },
-      [&](bool, int r, int, int i) {
+      [&](bool valid, int pos) { return valid ? ed.col[pos] : -1; },
+      [&](int w) { return w >= 0 ? ed.tab[w] - ed.bias : -1; },
+      [&](bool, int r, int, int, int i) {
         if (i >= 0) cls_edge(b, t, keys, vidx, i, r);
       });
 }
@@ -1987,7 +1986,7 @@ __device__ __noinline__ ClsList cls_build(uint32_t* at, uint32_t* end, int n, in
   }
   __syncwarp();
   const ClsRaw b{MB, MP, raw, st, nq};
-  if (!ed.ids) cls_edges_of_rows(b, keys, vidx, ed.tab, ed.bias, ed.L, nL);
+  if (!ed.ids) cls_edges_of_rows(b, keys, vidx, ed, nL);
   ROLLED for (int e0 = 0; e0 < ed.n; e0 += 64) {
     int id[2], ci[2];
 #pragma unroll
@@ -2202,18 +2201,6 @@ __device__ __noinline__ void t1_handoff(const T1 t, int x, int level, int kept, 
   uint64_t* lkey = W.A64(W.sl().lkey);
   const int32_t* aoff = W.A(W.sl().aoff);
   const int32_t* aadj = W.A(W.sl().aadj);
-  const auto selected = [&](int i) {
-    return i < t.nC && bound[i] > level && ncnt[i] > 0 && ncnt[i] < kept;
-  };
-  int nsub = 0, nq = 0;
-  ROLLED for (int i = lane; i < t.nC; i += 32) {
-    const bool sel = selected(i);
-    nsub += sel;
-    nq += sel && i < x;  // candidates before x are Q
-  }
-  nsub = (int)__reduce_add_sync(kFull, (unsigned)nsub);
-  nq = (int)__reduce_add_sync(kFull, (unsigned)nq);
-  const int K = words_k(kept);
   // L_sub positions
   int n = 0;
   ROLLED for (int c0 = 0; c0 < t.nL; c0 += 32) {
@@ -2228,44 +2215,37 @@ __device__ __noinline__ void t1_handoff(const T1 t, int x, int level, int kept, 
     }
     n += __popc(bal);
   }
-  if (nsub > 0) {
-    uint32_t* at = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub));
-    uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)) - cls_stride(nsub);
-    int32_t* cpos = reinterpret_cast<int32_t*>(end);  // C index of each candidate
-    int o = 0;
-    ROLLED for (int c0 = 0; c0 < t.nC; c0 += 32) {
-      const int i = c0 + lane;
-      const bool sel = selected(i);
-      const unsigned bal = __ballot_sync(kFull, sel);
-      if (sel) {
-        const int s = o + __popc(bal & lanemask_lt());
-        sidx[i] = s;
-        cpos[s] = i;
-      } else if (i < t.nC) {
-        sidx[i] = -1;
-      }
-      o += __popc(bal);
+  // candidates, their C indices at the arena's end
+  uint32_t* end = reinterpret_cast<uint32_t*>(W.A(W.sl().ar_end)) - cls_stride(t.nC);
+  int32_t* cpos = reinterpret_cast<int32_t*>(end);
+  int nsub = 0, nq = 0;
+  ROLLED for (int c0 = 0; c0 < t.nC; c0 += 64) {
+    int b[2], c[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = c0 + 32 * u + lane;
+      b[u] = i < t.nC ? bound[i] : -1;
+      c[u] = i < t.nC ? ncnt[i] : 0;
     }
-    __syncwarp();
-    int nend = nsub, ne = 0;
-    int32_t* ent = W.A(W.sl().ent);
-    flat_rows(
-        n,
-        [&](int r, int& beg, int& len) {
-          int l = lp[r];
-          beg = aoff[l];
-          len = aoff[l + 1] - beg;
-        },
-        [&](bool valid, int pos) { return valid ? aadj[pos] : -1; },
-        [&](bool, int r, int, int p) {
-          const unsigned be = __ballot_sync(kFull, p >= 0);
-          if (p >= 0) ent[ne + __popc(be & lanemask_lt())] = (p << 7) | r;
-          ne += __popc(be);
-        });
-    __syncwarp();
-    const ClsList l =
-        cls_build(at, end, nsub, nq, K, n, &nend, nullptr, ckey, cpos,
-                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr}, reinterpret_cast<uint32_t*>(W.A(W.sl().tcls)));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = c0 + 32 * u + lane;
+      const bool sel = b[u] > level && c[u] > 0 && c[u] < kept;
+      const unsigned bal = __ballot_sync(kFull, sel);
+      const int s = nsub + __popc(bal & lanemask_lt());
+      if (sel) cpos[s] = i;
+      if (i < t.nC) sidx[i] = sel ? s : -1;
+      nsub += __popc(bal);
+      nq += __popc(__ballot_sync(kFull, sel && i < x));  // candidates before x are Q
+    }
+  }
+  __syncwarp();
+  if (nsub > 0) {
+    int nend = nsub;
+    const ClsList l = cls_build(
+        reinterpret_cast<uint32_t*>(W.A(W.sl().ar_sub)), end, nsub, nq, words_k(kept), n, &nend,
+        nullptr, ckey, cpos, ClsEdges{nullptr, nullptr, sidx, 0, 0, lp, aoff, aadj},
+        reinterpret_cast<uint32_t*>(W.A(W.sl().tcls)));
     tier2(W, l, n, nend, sR, nR);
   }
   __syncwarp();
@@ -2443,7 +2423,7 @@ __device__ __noinline__ void t1_sparse_push(const T1 t, int x, int level, int ke
     int nend = ncand;
     const ClsList l =
         cls_build(at, end, ncand, nqc, K, n, &nend, nullptr, ckey, cpos,
-                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr}, reinterpret_cast<uint32_t*>(tcls));
+                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr, nullptr, nullptr}, reinterpret_cast<uint32_t*>(tcls));
     // To an idle warp when some want work and the child is big enough by
     // GMBE's split test, else it runs here.
     int slot = -1;
@@ -3795,7 +3775,7 @@ __device__ __noinline__ void run_task(const Task& t) {
       const ClsList cl = cls_build(
           at + cls_key_words(K), end, nC, nq, K, nL, &nend, ncnt, g.vkey, cv,
           ClsEdges{laid_out ? W.A(W.sl().aadj) : nullptr, W.A(W.sl().ent), map,
-                   laid_out ? entries : 0, 1, L},
+                   laid_out ? entries : 0, 1, L, g.rev_off, g.rev_col},
           nullptr);
       cls_run(cl, first_bits(nL, lane), nend, lkey, lid, sR, nR,
               cl.m + cls_list_words(cl.n, cl.K), end);
