@@ -993,19 +993,19 @@ struct Tally {
   int swapped;
   int share_floor;        // |P|*|L| from which a child may be shared out
 };
-// Adds the counts to the totals; whether the walk should stop.
-__device__ __noinline__ bool tally_look(uint32_t cnt, uint32_t nonmax) {
+// Adds the counts to the totals; at a look, whether the walk should stop.
+__device__ __noinline__ bool tally_add(uint32_t cnt, uint32_t nonmax, bool look) {
   Warp& W = this_warp();
   acc(W.cnt, cnt);
   acc(W.nonmax, nonmax);
   acc(W.pushes, (unsigned long long)(cnt + nonmax) << 32);
-  return must_stop();
+  return look && must_stop();
 }
 // Counts a step; whether the walk should stop.  `every`: steps between looks, a
 // divisor of kLookSteps.
 __device__ __forceinline__ bool tally_step(Tally& y, uint32_t every) {
   if ((++y.steps & (every - 1u)) != 0u) return false;
-  const bool stop = tally_look(y.cnt, y.nonmax);
+  const bool stop = tally_add(y.cnt, y.nonmax, true);
   y.cnt = y.nonmax = 0u;
   return stop;
 }
@@ -1802,7 +1802,7 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     }
   }
   hash += warp_sum64(y.hl);
-  tally_look(y.cnt, y.nonmax);
+  tally_add(y.cnt, y.nonmax, false);
   Warp& W = this_warp();
   acc(W.hash, hash);
   acc(W.ns_t2, globaltimer_ns() - t0);

@@ -24,9 +24,9 @@ int main() {
     for (int K : {1, 2, 4}) {
       const int levels = cls_levels(32 * K, (int)n);
       const long long sub = cls_sub_words(C);
-      // below a counts-tier push: the candidates' C indices beside the list;
+      // below a counts-tier push: the candidates' C indices at its end;
       // mpos lies in the counts tier's tcls (C words)
-      build.take(sub - cls_list_words(n, K) - cls_build_words(n, K, false) - cls_stride(n), C, n, K);
+      build.take(sub - cls_list_words(n, K) - cls_build_words(n, K, false) - cls_stride(C), C, n, K);
       run.take(sub - cls_need(n, K, levels), C, n, K);
       // a root's arena also has bound, coff, fill, sidx, tcls, tlist and ckey
       root.take(sub + 8 * C - cls_key_words(K) - cls_need(n, K, levels) -
