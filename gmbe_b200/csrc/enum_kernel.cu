@@ -31,11 +31,11 @@
 
 // Loops are kept rolled unless they say otherwise, and what several places call
 // stays out of line.  The kernel is bound by instruction fetch: its warps are
-// each in another part of the code, a third of their fetches missed, and most
-// of their stalls were for want of an instruction.  Unrolled and inlined by the
-// compiler's own choice the code was 864 KB, rolled it is 303 KB; the bitmap
-// tier's time on a 300,000-edge graph, summed over the warps, went from 50 to
-// 20 s by that alone.
+// each in another part of the code, and half of their stalls are for want of an
+// instruction, the instruction caches at three quarters of their peak (a
+// 32-graph batch).  Rolled it is 336 KB, with loops unrolled as the compiler
+// would 498 KB; whole calls, rolled / unrolled: 256-graph batch 163 / 262 ms,
+// 300,000-edge graph 44 / 64 ms, medium graph 302 / 391 ms.
 #define ROLLED _Pragma("unroll 1")
 
 namespace gmbe {
@@ -453,9 +453,12 @@ __device__ __forceinline__ void graph_spawned(const Warp& W, unsigned long long 
 // What a push costs is the list it goes through.  On a 300,000-edge graph the
 // average push met 848 candidates and meets 88 classes (319 and 62, 190 and 34
 // on graphs of 20,000 to 40,000 edges), and 73 % of the pushes have at most 32,
-// one per lane.  Together with the rolled code: 28 x 40 vertices at
-// density 0.8 10.1 -> 2.2 ms, 160 graphs through a server 447 -> 336 ms, the 300,000-edge
-// graph 61 -> 52 ms (where one root's counts tier, on one warp, is most of it).
+// one per lane.  Kernel times with single candidates (unrolled code) / now: 28 x
+// 40 vertices at density 0.8 8.2 / 1.65 ms, 300 x 200 with planted blocks 0.83 /
+// 0.25 ms, 20,000 edges 1.09 / 0.79 ms.  Where next to no candidates are equal, a
+// child of 33 to 128 classes costs more than it did, and a launch that waits for
+// one warp's chain of them longer: 60 x 40 at density 0.6 5.1 / 6.8 ms in one
+// vertex order, 5.5 / 5.4 in the other, 80 x 36 7.4 / 10.6 ms.
 //
 // Lists live in memory as planes (word w of class i at m[w * stride + i]), so
 // a warp's sweep over 32 classes reads one line per mask word.
@@ -4120,8 +4123,9 @@ __device__ __forceinline__ void enum_main(const DevGraph* graphs, const long lon
     // Until something may have changed.  One idle warp of the block looks at
     // the queue, the others at the block's own flag in shared memory until they
     // take the lookout over: thousands of warps reading the launch's counters
-    // kept one L2 slice busy and held up everyone's memory traffic (a half-size
-    // grid was a third faster).
+    // keep one L2 slice busy and hold up everyone's memory traffic (a shard of
+    // eight of the medium graph, on which most warps idle: 139-148 ms, with
+    // every idle warp looking 153 ms; the 256-graph batch 164 / 165 ms).
     if (lane == 0) {
       bool look = false;
       ROLLED for (int r = 0; r < 16; ++r) {
