@@ -119,15 +119,17 @@ int ensure_captured(mbe_batch* b, Workspace& ws, const mbe_params& prm) {
     b->plan.clear_maps = !engine_maps_clean(ws, b->plan);
     return engine_clear_maps(ws, &b->plan, b->stream);
   }
+  // The captured launch goes with its plan: a preparation that fails leaves
+  // neither.
+  if (b->exec) {
+    cudaGraphExecDestroy(b->exec);
+    b->exec = nullptr;
+  }
   LaunchPlan& plan = b->plan;
   int rc = engine_prepare(ws, b->spec, prm, &plan);
   if (rc) return rc;
   if ((rc = engine_clear_maps(ws, &plan, b->stream))) return rc;
   BCK(cudaStreamSynchronize(b->stream));
-  if (b->exec) {
-    cudaGraphExecDestroy(b->exec);
-    b->exec = nullptr;
-  }
   cudaGraph_t graph = nullptr;
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   rc = engine_enqueue(ws, &plan, b->d_graphs, b->d_prefix, b->d_gres, b->n, b->stream, nullptr,

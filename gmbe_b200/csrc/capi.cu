@@ -319,15 +319,17 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
   plan->map_words = spec.map_words;
   size_t need = scratch_bytes(plan->sl, big_sl, plan->warps, n_big);
   if (need > ws.scratch_bytes) {
+    // (Captured launches refer to what is freed here, whether or not there is
+    // anything in its place afterwards.)
+    ++ws.gen;
     cudaFree(ws.scratch);
     ws.scratch = nullptr;
     ws.scratch_bytes = 0;
+    ws.map_pitch_words = -1;
     cudaError_t e = cudaMalloc((void**)&ws.scratch, need);
     if (e != cudaSuccess)
       return set_error(MBE_ERR_NOMEM, "scratch of %.2f GB: %s", need / 1e9, cudaGetErrorString(e));
     ws.scratch_bytes = need;
-    ws.map_pitch_words = -1;
-    ++ws.gen;
   }
   // Every task leaves its warp's dense count map all-zero.  A different
   // layout puts the maps elsewhere: they are cleared (strided, maps only).
@@ -339,6 +341,7 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
                      : (int32_t)std::min<int64_t>(1 << 22,
                                                   std::max<int64_t>(1 << 16, 8LL * spec.map_words));
   if (qcap != ws.q_cap) {
+    ++ws.gen;
     cudaFree(ws.q_tasks);
     cudaFree(ws.q_seq);
     ws.q_tasks = nullptr;
@@ -347,7 +350,6 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
     CK(cudaMalloc((void**)&ws.q_tasks, sizeof(Task) * (size_t)qcap));
     CK(cudaMalloc((void**)&ws.q_seq, sizeof(unsigned long long) * (size_t)qcap));
     ws.q_cap = qcap;
-    ++ws.gen;
   }
   if (!ws.ctl) {
     CK(cudaMalloc((void**)&ws.ctl, sizeof(EnumCtl)));
@@ -371,12 +373,12 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
     ++ws.gen;
   }
   if (plan->blocks > ws.exit_cap) {
+    ++ws.gen;
     cudaFree(ws.exit_ns);
     ws.exit_ns = nullptr;
     ws.exit_cap = 0;
     CK(cudaMalloc((void**)&ws.exit_ns, 2 * sizeof(unsigned long long) * (size_t)plan->blocks));
     ws.exit_cap = plan->blocks;
-    ++ws.gen;
   }
   if (!ws.d_graph1) {
     CK(cudaMalloc((void**)&ws.d_graph1, sizeof(DevGraph)));
