@@ -571,7 +571,8 @@ __device__ int slot_alloc_for(Warp& W, int n, int K) {
 // Whether a child of n classes and so many levels can be exported at all:
 // some kind of slot holds it, and every warp of the launch can run it.
 __device__ __forceinline__ bool slot_fits(const Warp& W, int n, int K, int levels) {
-  if (s_blk.nslot == 0 || cls_need(n, K, levels) + cls_key_words(K) > s_blk.import_words) return false;
+  if (s_blk.nslot == 0 || cls_need(n, K, levels) + cls_key_words(K) > s_blk.import_words)
+    return false;
   return regular_fits(W, n, K) || (s_blk.nbig > 0 && n <= big_slot_cap(K));
 }
 
