@@ -51,7 +51,7 @@ namespace {
 #define BCK(call)                                                                         \
   do {                                                                                    \
     cudaError_t _e = (call);                                                              \
-    if (_e != cudaSuccess) return set_error(MBE_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e)); \
+    if (_e != cudaSuccess) return set_error(MBE_ERR_CUDA, "%s: %s", #call, cuda_error_text(_e)); \
   } while (0)
 
 double now_ms() {
@@ -151,7 +151,7 @@ int ensure_captured(mbe_batch* b, Workspace& ws, const mbe_params& prm) {
   cudaGraphDestroy(graph);
   if (e4 != cudaSuccess) {
     b->exec = nullptr;
-    return set_error(MBE_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e4));
+    return set_error(MBE_ERR_CUDA, "cudaGraphInstantiate: %s", cuda_error_text(e4));
   }
   b->exec_gen = ws.gen;
   b->exec_prm = prm;
@@ -260,7 +260,7 @@ int mbe_batch_from_csr(int32_t n, const int32_t* const* row_offs, const int32_t*
                       cudaMemcpyHostToDevice)) != cudaSuccess) {
     batch_release(b);
     delete b;
-    return set_error(MBE_ERR_NOMEM, "batch arena: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_NOMEM, "batch arena: %s", cuda_error_text(e));
   }
   mbe_params def;
   mbe_params_default(&def);

@@ -27,7 +27,7 @@ double now_s() {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
-  return set_error(MBE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  return set_error(MBE_ERR_CUDA, "%s: %s", what, cuda_error_text(e));
 }
 
 #define CK(call)                                        \
@@ -328,7 +328,7 @@ int engine_prepare(Workspace& ws, const LaunchSpec& spec, const mbe_params& prm,
     ws.map_pitch_words = -1;
     cudaError_t e = cudaMalloc((void**)&ws.scratch, need);
     if (e != cudaSuccess)
-      return set_error(MBE_ERR_NOMEM, "scratch of %.2f GB: %s", need / 1e9, cudaGetErrorString(e));
+      return set_error(MBE_ERR_NOMEM, "scratch of %.2f GB: %s", need / 1e9, cuda_error_text(e));
     ws.scratch_bytes = need;
   }
   // Every task leaves its warp's dense count map all-zero.  A different
@@ -959,7 +959,7 @@ extern "C" int mbe_enumerate_emit_stream(mbe_graph* g, const mbe_params* params,
   if (e != cudaSuccess) {
     if (h_ring) cudaFreeHost(h_ring);
     if (h_read) cudaFreeHost(h_read);
-    return set_error(MBE_ERR_NOMEM, "emission ring of %lld words: %s", cap, cudaGetErrorString(e));
+    return set_error(MBE_ERR_NOMEM, "emission ring of %lld words: %s", cap, cuda_error_text(e));
   }
   const HostGraph& h = g->h;
   unsigned long long consumed = 0;

@@ -32,7 +32,7 @@ namespace {
   do {                                                                                     \
     cudaError_t _e = (call);                                                               \
     if (_e != cudaSuccess) {                                                               \
-      rc = set_error(MBE_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e));               \
+      rc = set_error(MBE_ERR_CUDA, "%s: %s", #call, cuda_error_text(_e));               \
       goto done;                                                                           \
     }                                                                                      \
   } while (0)
@@ -355,7 +355,7 @@ int ensure_host_csr(mbe_graph* g) {
                    cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
     h.row_off.clear();
-    return set_error(MBE_ERR_CUDA, "fetching the graph: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_CUDA, "fetching the graph: %s", cuda_error_text(e));
   }
   return MBE_OK;
 }

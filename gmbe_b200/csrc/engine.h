@@ -11,6 +11,14 @@
 
 namespace gmbe {
 
+// The text of a failed CUDA call, for the error that is reported.  The call's
+// error is taken off the thread with it: a later launch that asks for the last
+// error finds its own.
+inline const char* cuda_error_text(cudaError_t e) {
+  cudaGetLastError();
+  return cudaGetErrorString(e);
+}
+
 // Engine workspace, one per device, shared by every graph and batch on that
 // device and reused across calls (grown on demand).  A call holds the
 // device's workspace for its whole duration.

@@ -95,7 +95,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
   else mbe_params_default(&prm);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "cudaGetDevice: %s", cuda_error_text(e));
   if (dev < 0 || dev >= kNoAllocMaxDevices) return set_error(MBE_ERR_INVALID, "device %d", dev);
 
   // One-time set-up per device, with that device current: the pool's device
@@ -108,7 +108,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
       void* p = nullptr;
       e = cudaGetSymbolAddress(&p, g_noalloc_pool);
       if (e != cudaSuccess)
-        return set_error(MBE_ERR_CUDA, "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
+        return set_error(MBE_ERR_CUDA, "cudaGetSymbolAddress: %s", cuda_error_text(e));
       g_pool_addr[dev].ptr = static_cast<unsigned char*>(p);
     }
     pool = g_pool_addr[dev].ptr;
@@ -160,7 +160,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
                      per_block, kEnumWarps, kNoAllocPoolBytes);
   int sms = 0, occ = 0;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-    return set_error(MBE_ERR_CUDA, "device query: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_CUDA, "device query: %s", cuda_error_text(e));
   if (int rc0 = enum_blocks_per_sm(false, enum_smem_bytes(sl), &occ)) return rc0;
   int blocks = std::min(fit_blocks, std::max(1, sms * occ));
   if (prm.blocks > 0) blocks = std::min(blocks, prm.blocks);
@@ -186,7 +186,7 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
       (e = cudaMemset2DAsync(scratch, (size_t)sl.words_per_warp * sizeof(int32_t), 0,
                              (size_t)sl.zero_words * sizeof(int32_t), (size_t)warps, st)) !=
           cudaSuccess)
-    return set_error(MBE_ERR_CUDA, "clearing the pool: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_CUDA, "clearing the pool: %s", cuda_error_text(e));
   noalloc_keys<<<std::max(1, std::min(1024, (nU + nV + 255) / 256)), 256, 0, st>>>(ukey, nU, vkey,
                                                                                   nV);
 
@@ -230,6 +230,6 @@ extern "C" int mbe_enumerate_device_noalloc(const int32_t* d_row_off, const int3
                                                    q_seq, none, scratch, exit_ns);
   noalloc_finish<<<1, 32, 0, st>>>(ctl, d_gres, d_out);
   if ((e = cudaGetLastError()) != cudaSuccess)
-    return set_error(MBE_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_CUDA, "launch: %s", cuda_error_text(e));
   return MBE_OK;
 }

@@ -7,6 +7,7 @@
 
 #include <algorithm>
 
+#include "engine.h"
 #include "internal.h"
 #include "mbe.h"
 
@@ -35,7 +36,7 @@ extern "C" int mbe_measure_l2_read(int32_t device, int64_t bytes, int32_t passes
     return set_error(MBE_ERR_INVALID, "bytes must be 1-96 MiB and passes 1-1000");
   *gbs = 0;
   cudaError_t e = cudaSetDevice(device);
-  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "cudaSetDevice: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "cudaSetDevice: %s", cuda_error_text(e));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const size_t n16 = (size_t)bytes / 16;
@@ -68,7 +69,7 @@ extern "C" int mbe_measure_l2_read(int32_t device, int64_t bytes, int32_t passes
   if (st) cudaStreamDestroy(st);
   cudaFree(sink);
   cudaFree(buf);
-  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "L2 read measurement: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return set_error(MBE_ERR_CUDA, "L2 read measurement: %s", cuda_error_text(e));
   if (ms <= 0) return set_error(MBE_ERR_CUDA, "L2 read measurement: no elapsed time");
   *gbs = (double)n16 * 16.0 * passes / (ms / 1e3) / 1e9;
   return MBE_OK;

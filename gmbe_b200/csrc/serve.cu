@@ -161,7 +161,7 @@ namespace {
   do {                                                                                     \
     cudaError_t _e = (call);                                                               \
     if (_e != cudaSuccess)                                                                 \
-      return set_error(MBE_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e));             \
+      return set_error(MBE_ERR_CUDA, "%s: %s", #call, cuda_error_text(_e));             \
   } while (0)
 
 void release(mbe_server* s) {
@@ -351,7 +351,7 @@ int admit(mbe_server* s, Request* r, std::unique_lock<std::mutex>& lk) {
   if (e == cudaSuccess) e = cudaEventRecord(s->ev_copy, s->s_copy);
   lk.lock();
   if (e != cudaSuccess)
-    return set_error(MBE_ERR_CUDA, "copying a graph to the device: %s", cudaGetErrorString(e));
+    return set_error(MBE_ERR_CUDA, "copying a graph to the device: %s", cuda_error_text(e));
   return MBE_OK;
 }
 
@@ -492,7 +492,7 @@ void server_loop(mbe_server* s) {
       if (e != cudaSuccess || ctl.status != 0) {
         s->fatal = e != cudaSuccess ? MBE_ERR_CUDA
                                     : (ctl.status == kStCapacity ? MBE_ERR_CAPACITY : MBE_ERR_TIMEOUT);
-        s->fatal_msg = e != cudaSuccess ? cudaGetErrorString(e) : "device status";
+        s->fatal_msg = e != cudaSuccess ? cuda_error_text(e) : "device status";
         fail_all(s, s->fatal);
       }
       progress = true;
@@ -911,7 +911,7 @@ int mbe_server_set_emit(mbe_server* s, int64_t ring_words, mbe_server_emit_fn fn
     if (h_read) cudaFreeHost(h_read);
     s->d_ring = nullptr;
     s->d_read = nullptr;
-    return set_error(MBE_ERR_NOMEM, "emission ring of %lld words: %s", cap, cudaGetErrorString(e));
+    return set_error(MBE_ERR_NOMEM, "emission ring of %lld words: %s", cap, cuda_error_text(e));
   }
   s->h_ring = h_ring;
   s->h_read = h_read;

@@ -33,6 +33,11 @@ def test_batch_after_another_ran_out_of_memory():
     assert ei.value.name == "MBE_ERR_NOMEM"
     del held
     torch.cuda.empty_cache()
+    # the failed allocation is reported once: the launches of a device build find
+    # no error that is not theirs
+    with gm.Graph.build_on_device(*graphs[0]) as G:
+        r = G.enumerate()
+        assert (r.count, r.set_hash) == want[0]
     run_small()
     # with memory the other one runs, on scratch of its own, and the first again
     per, _ = wide.run()
