@@ -1725,7 +1725,8 @@ __device__ __noinline__ void cls_run(ClsList l, uint32_t L, int nend, const uint
     }
     // A big enough child goes to an idle warp instead, at any depth, so that a
     // subtree that started here can still be shared once warps run out of work.
-    if (nselp * (long long)kn >= y.share_floor && cls_export(lnw, base, nsel, nselp, kn, sR, nR, cpos))
+    if (nselp * (long long)kn >= y.share_floor &&
+        cls_export(lnw, base, nsel, nselp, kn, sR, nR, cpos))
       continue;
     const int kc = words_k(kn);
     const int dK = kc <= kKMax && kc < K ? kc : K;
@@ -2427,7 +2428,8 @@ __device__ __noinline__ void t1_sparse_push(const T1 t, int x, int level, int ke
     int nend = ncand;
     const ClsList l =
         cls_build(at, end, ncand, nqc, K, n, &nend, nullptr, ckey, cpos,
-                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr, nullptr, nullptr}, reinterpret_cast<uint32_t*>(tcls));
+                  ClsEdges{ent, nullptr, sidx, ne, 0, nullptr, nullptr, nullptr},
+                  reinterpret_cast<uint32_t*>(tcls));
     // To an idle warp when some want work and the child is big enough by
     // GMBE's split test, else it runs here.
     int slot = -1;
